@@ -180,3 +180,64 @@ def tolerance(case):
     if kind == "stack":
         return {"rel": 8e-2}
     return {"rel": 1e-2}
+
+
+def _plain_quantize(w):
+    """The format in plain torch: a 128-group's scale is its largest magnitude over 7 in BF16, codes -7..7."""
+    groups = w.view(w.shape[0], -1, GROUP)
+    top = groups.abs().amax(dim=2)
+    scales = torch.where(top == 0, torch.ones_like(top), top / torch.full_like(top, 7)).to(torch.bfloat16)
+    codes = (groups / scales.float()[:, :, None]).round_().clamp_(-7, 7).to(torch.int8)
+    return codes, scales
+
+
+def _plain_matrix(gen, n, k):
+    """The matrix that `_weights` draws, slab by slab, as FP64 (rows, k) blocks of code * scale."""
+    slab = max(8, (1 << 28) // k // 8 * 8)
+    for r in range(0, n, slab):
+        w = torch.empty((min(slab, n - r), k), dtype=torch.float32, device="cuda").normal_(0.0, 0.02, generator=gen)
+        codes, scales = _plain_quantize(w)
+        yield (codes.double() * scales.double()[:, :, None]).view(w.shape)
+
+
+def _plain_ffn(x, gate_up, down, w_norm):
+    if w_norm is not None:
+        x = x * torch.rsqrt(x.square().mean(dim=1, keepdim=True) + 1e-6) * (1 + w_norm)
+    g, u = (x @ gate_up.T).chunk(2, dim=1)
+    return (torch.nn.functional.silu(g) * u) @ down.T
+
+
+def exact(case, seed):
+    gen = torch.Generator(device="cuda").manual_seed(seed)
+    kind = case["kind"]
+    if kind == "quantize":
+        w = torch.empty((case["n"], case["k"]), dtype=torch.float32, device="cuda").normal_(0.0, 0.02, generator=gen)
+        codes, scales = _plain_quantize(w)
+        pairs = codes.view(case["n"], -1, 2).to(torch.uint8) & 15
+        return pairs[:, :, 0] | pairs[:, :, 1] << 4, scales
+    if kind == "gemm":      # the weights are drawn before the activations
+        state = torch.Generator(device="cuda").manual_seed(seed)
+        for _ in _plain_matrix(gen, case["n"], case["k"]):
+            pass
+        a = _activations(gen, case["rows"], case["k"]).double()
+        return torch.cat([a @ w.T for w in _plain_matrix(state, case["n"], case["k"])], dim=1)
+    hidden, inter, tokens = case["hidden"], case["inter"], case["tokens"]
+    normed = kind == "stack" or bool(case.get("norm"))
+    again = torch.Generator(device="cuda").manual_seed(seed)
+
+    def layer(g):
+        gate_up = torch.cat(list(_plain_matrix(g, 2 * inter, hidden)))
+        down = torch.cat(list(_plain_matrix(g, hidden, inter)))
+        w_norm = torch.randn(hidden, generator=g, device="cuda").mul_(0.1).to(torch.bfloat16).double() if normed else None
+        return gate_up, down, w_norm
+
+    for _ in range(case.get("layers", 1)):
+        layer(gen)
+    x = _activations(gen, tokens, hidden).double()
+    if kind != "stack":
+        y = _plain_ffn(x, *layer(again))
+        return y.cpu() if kind == "host" else y
+    for _ in range(case["layers"]):
+        y = _plain_ffn(x, *layer(again))
+        x = x + y
+    return x, y
