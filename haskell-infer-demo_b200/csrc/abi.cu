@@ -58,6 +58,7 @@ static int mlp_common(cudaStream_t stream, const void *normed, void *ws, void *l
     if (g_fused_enabled) { /* 3..64 tokens per pass on the tensor cores; longer batches in blocks of 64 */
         unsigned *status = nullptr;
         if ((st = fused_status_word(&status))) return st;
+        if ((st = stream_tc_ffn_launch(stream, normed, act, layer_out, w, tokens, H, I, nullptr, nullptr, status)) != FFN_NOT_ADMITTED) return st;
         bool taken = true;
         for (int m0 = 0; m0 < tokens && taken; m0 += 64) {
             const int m = tokens - m0 < 64 ? tokens - m0 : 64;

@@ -940,6 +940,9 @@ int gemm_int4_dispatch(const void *a, const void *packed, const void *scales, vo
     if (M <= 2) {
         const int st = gemv_int4_stream(a, packed, scales, out, M, N, K, stream);
         if (st != FFN_NOT_ADMITTED) return st;
+    } else {
+        const int st = stream_tc_gemm(a, packed, scales, out, M, N, K, stream);
+        if (st != FFN_NOT_ADMITTED) return st;
     }
     return gemm_int4_generic(a, packed, scales, out, nullptr, M, N, K, stream);
 }

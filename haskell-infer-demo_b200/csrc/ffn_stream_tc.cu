@@ -1,0 +1,670 @@
+/*
+ * ffn_stream_tc.cu - INT4 matrix times three or more activation rows on the fifth-generation tensor cores:
+ * one rank's batched FFN (two launches: gate/up + SiLU*up, down + residual) and the stand-alone GEMM (LM
+ * head, projections).
+ *
+ *   swap-AB: 128 weight rows are the MMA's M (one row per tensor-memory lane), up to 128 tokens its N.  Per
+ *   128-wide quantization group the tensor core accumulates sum code * x in FP32 (codes exact in BF16,
+ *   products exact); the epilogue multiplies by the group's scale and adds up in FP32 registers - the
+ *   arithmetic of the other batched kernels, so dequantization is exact.
+ *
+ * Roofline: HBM up to some 64 tokens (a 128-row group is 8 KB = 350 cycles of an SM's share of the
+ * bandwidth; its eight MMAs take 167 cycles at 16 tokens, 334 at 64, 589 at 128), the tensor pipe beyond.
+ *
+ * Split: a unit is two groups of a block (128 rows x one block of up to 128 tokens).  All units form one
+ * line, block by block, token blocks innermost so that their weights come from L2, and every CTA takes an
+ * equal piece of it: no SM idles in a last wave whatever the shape.  A block shared by neighbouring CTAs is
+ * finished by the last of its contributors to arrive, which adds the partial sums in CTA order (FP32,
+ * through L2).  Nothing waits for another CTA.
+ *
+ * Roles of a CTA (one per SM):
+ *   producer   one thread: per unit a tiled TMA load of 128 bytes of 128 rows (gate/up: 64 gate and 64 up
+ *              rows) into the weight ring, per group one bulk copy of the activations into theirs.  Alone,
+ *              boxes of 128 bytes stream at 6.4 to 6.75 TB/s; 16-byte loads by the warps, eight rows an
+ *              instruction, at 4.6; bulk copies of 512 bytes of a row at 2.3.
+ *   conversion teams of four warps, one group each in turn: codes -> BF16, from registers straight into
+ *              tensor memory, where the MMA reads its A operand.
+ *   MMA        one elected thread.
+ *   epilogue   eight warps: warp = lane quadrant and half of the token columns.
+ *
+ * Gate/up blocks put pair 16*q + l in lanes l (gate) and l + 16 (up) of quadrant q, so SiLU * up is one
+ * shuffle away.  Activations are read in tile order (K blocks of 64 values, see ffn_tc.cu), one region per
+ * token block; the gate/up epilogue writes act that way for the down launch and in natural order for the
+ * caller.  Every wait is bounded; a wait that runs out records where, and every thread still reaches the
+ * end of the kernel, where tensor memory is released.
+ */
+#include <mutex>
+
+#include "kernels.h"
+#include "tc_common.cuh"
+
+namespace ffn {
+
+constexpr int kStMaxTokens = 128;            /* tokens of a block = MMA columns */
+constexpr int kStSlab = 512;                 /* tokens of a launch */
+constexpr int kStEpiWarps = 8;
+constexpr int kStMaxRing = 10, kStMaxA = 6, kStMaxD = 4;
+constexpr int kStUnitBytes = kTcRows * 128;  /* packed bytes of a unit */
+constexpr int kStHeader = 1024;
+constexpr int kStSmem = 232448;
+
+/* where a bounded wait gave up, the tcgen05 pair's numbering */
+enum { ST_ST_STAGE_EMPTY = 20, ST_ST_STAGE_FULL = 21, ST_ST_A_EMPTY = 22, ST_ST_A_READY = 23, ST_ST_D_EMPTY = 24, ST_ST_D_FULL = 25 };
+
+struct StreamTcParams {
+    CUtensorMap wmap;       /* packed rows as a 2-D byte tensor, box 128 bytes x 128 rows (PAIRS: x 64), 128-byte swizzle */
+    const uint16_t *s;      /* scales [rows][K/128] */
+    const uint8_t *xt;      /* activations in tile order, one region per token block */
+    int M, per_block;       /* tokens; tokens of a block */
+    int token_blocks;
+    int N, K;               /* output rows (PAIRS: gate/up pairs); columns */
+    int up_offset;          /* PAIRS: row of up row 0 */
+    int blocks;             /* row blocks x token blocks */
+    uint16_t *out;          /* bf16 [M][N] (PAIRS: act) */
+    uint8_t *act_t;         /* PAIRS: the same in tile order */
+    uint16_t *residual;     /* optional bf16 [M][N], h <- bf16(h + y) */
+    float *partial;         /* [CTA][2][columns][128] */
+    unsigned *arrivals;     /* [CTA][8], zero at the start */
+    unsigned *status;
+};
+
+/* Geometry for NP token columns. */
+template <int NP>
+struct StPlan {
+    static constexpr int kSlice = NP * 256;                            /* activations of a group */
+    static constexpr int kConvTeams = NP <= 64 ? 3 : 2;                /* beyond, the accumulators need the registers and the MMAs take longer than the conversion */
+    static constexpr int kConvWarps = kConvTeams * 4;
+    static constexpr int kProducerWarp = kStEpiWarps + kConvWarps, kMmaWarp = kProducerWarp + 1;
+    static constexpr int kThreads = (kMmaWarp + 1) * 32;
+    static constexpr int kD = NP <= 64 ? 4 : 2;                        /* accumulators */
+    static constexpr int kAFree = (512 - kD * NP) / 64;
+    static constexpr int kA = kAFree < kStMaxA ? kAFree : kStMaxA;     /* operand buffers of 64 columns */
+    static constexpr int kAFirst = 512 - kA * 64;
+    /* weight ring: at least 64 KB in flight; the rest of shared memory holds activation slices, two or more units' worth */
+    static constexpr int kX = NP <= 32 ? 8 : NP <= 64 ? 6 : 4;
+    static constexpr int kWFree = (kStSmem - kStHeader - kX * kSlice) / kStUnitBytes;
+    static constexpr int kW = kWFree < kStMaxRing ? kWFree : kStMaxRing;
+    static constexpr int kSmem = kStHeader + kX * kSlice + kW * kStUnitBytes;
+    static_assert(kW >= 4 && kA >= 4 && kSmem <= kStSmem && kD * NP <= kAFirst, "geometry");
+};
+
+struct StSmem {
+    uint64_t w_full[kStMaxRing], w_empty[kStMaxRing];
+    uint64_t x_full[8], x_empty[8];
+    uint64_t a_ready[kStMaxA], a_empty[kStMaxA];
+    uint64_t d_full[kStMaxD], d_empty[kStMaxD];
+    uint32_t tmem_base;
+    int abort_flag;
+};
+static_assert(sizeof(StSmem) <= kStHeader, "header");
+
+/* Eight codes of a word as four pairs of BF16 values code / 64, pairs (0,4) (1,5) (2,6) (3,7).  A nibble
+ * (sign bit flipped: code + 8) left where it is in the low byte of a half is a subnormal BF16, a multiple
+ * of 2^-133, and one exact FMA scales it and takes the 8 away: five ALU and four FMA-pipe instructions
+ * for eight codes, where shifting every nibble down takes seven and four (the ALU pipe bounds it). */
+__device__ __forceinline__ void st_codes(uint32_t w, uint32_t *v) {
+    const uint32_t h = w >> 8;
+    const uint32_t lo = lop3_and_xor(w, 0x000F000Fu, 0x00080008u), hi = lop3_and_xor(w, 0x00F000F0u, 0x00800080u);
+    const uint32_t lo2 = lop3_and_xor(h, 0x000F000Fu, 0x00080008u), hi2 = lop3_and_xor(h, 0x00F000F0u, 0x00800080u);
+    const uint32_t up0 = 0x7F007F00u /* 2^127 */, up1 = 0x7D007D00u /* 2^123 */, off = 0xBE00BE00u /* -8/64 */;
+    asm("fma.rn.bf16x2 %0, %1, %2, %3;" : "=r"(v[0]) : "r"(lo), "r"(up0), "r"(off));
+    asm("fma.rn.bf16x2 %0, %1, %2, %3;" : "=r"(v[1]) : "r"(hi), "r"(up1), "r"(off));
+    asm("fma.rn.bf16x2 %0, %1, %2, %3;" : "=r"(v[2]) : "r"(lo2), "r"(up0), "r"(off));
+    asm("fma.rn.bf16x2 %0, %1, %2, %3;" : "=r"(v[3]) : "r"(hi2), "r"(up1), "r"(off));
+}
+constexpr float kStCodeScale = 64.0f; /* undone once, on the finished sum */
+
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t *d) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3]), "=r"(d[4]), "=r"(d[5]), "=r"(d[6]), "=r"(d[7]) : "r"(taddr));
+}
+__device__ __forceinline__ uint16_t ld_scale(const uint16_t *p) {
+    uint16_t v;
+    asm volatile("ld.global.nc.u16 %0, [%1];" : "=h"(v) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ void st_give_up(StSmem *sm, unsigned *status, int where) {
+    *(volatile int *)&sm->abort_flag = 1;
+    atomicCAS(status, 0u, (unsigned)where | ((unsigned)blockIdx.x << 8));
+}
+/* a slot of a ring and the parity of its current round */
+struct StRing {
+    uint32_t slot = 0, phase = 0;
+    __device__ __forceinline__ void next(uint32_t n) { if (++slot == n) { slot = 0; phase ^= 1u; } }
+};
+
+/* One row's finished sums (HALF columns from column c0 of a token block): rounding, SiLU * up, residual. */
+template <int HALF, int NP, bool PAIRS>
+__device__ __forceinline__ void st_finish(const StreamTcParams &P, const float (&acc)[HALF], int rb, int tb, int quadrant, int lane, int c0) {
+    const int m0 = tb * P.per_block, count = min(P.per_block, P.M - m0);
+    if (PAIRS) {
+        const int p = rb * 64 + quadrant * 16 + (lane & 15);
+        uint8_t *tile = P.act_t + (size_t)tb * P.N * NP * 2 + (size_t)(p >> 6) * NP * 128 + tc_permute8(p & 7) * 2;
+#pragma unroll
+        for (int c = 0; c < HALF; ++c) {
+            const float mine = round_bf16(acc[c] * kStCodeScale), other = __shfl_xor_sync(~0u, mine, 16);
+            /* the pair's gate lane finishes the even columns, its up lane the odd ones */
+            if ((c & 1) == (lane >> 4) && c0 + c < count && p < P.N) {
+                const uint16_t a = f32_to_bf16_bits(silu_mul(lane < 16 ? mine : other, lane < 16 ? other : mine));
+                P.out[(size_t)(m0 + c0 + c) * P.N + p] = a;
+                *(uint16_t *)(tile + tc_tile_offset(c0 + c, (p >> 3) & 7)) = a;
+            }
+        }
+    } else {
+        const int row = rb * kTcRows + quadrant * 32 + lane;
+        if (row >= P.N) return;
+#pragma unroll
+        for (int c = 0; c < HALF; ++c)
+            if (c0 + c < count) {
+                const size_t o = (size_t)(m0 + c0 + c) * P.N + row;
+                const float y = round_bf16(acc[c] * kStCodeScale);
+                P.out[o] = f32_to_bf16_bits(y);
+                if (P.residual) P.residual[o] = f32_to_bf16_bits(bf16_bits_to_f32(P.residual[o]) + y);
+            }
+    }
+}
+
+template <int NP, bool PAIRS>
+__global__ void __launch_bounds__(StPlan<NP>::kThreads, 1) stream_tc_kernel(const __grid_constant__ StreamTcParams P) {
+    using L = StPlan<NP>;
+    extern __shared__ __align__(1024) uint8_t smem_raw[];
+    StSmem *sm = (StSmem *)smem_raw;
+    uint8_t *w_ring = smem_raw + kStHeader, *x_ring = w_ring + L::kW * kStUnitBytes;
+    volatile int *abort_flag = &sm->abort_flag;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int G = P.K / FFN_INT4_GROUP, U = (G + 1) / 2;
+    const long long total = (long long)P.blocks * U;
+    const long long it0 = total * blockIdx.x / gridDim.x, it1 = total * (blockIdx.x + 1) / gridDim.x;
+    const int count = (int)(it1 - it0);
+    int block = (int)(it0 / U), unit = (int)(it0 % U);
+
+    griddep_launch();
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < L::kW; ++i) { mbar_init(&sm->w_full[i], 1); mbar_init(&sm->w_empty[i], 8); }
+        for (int i = 0; i < L::kX; ++i) { mbar_init(&sm->x_full[i], 1); mbar_init(&sm->x_empty[i], 1); }
+        for (int i = 0; i < L::kA; ++i) { mbar_init(&sm->a_ready[i], 4); mbar_init(&sm->a_empty[i], 1); }
+        for (int i = 0; i < L::kD; ++i) { mbar_init(&sm->d_full[i], 1); mbar_init(&sm->d_empty[i], kStEpiWarps); }
+        sm->abort_flag = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == L::kMmaWarp) {
+        tmem_alloc(&sm->tmem_base, 512);
+        tmem_relinquish();
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = sm->tmem_base;
+
+    if (warp == L::kProducerWarp) {
+        /* ---------------- producer ---------------- */
+        if (elect_one()) {
+            auto w_copy = [&](int slot, int b, int u) {
+                const int rb = b / P.token_blocks;
+                uint8_t *to = w_ring + (size_t)slot * kStUnitBytes;
+                mbar_expect_tx(&sm->w_full[slot], kStUnitBytes);
+                /* rows and bytes past the matrix (a ragged last block, an odd tail's second group) arrive as zeros */
+                if (PAIRS) {
+                    tma_load_2d(to, &P.wmap, u * 128, rb * 64, &sm->w_full[slot]);
+                    tma_load_2d(to + kStUnitBytes / 2, &P.wmap, u * 128, P.up_offset + rb * 64, &sm->w_full[slot]);
+                } else {
+                    tma_load_2d(to, &P.wmap, u * 128, rb * kTcRows, &sm->w_full[slot]);
+                }
+            };
+            /* The weights never change: the first of them are on their way before the launch this one
+             * depends on, which writes the activations, is over. */
+            int w_block = block, w_unit = unit, w_done = 0;
+            uint32_t x_done = 0;
+            bool ok = true;
+            for (int i = 0; i < count && ok; ++i) {
+                for (; w_done < count && w_done < i + L::kW; ++w_done) {
+                    const int slot = w_done % L::kW;
+                    if (w_done >= L::kW) {
+                        /* the slot's unit before: waited for only when it is the next one needed */
+                        const uint32_t parity = (uint32_t)(w_done / L::kW - 1) & 1u;
+                        if (w_done > i) {
+                            if (!mbar_test_wait(&sm->w_empty[slot], parity)) break;
+                        } else if (!mbar_wait<20>(&sm->w_empty[slot], parity, abort_flag)) {
+                            st_give_up(sm, P.status, ST_ST_STAGE_EMPTY);
+                            ok = false;
+                            break;
+                        }
+                    }
+                    w_copy(slot, w_block, w_unit);
+                    if (++w_unit == U) { w_unit = 0; ++w_block; }
+                }
+                if (!ok) break;
+                if (i == 0) griddep_wait();
+                const int ng = min(2, G - 2 * unit);
+                const uint8_t *from = P.xt + (size_t)(block % P.token_blocks) * G * L::kSlice + (size_t)(2 * unit) * L::kSlice;
+                for (int k = 0; k < ng; ++k, ++x_done) {
+                    const uint32_t slot = x_done % L::kX;
+                    if (x_done >= (uint32_t)L::kX && !mbar_wait<20>(&sm->x_empty[slot], (x_done / L::kX - 1) & 1u, abort_flag)) {
+                        st_give_up(sm, P.status, ST_ST_STAGE_EMPTY);
+                        ok = false;
+                        break;
+                    }
+                    mbar_expect_tx(&sm->x_full[slot], L::kSlice);
+                    bulk_g2s(x_ring + (size_t)slot * L::kSlice, from + (size_t)k * L::kSlice, L::kSlice, &sm->x_full[slot]);
+                }
+                if (++unit == U) { unit = 0; ++block; }
+            }
+            /* never leave with a copy in flight: wait (bounded) for the last fill of every slot */
+            bool drained = true;
+            for (int f = w_done > L::kW ? w_done - L::kW : 0; f < w_done; ++f) {
+                bool done = false;
+                for (uint32_t q = 0; q < kSpinLimit && !done; ++q) done = mbar_try_wait(&sm->w_full[f % L::kW], (uint32_t)(f / L::kW) & 1u);
+                drained = drained && done;
+            }
+            for (uint32_t f = x_done > (uint32_t)L::kX ? x_done - L::kX : 0u; f < x_done; ++f) {
+                bool done = false;
+                for (uint32_t q = 0; q < kSpinLimit && !done; ++q) done = mbar_try_wait(&sm->x_full[f % L::kX], (f / L::kX) & 1u);
+                drained = drained && done;
+            }
+            if (!drained) atomicCAS(P.status, 0u, (unsigned)ST_DRAIN | ((unsigned)blockIdx.x << 8));
+        }
+        __syncwarp();
+    } else if (warp == L::kMmaWarp) {
+        /* ---------------- MMA issue ---------------- */
+        if (elect_one()) {
+            const uint32_t idesc = tc_instr_desc(NP);
+            const uint64_t bdesc0 = tc_smem_desc(smem_u32(x_ring), 1024);
+            StRing a, d, x;
+            uint32_t d_used = 0;
+            bool ok = true;
+            for (int i = 0; i < count && ok; ++i) {
+                const int ng = min(2, G - 2 * unit);
+                for (int k = 0; k < ng; ++k, ++d_used) {
+                    if (!mbar_wait<20>(&sm->x_full[x.slot], x.phase, abort_flag)) { st_give_up(sm, P.status, ST_ST_STAGE_FULL); ok = false; break; }
+                    if (d_used >= (uint32_t)L::kD && !mbar_wait<20>(&sm->d_empty[d.slot], d.phase ^ 1u, abort_flag)) { st_give_up(sm, P.status, ST_ST_D_EMPTY); ok = false; break; }
+                    if (!mbar_wait<20>(&sm->a_ready[a.slot], a.phase, abort_flag)) { st_give_up(sm, P.status, ST_ST_A_READY); ok = false; break; }
+                    tc_fence_after();
+                    const uint64_t bdesc = bdesc0 + (uint64_t)((x.slot * (uint32_t)L::kSlice) >> 4);
+                    const uint32_t acol = tmem + (uint32_t)L::kAFirst + a.slot * 64u, dcol = tmem + d.slot * (uint32_t)NP;
+#pragma unroll
+                    for (int q = 0; q < FFN_INT4_GROUP / 16; ++q)
+                        tc_mma_ts(dcol, acol + (uint32_t)(q * 8), bdesc + (uint64_t)(((q >> 2) * NP * 128 + (q & 3) * 32) >> 4), idesc, q > 0 ? 1u : 0u);
+                    tc_commit(&sm->x_empty[x.slot]);
+                    tc_commit(&sm->a_empty[a.slot]);
+                    tc_commit(&sm->d_full[d.slot]);
+                    a.next(L::kA); d.next(L::kD); x.next(L::kX);
+                }
+                if (++unit == U) unit = 0;
+            }
+        }
+        __syncwarp();
+    } else if (warp >= kStEpiWarps) {
+        /* ---------------- conversion: one group per team in turn ---------------- */
+        const uint32_t team = (uint32_t)((warp - kStEpiWarps) >> 2);
+        /* lane of tensor memory -> row of the stage: plain, or pair 16q + l in lanes l (gate) and l + 16 (up) */
+        const int q4 = warp & 3;
+        const int row = PAIRS ? q4 * 16 + (lane & 15) + (lane >> 4) * 64 : q4 * 32 + lane;
+        const uint32_t a_lane = tmem + ((uint32_t)(q4 * 32) << 16) + (uint32_t)L::kAFirst;
+        StRing w, a;
+        uint32_t turn = 0, groups = 0;
+        bool ok = true;
+        for (int i = 0; i < count && ok; ++i) {
+            const int ng = min(2, G - 2 * unit);
+            for (int k = 0; k < ng; ++k, ++groups) {
+                if (turn == team) {
+                    ok = tc_warp_wait(&sm->w_full[w.slot], w.phase, abort_flag, lane); /* tcgen05.st is warp-wide: the warp goes on together or not at all */
+                    if (!ok) { if (lane == 0) st_give_up(sm, P.status, ST_ST_STAGE_FULL); break; }
+                    const uint32_t src = smem_u32(w_ring + (size_t)w.slot * kStUnitBytes) + (uint32_t)(row * 128);
+                    uint4 packed[4];
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) packed[q] = lds16_at(src + (uint32_t)(((k * 4 + q) ^ (row & 7)) << 4));
+                    if (groups >= (uint32_t)L::kA) {
+                        ok = tc_warp_wait(&sm->a_empty[a.slot], a.phase ^ 1u, abort_flag, lane);
+                        if (!ok) { if (lane == 0) st_give_up(sm, P.status, ST_ST_A_EMPTY); break; }
+                        tc_fence_after();
+                    }
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        uint32_t v[16];
+                        st_codes(packed[q].x, v); st_codes(packed[q].y, v + 4); st_codes(packed[q].z, v + 8); st_codes(packed[q].w, v + 12);
+                        tmem_st16(a_lane + a.slot * 64u + (uint32_t)(q * 16), v);
+                    }
+                    tmem_st_wait();
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) {
+                        mbar_arrive(&sm->a_ready[a.slot]);
+                        /* eight arrivals free a unit: four per group, and at an odd tail the missing group's too */
+                        mbar_arrive(&sm->w_empty[w.slot]);
+                        if (ng == 1) mbar_arrive(&sm->w_empty[w.slot]);
+                    }
+                }
+                a.next(L::kA);
+                if (++turn == (uint32_t)L::kConvTeams) turn = 0;
+            }
+            w.next(L::kW);
+            if (++unit == U) unit = 0;
+        }
+    } else {
+        /* ---------------- epilogue ---------------- */
+        constexpr int HALF = NP / 2;
+        const int quadrant = warp & 3, c0 = (warp >> 2) * HALF;
+        const uint32_t d_lane = tmem + ((uint32_t)(quadrant * 32) << 16) + (uint32_t)c0;
+        /* this lane's row of block b; rows past a ragged end read the last row's scales */
+        auto scale_row = [&](int b) {
+            const int rb = b / P.token_blocks;
+            if (PAIRS) return (lane < 16 ? 0 : P.up_offset) + min(rb * 64 + quadrant * 16 + (lane & 15), P.N - 1);
+            return min(rb * kTcRows + quadrant * 32 + lane, P.N - 1);
+        };
+        /* a unit's two scales, fetched two units ahead (the weights' scales never change) */
+        uint16_t sc[2][2] = {{0, 0}, {0, 0}};
+        int s_block = block, s_unit = unit, s_left = count;
+        const uint16_t *s_from = P.s + (size_t)scale_row(block) * G;
+        auto fetch = [&](uint16_t (&to)[2]) {
+            if (s_left <= 0) return;
+            --s_left;
+            to[0] = ld_scale(s_from + 2 * s_unit);
+            to[1] = ld_scale(s_from + min(2 * s_unit + 1, G - 1));
+            if (++s_unit == U) { s_unit = 0; if (s_left > 0) s_from = P.s + (size_t)scale_row(++s_block) * G; }
+        };
+        fetch(sc[0]);
+        fetch(sc[1]);
+        griddep_wait(); /* before the first write: earlier launches may still read what this one overwrites */
+        float acc[HALF];
+#pragma unroll
+        for (int c = 0; c < HALF; ++c) acc[c] = 0.0f;
+        StRing d;
+        bool ok = true;
+        for (int i0 = 0; i0 < count && ok; i0 += 2) {
+#pragma unroll
+            for (int par = 0; par < 2; ++par) {
+                const int i = i0 + par;
+                if (i >= count || !ok) break;
+                const float scale[2] = {bf16_bits_to_f32(sc[par][0]), bf16_bits_to_f32(sc[par][1])};
+                fetch(sc[par]);
+#pragma unroll
+                for (int k = 0; k < 2; ++k) {
+                    if (2 * unit + k >= G) break;
+                    ok = tc_warp_wait(&sm->d_full[d.slot], d.phase, abort_flag, lane); /* tcgen05.ld is warp-wide: the warp goes on together or not at all */
+                    if (!ok) { if (lane == 0) st_give_up(sm, P.status, ST_ST_D_FULL); break; }
+                    tc_fence_after();
+#pragma unroll
+                    for (int c = 0; c < HALF; c += 16) {
+                        uint32_t v[16];
+                        tmem_ld8(d_lane + d.slot * (uint32_t)NP + (uint32_t)c, v);
+                        if (c + 8 < HALF) tmem_ld8(d_lane + d.slot * (uint32_t)NP + (uint32_t)(c + 8), v + 8);
+                        tmem_ld_wait();
+#pragma unroll
+                        for (int j = 0; j < 16; ++j)
+                            if (c + j < HALF) acc[c + j] = fmaf(scale[k], __uint_as_float(v[j]), acc[c + j]);
+                    }
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&sm->d_empty[d.slot]);
+                    d.next(L::kD);
+                }
+                if (!ok) break;
+                if (++unit == U || i + 1 == count) {
+                    /* the end of a block, or of this CTA's piece of the line */
+                    const long long first = (long long)block * U, last = first + U;
+                    const int rb = block / P.token_blocks, tb = block % P.token_blocks;
+                    bool finish = true;
+                    if (first < it0 || last > it1) {
+                        /* slot 0: the block began in an earlier CTA; 1: it begins here */
+                        const size_t per_slot = (size_t)NP * kTcRows, mine = (size_t)c0 * kTcRows + quadrant * 32 + lane;
+                        float *to = P.partial + ((size_t)blockIdx.x * 2 + (it0 > first ? 0 : 1)) * per_slot + mine;
+#pragma unroll
+                        for (int c = 0; c < HALF; ++c) __stcg(to + c * kTcRows, acc[c]);
+                        __threadfence();
+                        __syncwarp();
+                        /* CTA q holds unit u when q = floor(((u + 1) * CTAs - 1) / total) */
+                        const int q0 = (int)(((first + 1) * gridDim.x - 1) / total), q1 = (int)((last * gridDim.x - 1) / total);
+                        unsigned before = 0;
+                        if (lane == 0) before = atomicAdd(P.arrivals + (size_t)q0 * kStEpiWarps + warp, 1u);
+                        finish = __shfl_sync(~0u, before, 0) == (unsigned)(q1 - q0);
+                        if (finish) {
+                            __threadfence();
+#pragma unroll
+                            for (int c = 0; c < HALF; ++c) acc[c] = 0.0f;
+                            for (int q = q0; q <= q1; ++q) {
+                                const float *from = P.partial + ((size_t)q * 2 + (total * q / gridDim.x > first ? 0 : 1)) * per_slot + mine;
+#pragma unroll
+                                for (int c = 0; c < HALF; ++c) acc[c] += __ldcg(from + c * kTcRows);
+                            }
+                        }
+                    }
+                    if (finish) st_finish<HALF, NP, PAIRS>(P, acc, rb, tb, quadrant, lane, c0);
+#pragma unroll
+                    for (int c = 0; c < HALF; ++c) acc[c] = 0.0f;
+                    if (unit == U) { unit = 0; ++block; }
+                }
+            }
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == L::kMmaWarp) {
+        tc_fence_after();
+        tmem_dealloc(tmem, 512);
+    }
+}
+
+/* x bf16 [M][K] -> tile order, one region of np columns per token block, optionally through RMSNorm (the
+ * reference's expression and its BF16 rounding); columns without a token become zeros.  One CTA per column;
+ * the first clears the arrival counters of the launches that follow. */
+constexpr int kTileThreads = 512;
+__global__ void __launch_bounds__(kTileThreads) stream_tile_input_kernel(uint8_t *__restrict__ xt, const uint16_t *__restrict__ x,
+                                                                        const uint16_t *__restrict__ norm_w, float eps, float gemma, int M,
+                                                                        int per_block, int np, int K, unsigned *arrivals, int counters) {
+    __shared__ float red[kTileThreads / 32];
+    griddep_launch();
+    if (blockIdx.x == 0)
+        for (int i = threadIdx.x; i < counters; i += kTileThreads) arrivals[i] = 0u;
+    const int tb = blockIdx.x / np, n = blockIdx.x % np, m = tb * per_block + n;
+    const bool live = n < per_block && m < M;
+    const uint16_t *row = x + (size_t)m * K;
+    uint8_t *region = xt + (size_t)tb * K * np * 2;
+    float inv = 0.0f;
+    if (norm_w && live) {
+        float ss = 0.0f;
+        for (int p = threadIdx.x; p < K / 8; p += kTileThreads) {
+            const uint4 v = *(const uint4 *)(row + p * 8);
+            const uint32_t e[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+            for (int i = 0; i < 4; ++i) { ss = fmaf(bf16_lo(e[i]), bf16_lo(e[i]), ss); ss = fmaf(bf16_hi(e[i]), bf16_hi(e[i]), ss); }
+        }
+        ss = warp_sum(ss);
+        if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = ss;
+        __syncthreads();
+        float all = 0.0f;
+#pragma unroll
+        for (int i = 0; i < kTileThreads / 32; ++i) all += red[i];
+        inv = rsqrtf(all / (float)K + eps);
+    }
+    for (int p = threadIdx.x; p < K / 8; p += kTileThreads) {
+        uint4 v = make_uint4(0u, 0u, 0u, 0u);
+        if (live) {
+            v = *(const uint4 *)(row + p * 8);
+            if (norm_w) {
+                uint32_t e[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const float w0 = bf16_bits_to_f32(norm_w[p * 8 + 2 * i]) + gemma, w1 = bf16_bits_to_f32(norm_w[p * 8 + 2 * i + 1]) + gemma;
+                    e[i] = (uint32_t)f32_to_bf16_bits(bf16_lo(e[i]) * inv * w0) | ((uint32_t)f32_to_bf16_bits(bf16_hi(e[i]) * inv * w1) << 16);
+                }
+                v = make_uint4(e[0], e[1], e[2], e[3]);
+            }
+        }
+        const uint4 o = make_uint4(prmt(v.x, v.z, 0x5410), prmt(v.x, v.z, 0x7632), prmt(v.y, v.w, 0x5410), prmt(v.y, v.w, 0x7632));
+        *(uint4 *)(region + (size_t)(p >> 3) * np * 128 + tc_tile_offset(n, p & 7)) = o;
+    }
+}
+
+/* ---- host ----------------------------------------------------------------------------------- */
+static size_t st_round(size_t n) { return (n + 255) / 256 * 256; }
+/* Tokens of a launch in equal blocks of at most 128; a block's columns are its tokens padded to 16. */
+struct StTokens {
+    int blocks, per_block, np;
+};
+static StTokens st_tokens(int tokens) {
+    StTokens t;
+    t.blocks = (tokens + kStMaxTokens - 1) / kStMaxTokens;
+    t.per_block = (tokens + t.blocks - 1) / t.blocks;
+    t.np = (t.per_block + 15) / 16 * 16;
+    return t;
+}
+/* One CTA per SM, and none without a unit. */
+static int st_ctas(int blocks, int G, int sm_count) {
+    const long long n = (long long)blocks * ((G + 1) / 2);
+    return n < sm_count ? (int)n : sm_count;
+}
+static size_t st_counter_bytes(int sm_count) { return st_round((size_t)sm_count * kStEpiWarps * sizeof(unsigned)); }
+static size_t st_partial_bytes(int sm_count, int np) { return (size_t)sm_count * 2 * np * kTcRows * sizeof(float); }
+static size_t st_tile_bytes(const StTokens &t, int K) { return st_round((size_t)t.blocks * t.np * K * 2); }
+
+template <int NP, bool PAIRS>
+static int st_launch(const StreamTcParams &P, int ctas, cudaStream_t stream) {
+    using L = StPlan<NP>;
+    FFN_CUDA_TRY(cudaFuncSetAttribute(stream_tc_kernel<NP, PAIRS>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kSmem), "streaming tcgen05: shared-memory opt-in");
+    cudaLaunchAttribute attr = {};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)ctas); cfg.blockDim = dim3(L::kThreads); cfg.dynamicSmemBytes = L::kSmem; cfg.stream = stream;
+    cfg.attrs = &attr; cfg.numAttrs = 1;
+    FFN_CUDA_TRY(cudaLaunchKernelEx(&cfg, stream_tc_kernel<NP, PAIRS>, P), "streaming tcgen05 launch");
+    return FFN_OK;
+}
+template <bool PAIRS>
+static int st_launch_np(const StreamTcParams &P, int np, int ctas, cudaStream_t stream) {
+    switch (np) {
+        case 16: return st_launch<16, PAIRS>(P, ctas, stream);
+        case 32: return st_launch<32, PAIRS>(P, ctas, stream);
+        case 48: return st_launch<48, PAIRS>(P, ctas, stream);
+        case 64: return st_launch<64, PAIRS>(P, ctas, stream);
+        case 80: return st_launch<80, PAIRS>(P, ctas, stream);
+        case 96: return st_launch<96, PAIRS>(P, ctas, stream);
+        case 112: return st_launch<112, PAIRS>(P, ctas, stream);
+        default: return st_launch<128, PAIRS>(P, ctas, stream);
+    }
+}
+static int st_tile_input(uint8_t *xt, const void *x, const FusedNorm *norm, int M, const StTokens &t, int K, unsigned *arrivals, size_t counter_bytes, cudaStream_t stream) {
+    stream_tile_input_kernel<<<t.blocks * t.np, kTileThreads, 0, stream>>>(xt, (const uint16_t *)x, norm ? (const uint16_t *)norm->weight : nullptr,
+                                                                           norm ? norm->eps : 1.0f, norm && norm->gemma ? 1.0f : 0.0f, M, t.per_block, t.np, K,
+                                                                           arrivals, (int)(counter_bytes / sizeof(unsigned)));
+    FFN_CUDA_TRY(cudaGetLastError(), "tile-order input launch");
+    return FFN_OK;
+}
+static int st_device(int *dev, int *sm_count) {
+    int smem = 0;
+    FFN_CUDA_TRY(cudaGetDevice(dev), "cudaGetDevice");
+    if (*dev < 0 || *dev >= 64) return fail(FFN_ERR_CONFIG, "device index %d out of range", *dev);
+    FFN_CUDA_TRY(cudaDeviceGetAttribute(sm_count, cudaDevAttrMultiProcessorCount, *dev), "SM count");
+    FFN_CUDA_TRY(cudaDeviceGetAttribute(&smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, *dev), "smem opt-in");
+    return smem >= kStSmem ? FFN_OK : FFN_NOT_ADMITTED;
+}
+
+/* Scratch of the FFN pair per device, sized for a whole slab of tokens and grown for larger layers (calls
+ * on one device are serialised by the caller). */
+struct StScratch {
+    uint8_t *base = nullptr;
+    size_t bytes = 0;
+};
+static StScratch g_st_scratch[64];
+static std::mutex g_st_mutex;
+
+int stream_tc_ffn_launch(cudaStream_t stream, const void *x, void *act, void *layer_out, const FfnMlpWeights *w, int tokens, int H,
+                         int I, void *residual, const FusedNorm *norm, unsigned *status) {
+    if (tokens <= 16 || tc_get_mode() != 2) return FFN_NOT_ADMITTED; /* 3..16 tokens: the mma.sync pair, 63 against 81 us at 8 on the 5120 x 17408 layer */
+    if (((uintptr_t)w->gate_up_i4 & 15) || ((uintptr_t)w->down_i4 & 15) || ((uintptr_t)x & 15)) return FFN_NOT_ADMITTED;
+    int dev = 0, sm_count = 0, st = st_device(&dev, &sm_count);
+    if (st) return st;
+    /* layout: [arrivals of both launches | partial sums | input | act] */
+    const StTokens most = {kStSlab / kStMaxTokens, kStMaxTokens, kStMaxTokens};
+    const size_t counters = st_counter_bytes(sm_count), partial = st_partial_bytes(sm_count, kStMaxTokens);
+    const size_t want = 2 * counters + partial + st_tile_bytes(most, H) + st_tile_bytes(most, I);
+    std::lock_guard<std::mutex> lock(g_st_mutex);
+    StScratch &sc = g_st_scratch[dev];
+    if (sc.bytes < want) {
+        if (sc.base) { FFN_CUDA_TRY(cudaDeviceSynchronize(), "streaming tcgen05: scratch regrow"); cudaFree(sc.base); }
+        sc.base = nullptr; sc.bytes = 0;
+        if (cudaMalloc(&sc.base, want) != cudaSuccess) { (void)cudaGetLastError(); return fail(FFN_ERR_ALLOC, "streaming tcgen05: cannot allocate %zu bytes of scratch", want); }
+        sc.bytes = want;
+    }
+    StreamTcParams A = {}, B = {};
+    if ((st = weight_tile_map(&A.wmap, w->gate_up_i4, 2 * I, H, 64))) return st;
+    if ((st = weight_tile_map(&B.wmap, w->down_i4, H, I, kTcRows))) return st;
+    for (int m0 = 0; m0 < tokens; m0 += kStSlab) {
+        const int m = tokens - m0 < kStSlab ? tokens - m0 : kStSlab;
+        const StTokens t = st_tokens(m);
+        uint8_t *xt = sc.base + 2 * counters + partial, *act_t = xt + st_tile_bytes(most, H);
+        if ((st = st_tile_input(xt, (const uint16_t *)x + (size_t)m0 * H, norm, m, t, H, (unsigned *)sc.base, 2 * counters, stream))) return st;
+        A.s = (const uint16_t *)w->gate_up_i4_scales; A.xt = xt;
+        A.M = m; A.per_block = t.per_block; A.token_blocks = t.blocks;
+        A.N = I; A.K = H; A.up_offset = I; A.blocks = (I / 64) * t.blocks;
+        A.out = (uint16_t *)act + (size_t)m0 * I; A.act_t = act_t;
+        A.partial = (float *)(sc.base + 2 * counters); A.arrivals = (unsigned *)sc.base; A.status = status;
+        if ((st = st_launch_np<true>(A, t.np, st_ctas(A.blocks, H / FFN_INT4_GROUP, sm_count), stream))) return st;
+        B.s = (const uint16_t *)w->down_i4_scales; B.xt = act_t;
+        B.M = m; B.per_block = t.per_block; B.token_blocks = t.blocks;
+        B.N = H; B.K = I; B.blocks = (H / kTcRows) * t.blocks;
+        B.out = (uint16_t *)layer_out + (size_t)m0 * H; B.residual = residual ? (uint16_t *)residual + (size_t)m0 * H : nullptr;
+        B.partial = A.partial; B.arrivals = (unsigned *)(sc.base + counters); B.status = status;
+        if ((st = st_launch_np<false>(B, t.np, st_ctas(B.blocks, I / FFN_INT4_GROUP, sm_count), stream))) return st;
+    }
+    return FFN_OK;
+}
+
+/* The GEMM's scratch comes from a stream-ordered pool of its own, so calls on different streams and threads
+ * never share it; the pool keeps at most 64 MiB between calls. */
+constexpr unsigned long long kStPoolKeep = 64ull << 20;
+static cudaMemPool_t g_st_pool[64];
+static std::mutex g_st_pool_mutex;
+static int st_pool(int dev, cudaMemPool_t *out) {
+    std::lock_guard<std::mutex> lock(g_st_pool_mutex);
+    if (!g_st_pool[dev]) {
+        cudaMemPoolProps props = {};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = dev;
+        cudaMemPool_t p = nullptr;
+        unsigned long long keep = kStPoolKeep;
+        if (cudaMemPoolCreate(&p, &props) != cudaSuccess || cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) {
+            (void)cudaGetLastError();
+            return FFN_NOT_ADMITTED;
+        }
+        g_st_pool[dev] = p;
+    }
+    *out = g_st_pool[dev];
+    return FFN_OK;
+}
+
+int stream_tc_gemm(const void *a, const void *packed, const void *scales, void *out, int M, int N, int K, cudaStream_t stream) {
+    int dev = 0, sm_count = 0, st = st_device(&dev, &sm_count);
+    if (st) return st;
+    unsigned *status = nullptr;
+    if ((st = fused_status_word(&status))) return st;
+    cudaMemPool_t pool;
+    if (st_pool(dev, &pool) != FFN_OK) return FFN_NOT_ADMITTED;
+    const StTokens most = st_tokens(M < kStSlab ? M : kStSlab);
+    const size_t counters = st_counter_bytes(sm_count), partial = st_partial_bytes(sm_count, M <= kStSlab ? most.np : kStMaxTokens);
+    const size_t tiles = M <= kStSlab ? st_tile_bytes(most, K) : st_round((size_t)kStSlab * K * 2);
+    StreamTcParams P = {};
+    if ((st = weight_tile_map(&P.wmap, packed, N, K, kTcRows))) return st;
+    uint8_t *base = nullptr;
+    if (cudaMallocFromPoolAsync((void **)&base, counters + partial + tiles, pool, stream) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return FFN_NOT_ADMITTED;
+    }
+    for (int m0 = 0; m0 < M && st == FFN_OK; m0 += kStSlab) {
+        const int m = M - m0 < kStSlab ? M - m0 : kStSlab;
+        const StTokens t = st_tokens(m);
+        uint8_t *xt = base + counters + partial;
+        if ((st = st_tile_input(xt, (const uint16_t *)a + (size_t)m0 * K, nullptr, m, t, K, (unsigned *)base, counters, stream))) break;
+        P.s = (const uint16_t *)scales; P.xt = xt;
+        P.M = m; P.per_block = t.per_block; P.token_blocks = t.blocks;
+        P.N = N; P.K = K; P.blocks = ((N + kTcRows - 1) / kTcRows) * t.blocks;
+        P.out = (uint16_t *)out + (size_t)m0 * N;
+        P.partial = (float *)(base + counters); P.arrivals = (unsigned *)base; P.status = status;
+        st = st_launch_np<false>(P, t.np, st_ctas(P.blocks, K / FFN_INT4_GROUP, sm_count), stream);
+    }
+    if (cudaFreeAsync(base, stream) != cudaSuccess && st == FFN_OK) st = fail(FFN_ERR_CUDA, "ffn_gemm_int4_bf16: %s", cudaGetErrorString(cudaGetLastError()));
+    return st;
+}
+
+}  // namespace ffn

@@ -52,11 +52,10 @@
 #include <cudaTypedefs.h>
 
 #include "kernels.h"
-#include "stream_common.cuh"
+#include "tc_common.cuh"
 
 namespace ffn {
 
-constexpr int kTcRows = 128;                  /* weight rows per unit = the MMA's M = tensor-memory lanes */
 constexpr int kTcGroupsPerStage = 2;
 constexpr int kTcGroupBytes = FFN_INT4_GROUP / 2;                       /* 64 packed bytes per row and group */
 constexpr int kTcRowPitch = kTcGroupsPerStage * kTcGroupBytes;          /* 128: one row of a stage = the TMA box's inner extent = the 128-byte swizzle span */
@@ -121,83 +120,7 @@ __device__ __forceinline__ void tc_stamp(const TcParams &P, int role, uint32_t g
     if (P.trace && blockIdx.x == 0 && gi < 64u) P.trace[role * 64 + gi] = clock64();
 }
 
-/* ---- tcgen05 wrappers ------------------------------------------------------------------------ */
-__device__ __forceinline__ void tmem_alloc(uint32_t *dst_smem, uint32_t ncols) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(dst_smem)), "r"(ncols) : "memory");
-}
-__device__ __forceinline__ void tmem_relinquish() { asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory"); }
-__device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols) {
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
-}
-__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_commit(uint64_t *bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-/* D[tmem] (+)= A[tmem] * B[smem]: M = 128 (lane = row), N and the operand types from the instruction
- * descriptor, K = 16; one column of A = two consecutive values of K in BF16 */
-__device__ __forceinline__ void tc_mma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-    asm volatile("{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\ntcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}"
-                 ::"r"(d_tmem), "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
-}
-/* 16 consecutive columns of this thread's lane */
-__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&v)[16]) {
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
-                 ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]),
-                   "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]) : "memory");
-}
-__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-/* 16 consecutive FP32 columns of this thread's lane */
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&d)[16]) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-                 : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3]), "=r"(d[4]), "=r"(d[5]), "=r"(d[6]), "=r"(d[7]),
-                   "=r"(d[8]), "=r"(d[9]), "=r"(d[10]), "=r"(d[11]), "=r"(d[12]), "=r"(d[13]), "=r"(d[14]), "=r"(d[15])
-                 : "r"(taddr));
-}
-/* tiled TMA load of one box: x = byte offset within the row (a multiple of 16), y = row */
-__device__ __forceinline__ void tma_load_2d(void *dst, const CUtensorMap *map, int x, int y, uint64_t *bar) {
-    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
-                 ::"r"(smem_u32(dst)), "l"(map), "r"(x), "r"(y), "r"(smem_u32(bar)) : "memory");
-}
-__device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void epi_bar() { asm volatile("bar.sync 1, 128;" ::: "memory"); } /* the four epilogue warps */
-
-/* Shared-memory operand descriptor: K-major, 128-byte swizzle.  A row of the operand is 128 bytes (64
- * values of K); 8 rows form a 1024-byte atom inside which the 16-byte piece c of row r sits at piece
- * c ^ (r & 7); `sbo` is the distance between 8-row atoms.  The leading-dimension field is not used by
- * swizzled K-major layouts (set to 1, as CUTLASS does); bits 46-47 = 1 is the descriptor version of this
- * architecture, layout type 2 (bits 61-63) the 128-byte swizzle.  An MMA's K = 16 (32 bytes) is
- * selected inside the 128-byte row by adding 32 bytes to the start address. */
-__device__ __forceinline__ uint64_t tc_smem_desc(uint32_t addr, uint32_t sbo) {
-    const uint32_t lo = ((addr >> 4) & 0x3FFFu) | (1u << 16);
-    const uint32_t hi = ((sbo >> 4) & 0x3FFFu) | (1u << 14) | (2u << 29);
-    return ((uint64_t)hi << 32) | lo;
-}
-/* Instruction descriptor of kind::f16: D = FP32 (bits 4-5 = 1), A = B = BF16 (bits 7-9, 10-12 = 1), both
- * K-major (bits 15, 16 = 0), N / 8 in bits 17-22, M / 16 in bits 24-28. */
-__device__ __forceinline__ uint32_t tc_instr_desc(int n) {
-    return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(kTcRows >> 4) << 24);
-}
-/* nibbles s and s+4 of a word as exact BF16 codes (low half: nibble s, high half: nibble s+4):
- * 0x4300 | n is 128 + n, the xor with 8 turns the two's-complement nibble into code + 8 */
-__device__ __forceinline__ uint32_t tc_codes(uint32_t w_shifted) {
-    uint32_t v, d;
-    asm("lop3.b32 %0, %1, 0x000F000F, 0x43084308, 0x6A;" : "=r"(v) : "r"(w_shifted));
-    asm("sub.rn.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(v), "r"(0x43084308u));
-    return d;
-}
-__device__ __forceinline__ int tc_permute8(int e) { return ((e & 3) << 1) | (e >> 2); }
-/* byte offset of token n's 16-byte piece c inside one K block of the activations' tile order */
-__host__ __device__ __forceinline__ int tc_tile_offset(int n, int c) { return (n >> 3) * 1024 + (n & 7) * 128 + ((c ^ (n & 7)) << 4); }
-
-/* Bounded wait of a whole warp: one lane polls, the result reaches the others through a shuffle (which
- * also orders their later accesses after the poll).  Thirty-two lanes polling the same barrier word
- * only multiply the shared-memory traffic that every other warp's loads and arrivals queue behind. */
-__device__ __forceinline__ bool tc_warp_wait(uint64_t *bar, uint32_t parity, volatile int *abort_flag, int lane) {
-    int ok = 1;
-    if (lane == 0) ok = mbar_wait<32>(bar, parity, abort_flag) ? 1 : 0;
-    return __shfl_sync(~0u, ok, 0) != 0;
-}
 
 struct TcUnit {
     int row_a, row_b;   /* weight rows of lanes 0-63 and 64-127 */
@@ -614,6 +537,7 @@ int tc_set_mode(int mode) {
     if (mode >= 0 && mode <= 2) g_tc_mode = mode;
     return old;
 }
+int tc_get_mode() { return g_tc_mode; }
 /* Measured on B200 (5120 x 17408, us per FFN, tcgen05 vs mma.sync pair): 8 tokens 79 vs 56, 16: 82 vs 73,
  * 24: 91 vs 93, 32: 93 vs 96, 48: 107 vs 177, 64: 123 vs 186; on TP=2 slices 32: 75 vs 77, 64: 114 vs 132.
  * So: more than 16 tokens, and enough gate/up units (intermediate size / 64) to occupy half the SMs -
@@ -625,8 +549,10 @@ static bool tc_wanted(int tokens, int I, int sm_count) {
 /* The driver's tensor-map encoder, through the runtime (no link against the driver library). */
 static PFN_cuTensorMapEncodeTiled_v12000 tc_encoder() {
     static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
+    static std::mutex m;
     static bool tried = false;
-    if (!tried) { /* callers hold g_tc_mutex */
+    std::lock_guard<std::mutex> lock(m);
+    if (!tried) {
         tried = true;
         void *p = nullptr;
         cudaDriverEntryPointQueryResult q = cudaDriverEntryPointSymbolNotFound;
@@ -637,19 +563,17 @@ static PFN_cuTensorMapEncodeTiled_v12000 tc_encoder() {
     }
     return fn;
 }
-/* packed rows [rows][K/2] as a 2-D byte tensor; a box is 128 bytes (two groups) of 64 rows, written to
- * shared memory with the 128-byte swizzle */
-static int tc_weight_map(CUtensorMap *map, const void *w, int rows, int K) {
+int weight_tile_map(CUtensorMap *map, const void *w, int rows, int K, int box_rows) {
     PFN_cuTensorMapEncodeTiled_v12000 encode = tc_encoder();
-    if (!encode) return fail(FFN_ERR_CUDA, "tcgen05 FFN: the driver offers no cuTensorMapEncodeTiled");
+    if (!encode) return fail(FFN_ERR_CUDA, "the driver offers no cuTensorMapEncodeTiled");
     const cuuint64_t dims[2] = {(cuuint64_t)(K / 2), (cuuint64_t)rows};
     const cuuint64_t strides[1] = {(cuuint64_t)(K / 2)};
-    const cuuint32_t box[2] = {(cuuint32_t)kTcRowPitch, (cuuint32_t)kTcBoxRows};
+    const cuuint32_t box[2] = {(cuuint32_t)kTcRowPitch, (cuuint32_t)box_rows};
     const cuuint32_t elem[2] = {1, 1};
     const CUresult r = encode(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void *>(w), dims, strides, box, elem,
                               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) return fail(FFN_ERR_CUDA, "tcgen05 FFN: cuTensorMapEncodeTiled failed (%d)", (int)r);
+    if (r != CUDA_SUCCESS) return fail(FFN_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d)", (int)r);
     return FFN_OK;
 }
 
@@ -745,7 +669,7 @@ int tc_ffn_launch(cudaStream_t stream, const void *normed, void *act, void *laye
     FFN_CUDA_TRY(cudaGetLastError(), "tile-order input launch");
 
     TcParams A = {};
-    int st = tc_weight_map(&A.wmap, w->gate_up_i4, 2 * I, H);
+    int st = weight_tile_map(&A.wmap, w->gate_up_i4, 2 * I, H, kTcBoxRows);
     if (st) return st;
     A.xt = xt; A.s = (const uint16_t *)w->gate_up_i4_scales;
     A.M = tokens; A.npad = npad; A.N = I; A.K = H; A.up_offset = I;
@@ -754,7 +678,7 @@ int tc_ffn_launch(cudaStream_t stream, const void *normed, void *act, void *laye
     A.act = (uint16_t *)act; A.act_t = act_t;
     A.tp = 1; A.status = status; A.trace = fused_get_trace();
     TcParams B = {};
-    if ((st = tc_weight_map(&B.wmap, w->down_i4, H, I))) return st;
+    if ((st = weight_tile_map(&B.wmap, w->down_i4, H, I, kTcBoxRows))) return st;
     B.xt = act_t; B.s = (const uint16_t *)w->down_i4_scales;
     B.M = tokens; B.npad = npad; B.N = H; B.K = I;
     B.splits = tc_splits(H, I, sm_count); B.units = (H / kTcRows) * B.splits;
@@ -786,7 +710,9 @@ long long tc_tile_order_offset(int token, int k, int npad) {
 /* 3..64 tokens: the tcgen05 pair where it takes the shape, else the mma.sync pair. */
 int batched_ffn_launch(cudaStream_t stream, const void *normed, void *act, void *layer_out,
                        const FfnMlpWeights *w, int tokens, int H, int I, const FusedTp *tp, void *residual, unsigned *status) {
-    const int st = tc_ffn_launch(stream, normed, act, layer_out, w, tokens, H, I, tp, residual, status);
+    int st = FFN_NOT_ADMITTED;
+    if (!tp || tp->tp < 2) st = stream_tc_ffn_launch(stream, normed, act, layer_out, w, tokens, H, I, residual, nullptr, status);
+    if (st == FFN_NOT_ADMITTED) st = tc_ffn_launch(stream, normed, act, layer_out, w, tokens, H, I, tp, residual, status);
     if (st != FFN_NOT_ADMITTED) return st;
     return mma_ffn_launch(stream, normed, act, layer_out, w, tokens, H, I, tp, residual, status);
 }

@@ -5,6 +5,8 @@
 
 #include "../../include/ffn_int4.h"
 
+struct CUtensorMap_st;
+
 namespace ffn {
 
 /* basic_kernels.cu */
@@ -153,10 +155,19 @@ int batched_ffn_launch(cudaStream_t stream, const void *normed, void *act, void 
                        const FfnMlpWeights *w, int tokens, int H, int I, const FusedTp *tp, void *residual, unsigned *status);
 bool tc_describe_plan(int tokens, int H, int I, int sm_count, int smem_optin, char *out, size_t out_bytes);
 int tc_set_mode(int mode);
+int tc_get_mode();
 long long tc_tile_order_offset(int token, int k, int npad);
 void tc_reset_sync();
 int mma_ffn_launch(cudaStream_t stream, const void *normed, void *act, void *layer_out,
                    const FfnMlpWeights *w, int tokens, int H, int I, const FusedTp *tp, void *residual, unsigned *status);
+/* Tensor map of packed rows [rows][K/2] as a 2-D byte tensor; a box is 128 bytes (two groups) of `box_rows`
+ * rows, written to shared memory with the 128-byte swizzle (ffn_tc.cu). */
+int weight_tile_map(CUtensorMap_st *map, const void *w, int rows, int K, int box_rows);
+/* ffn_stream_tc.cu: one rank's batched FFN for any number of tokens (optional RMSNorm in its input stage,
+ * optional residual update) and the GEMM for any number of rows. */
+int stream_tc_ffn_launch(cudaStream_t stream, const void *x, void *act, void *layer_out, const FfnMlpWeights *w, int tokens, int H,
+                         int I, void *residual, const FusedNorm *norm, unsigned *status);
+int stream_tc_gemm(const void *a, const void *packed, const void *scales, void *out, int M, int N, int K, cudaStream_t stream);
 /* Device address of the status word shared by the kernels of this library (allocating it on first use). */
 int fused_status_word(unsigned **out);
 /* The fused FFN with its scratch in a static device array: calls no allocating routine. */

@@ -1,0 +1,70 @@
+"""The streaming tensor-core kernel (three rows and more) at the edges of its row blocks, K pieces and token
+blocks: the GEMM against FP64 sums over the dequantized matrix, the FFN against the CPU oracle."""
+import numpy as np
+import pytest
+import torch
+
+from gpu_util import assert_ffn_close, dev_bf16, host_f32, upload_layer
+from haskell_infer_demo_b200 import lib as L
+from haskell_infer_demo_b200 import ops
+from oracle import ffn_oracle as o
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n,k", [(8, 128), (264, 256), (4104, 1280), (37896, 512), (512, 17408)])
+@pytest.mark.parametrize("rows", [3, 16, 17, 33, 48, 64, 65, 81, 112, 128, 129, 300, 513])
+def test_gemm_against_fp64(cuda, rows, n, k):
+    gen = torch.Generator(device="cuda").manual_seed(rows * 100003 + n)
+    packed, scales = ops.quantize_int4(torch.randn((n, k), generator=gen, device=cuda) * 0.02)
+    a = torch.randn((rows, k), generator=gen, device=cuda).to(torch.bfloat16)
+    got = ops.gemm_int4_bf16(a, packed, scales).double()
+    w = ops.dequantize_int4(packed, scales)[0].double()
+    want = a.double() @ w.T
+    # half a BF16 ulp of the result, and FP32 sums of k products: k * 2^-24 of the sum of magnitudes at most
+    bound = want.abs() * 2.0 ** -8 + (a.double().abs() @ w.abs().T) * (k * 2.0 ** -24)
+    assert (got - want).abs().le(bound).all()
+    assert torch.equal(ops.gemm_int4_bf16(a, packed, scales).double(), got)     # a fixed order of summation
+    L.device_status()
+
+
+@pytest.mark.parametrize("hidden,inter", [(128, 128), (384, 1152), (1024, 3072), (2560, 640)])
+@pytest.mark.parametrize("tokens", [3, 24, 48, 70, 128])
+def test_ffn_with_norm_against_oracle(cuda, tokens, hidden, inter):
+    x, layers = o.draw_config(hidden, inter, 5 + tokens, tokens=tokens, layers=1, with_norm=True)
+    layer = layers[0]
+    want, _, act = o.ffn(layer, o.gemma_rmsnorm(x, layer.w_norm), intermediates=True)
+    mlp = upload_layer(layer, cuda, with_norm=True)
+    ws = mlp.workspace(tokens)
+    got = mlp.forward_mlp(dev_bf16(x, cuda), ws=ws)
+    L.device_status()
+    assert_ffn_close(host_f32(got), want, f"{hidden}x{inter} M={tokens}")
+    left = host_f32(ws[tokens * (hidden + 2 * inter):tokens * (hidden + 3 * inter)].view(tokens, inter))
+    assert o.compare(left, act)[1] <= 5e-3
+
+
+def test_more_tokens_than_one_launch_takes(cuda):
+    """600 tokens are a launch of 512 and one of 88: every row as its own small call gives it."""
+    _, layers = o.draw_config(512, 640, 3, tokens=1, layers=1)
+    mlp = upload_layer(layers[0], cuda)
+    mlp.dims.max_chunk = 600
+    x = torch.randn((600, 512), device=cuda).to(torch.bfloat16)
+    got = mlp.forward_mlp_prepared(x)
+    for m in range(0, 600, 100):
+        want = mlp.forward_mlp_prepared(x[m:m + 100].contiguous())
+        # the split of K over CTAs differs with the number of tokens: FP32 order, then BF16 roundings of act and y
+        err = (got[m:m + 100].float() - want.float()).norm() / want.float().norm()
+        assert err <= 2.0 ** -8
+    L.device_status()
+
+
+def test_a_row_with_nan_stays_alone(cuda):
+    packed, scales = ops.quantize_int4(torch.randn((520, 640), device=cuda) * 0.02)
+    a = torch.randn((21, 640), device=cuda).to(torch.bfloat16)
+    want = ops.gemm_int4_bf16(a, packed, scales)
+    a[9, 333] = float("nan")
+    got = ops.gemm_int4_bf16(a, packed, scales)
+    assert got[9].isnan().all()
+    keep = [m for m in range(21) if m != 9]
+    assert torch.equal(got[keep], want[keep])
+    assert np.isfinite(host_f32(got[keep])).all()
