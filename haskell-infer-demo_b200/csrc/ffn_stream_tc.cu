@@ -11,7 +11,8 @@
  * Roofline: HBM up to some 64 tokens (a 128-row group is 8 KB = 350 cycles of an SM's share of the
  * bandwidth; its eight MMAs take 167 cycles at 16 tokens, 334 at 64, 589 at 128), the tensor pipe beyond.
  *
- * Split: a unit is two groups of a block (128 rows x one block of up to 128 tokens).  All units form one
+ * Split: a unit is two groups of a block (128 rows x one block of up to 128 tokens; where K holds an odd
+ * number of groups, the last unit's second one goes through the pipeline and is not added).  All units form one
  * line, block by block, token blocks innermost so that their weights come from L2, and every CTA takes an
  * equal piece of it: no SM idles in a last wave whatever the shape.  A block shared by neighbouring CTAs is
  * finished by the last of its contributors to arrive, which adds the partial sums in CTA order (FP32,
@@ -22,9 +23,10 @@
  *              rows) into the weight ring, per group one bulk copy of the activations into theirs.  Alone,
  *              boxes of 128 bytes stream at 6.4 to 6.75 TB/s; 16-byte loads by the warps, eight rows an
  *              instruction, at 4.6; bulk copies of 512 bytes of a row at 2.3.
- *   conversion teams of four warps, one group each in turn: codes -> BF16, from registers straight into
+ *   conversion teams of four warps, one unit each in turn: codes -> BF16, from registers straight into
  *              tensor memory, where the MMA reads its A operand.
- *   MMA        one elected thread.
+ *   MMA        three warps, one group each in turn, one elected thread issues: a group costs a warp some
+ *              1000 cycles of waits, issue and commits among 20 other warps, whatever its MMAs take.
  *   epilogue   eight warps: warp = lane quadrant and half of the token columns.
  *
  * Gate/up blocks put pair 16*q + l in lanes l (gate) and l + 16 (up) of quadrant q, so SiLU * up is one
@@ -72,20 +74,26 @@ struct StreamTcParams {
 template <int NP>
 struct StPlan {
     static constexpr int kSlice = NP * 256;                            /* activations of a group */
-    static constexpr int kConvTeams = NP <= 64 ? 3 : 2;                /* beyond, the accumulators need the registers and the MMAs take longer than the conversion */
+    static constexpr int kConvTeams = NP <= 32 ? 3 : 2;
     static constexpr int kConvWarps = kConvTeams * 4;
+    static constexpr int kMmaWarps = NP <= 64 ? 3 : 2;
     static constexpr int kProducerWarp = kStEpiWarps + kConvWarps, kMmaWarp = kProducerWarp + 1;
-    static constexpr int kThreads = (kMmaWarp + 1) * 32;
+    static constexpr int kThreads = (kMmaWarp + kMmaWarps) * 32;
     static constexpr int kD = NP <= 64 ? 4 : 2;                        /* accumulators */
-    static constexpr int kAFree = (512 - kD * NP) / 64;
-    static constexpr int kA = kAFree < kStMaxA ? kAFree : kStMaxA;     /* operand buffers of 64 columns */
+    static constexpr int kA = 2 * kConvTeams;                          /* operand buffers of 64 columns: a team has two of its own */
     static constexpr int kAFirst = 512 - kA * 64;
     /* weight ring: at least 64 KB in flight; the rest of shared memory holds activation slices, two or more units' worth */
     static constexpr int kX = NP <= 32 ? 8 : NP <= 64 ? 6 : 4;
     static constexpr int kWFree = (kStSmem - kStHeader - kX * kSlice) / kStUnitBytes;
     static constexpr int kW = kWFree < kStMaxRing ? kWFree : kStMaxRing;
     static constexpr int kSmem = kStHeader + kX * kSlice + kW * kStUnitBytes;
-    static_assert(kW >= 4 && kA >= 4 && kSmem <= kStSmem && kD * NP <= kAFirst, "geometry");
+    static_assert(kW >= 4 && kSmem <= kStSmem && kD * NP <= kAFirst, "geometry");
+    /* A waiter tells rounds of a slot apart by one bit, so none may run a whole ring ahead of another:
+     * an MMA warp at group v has waited for the accumulator of group v - kMmaWarps, so the epilogue, which
+     * goes in order, is past v - kMmaWarps - kD >= v - 2 kD; that wait comes before the operand's, so the
+     * operand of v - kA <= v - kD has been used; a team at unit i has had the MMAs of its unit i - 2
+     * kConvTeams, so every team is past unit i - 2 kConvTeams - kD / 2, i.e. past i - kW. */
+    static_assert(kMmaWarps <= kD && kD <= kA && kW >= 2 * kConvTeams + kD / 2, "no role runs a ring ahead");
 };
 
 struct StSmem {
@@ -126,6 +134,18 @@ __device__ __forceinline__ uint16_t ld_scale(const uint16_t *p) {
 __device__ __forceinline__ void st_give_up(StSmem *sm, unsigned *status, int where) {
     *(volatile int *)&sm->abort_flag = 1;
     atomicCAS(status, 0u, (unsigned)where | ((unsigned)blockIdx.x << 8));
+}
+/* Bounded wait.  try_wait suspends the thread in hardware, so there is no sleep between polls: a role's
+ * turn is a chain of such waits, and a sleeping thread would answer late. */
+__device__ __forceinline__ bool st_wait(uint64_t *bar, uint32_t parity, volatile int *abort_flag) {
+    for (uint32_t i = 0; i < kSpinLimit; ++i) {
+        if (mbar_try_wait(bar, parity)) return true;
+        if ((i & 255) == 255 && *abort_flag) return false;
+    }
+    return false;
+}
+__device__ __forceinline__ bool st_warp_wait(uint64_t *bar, uint32_t parity, volatile int *abort_flag) {
+    return __all_sync(~0u, st_wait(bar, parity, abort_flag));
 }
 /* a slot of a ring and the parity of its current round */
 struct StRing {
@@ -171,7 +191,7 @@ __global__ void __launch_bounds__(StPlan<NP>::kThreads, 1) stream_tc_kernel(cons
     StSmem *sm = (StSmem *)smem_raw;
     uint8_t *w_ring = smem_raw + kStHeader, *x_ring = w_ring + L::kW * kStUnitBytes;
     volatile int *abort_flag = &sm->abort_flag;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(~0u, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31; /* known uniform */
     const int G = P.K / FFN_INT4_GROUP, U = (G + 1) / 2;
     const long long total = (long long)P.blocks * U;
     const long long it0 = total * blockIdx.x / gridDim.x, it1 = total * (blockIdx.x + 1) / gridDim.x;
@@ -180,7 +200,7 @@ __global__ void __launch_bounds__(StPlan<NP>::kThreads, 1) stream_tc_kernel(cons
 
     griddep_launch();
     if (threadIdx.x == 0) {
-        for (int i = 0; i < L::kW; ++i) { mbar_init(&sm->w_full[i], 1); mbar_init(&sm->w_empty[i], 8); }
+        for (int i = 0; i < L::kW; ++i) { mbar_init(&sm->w_full[i], 1); mbar_init(&sm->w_empty[i], 4); }
         for (int i = 0; i < L::kX; ++i) { mbar_init(&sm->x_full[i], 1); mbar_init(&sm->x_empty[i], 1); }
         for (int i = 0; i < L::kA; ++i) { mbar_init(&sm->a_ready[i], 4); mbar_init(&sm->a_empty[i], 1); }
         for (int i = 0; i < L::kD; ++i) { mbar_init(&sm->d_full[i], 1); mbar_init(&sm->d_empty[i], kStEpiWarps); }
@@ -224,7 +244,7 @@ __global__ void __launch_bounds__(StPlan<NP>::kThreads, 1) stream_tc_kernel(cons
                         const uint32_t parity = (uint32_t)(w_done / L::kW - 1) & 1u;
                         if (w_done > i) {
                             if (!mbar_test_wait(&sm->w_empty[slot], parity)) break;
-                        } else if (!mbar_wait<20>(&sm->w_empty[slot], parity, abort_flag)) {
+                        } else if (!st_wait(&sm->w_empty[slot], parity, abort_flag)) {
                             st_give_up(sm, P.status, ST_ST_STAGE_EMPTY);
                             ok = false;
                             break;
@@ -235,17 +255,16 @@ __global__ void __launch_bounds__(StPlan<NP>::kThreads, 1) stream_tc_kernel(cons
                 }
                 if (!ok) break;
                 if (i == 0) griddep_wait();
-                const int ng = min(2, G - 2 * unit);
-                const uint8_t *from = P.xt + (size_t)(block % P.token_blocks) * G * L::kSlice + (size_t)(2 * unit) * L::kSlice;
-                for (int k = 0; k < ng; ++k, ++x_done) {
+                const uint8_t *from = P.xt + (size_t)(block % P.token_blocks) * G * L::kSlice;
+                for (int k = 0; k < 2; ++k, ++x_done) {
                     const uint32_t slot = x_done % L::kX;
-                    if (x_done >= (uint32_t)L::kX && !mbar_wait<20>(&sm->x_empty[slot], (x_done / L::kX - 1) & 1u, abort_flag)) {
+                    if (x_done >= (uint32_t)L::kX && !st_wait(&sm->x_empty[slot], (x_done / L::kX - 1) & 1u, abort_flag)) {
                         st_give_up(sm, P.status, ST_ST_STAGE_EMPTY);
                         ok = false;
                         break;
                     }
                     mbar_expect_tx(&sm->x_full[slot], L::kSlice);
-                    bulk_g2s(x_ring + (size_t)slot * L::kSlice, from + (size_t)k * L::kSlice, L::kSlice, &sm->x_full[slot]);
+                    bulk_g2s(x_ring + (size_t)slot * L::kSlice, from + (size_t)min(2 * unit + k, G - 1) * L::kSlice, L::kSlice, &sm->x_full[slot]);
                 }
                 if (++unit == U) { unit = 0; ++block; }
             }
@@ -264,81 +283,79 @@ __global__ void __launch_bounds__(StPlan<NP>::kThreads, 1) stream_tc_kernel(cons
             if (!drained) atomicCAS(P.status, 0u, (unsigned)ST_DRAIN | ((unsigned)blockIdx.x << 8));
         }
         __syncwarp();
-    } else if (warp == L::kMmaWarp) {
-        /* ---------------- MMA issue ---------------- */
-        if (elect_one()) {
-            const uint32_t idesc = tc_instr_desc(NP);
-            const uint64_t bdesc0 = tc_smem_desc(smem_u32(x_ring), 1024);
-            StRing a, d, x;
-            uint32_t d_used = 0;
-            bool ok = true;
-            for (int i = 0; i < count && ok; ++i) {
-                const int ng = min(2, G - 2 * unit);
-                for (int k = 0; k < ng; ++k, ++d_used) {
-                    if (!mbar_wait<20>(&sm->x_full[x.slot], x.phase, abort_flag)) { st_give_up(sm, P.status, ST_ST_STAGE_FULL); ok = false; break; }
-                    if (d_used >= (uint32_t)L::kD && !mbar_wait<20>(&sm->d_empty[d.slot], d.phase ^ 1u, abort_flag)) { st_give_up(sm, P.status, ST_ST_D_EMPTY); ok = false; break; }
-                    if (!mbar_wait<20>(&sm->a_ready[a.slot], a.phase, abort_flag)) { st_give_up(sm, P.status, ST_ST_A_READY); ok = false; break; }
-                    tc_fence_after();
-                    const uint64_t bdesc = bdesc0 + (uint64_t)((x.slot * (uint32_t)L::kSlice) >> 4);
-                    const uint32_t acol = tmem + (uint32_t)L::kAFirst + a.slot * 64u, dcol = tmem + d.slot * (uint32_t)NP;
+    } else if (warp >= L::kMmaWarp) {
+        /* ---------------- MMA issue: the warp waits together, one thread issues ---------------- */
+        uint32_t turn = (uint32_t)(warp - L::kMmaWarp); /* groups until this warp's next */
+        const uint32_t idesc = tc_instr_desc(NP);
+        const uint64_t bdesc0 = tc_smem_desc(smem_u32(x_ring), 1024);
+        StRing a, d, x;
+        uint32_t d_used = 0;
+        bool ok = true;
+        for (int i = 0; i < count && ok; ++i) {
+            for (int k = 0; k < 2; ++k, ++d_used, a.next(L::kA), d.next(L::kD), x.next(L::kX)) {
+                if (turn-- != 0) continue;
+                turn = L::kMmaWarps - 1;
+                ok = st_warp_wait(&sm->x_full[x.slot], x.phase, abort_flag);
+                if (!ok) { if (lane == 0) st_give_up(sm, P.status, ST_ST_STAGE_FULL); break; }
+                if (d_used >= (uint32_t)L::kD) {
+                    ok = st_warp_wait(&sm->d_empty[d.slot], d.phase ^ 1u, abort_flag);
+                    if (!ok) { if (lane == 0) st_give_up(sm, P.status, ST_ST_D_EMPTY); break; }
+                }
+                ok = st_warp_wait(&sm->a_ready[a.slot], a.phase, abort_flag);
+                if (!ok) { if (lane == 0) st_give_up(sm, P.status, ST_ST_A_READY); break; }
+                tc_fence_after();
+                const uint64_t bdesc = bdesc0 + (uint64_t)((x.slot * (uint32_t)L::kSlice) >> 4);
+                const uint32_t acol = tmem + (uint32_t)L::kAFirst + a.slot * 64u, dcol = tmem + d.slot * (uint32_t)NP;
+                if (elect_one()) {
 #pragma unroll
                     for (int q = 0; q < FFN_INT4_GROUP / 16; ++q)
                         tc_mma_ts(dcol, acol + (uint32_t)(q * 8), bdesc + (uint64_t)(((q >> 2) * NP * 128 + (q & 3) * 32) >> 4), idesc, q > 0 ? 1u : 0u);
                     tc_commit(&sm->x_empty[x.slot]);
                     tc_commit(&sm->a_empty[a.slot]);
                     tc_commit(&sm->d_full[d.slot]);
-                    a.next(L::kA); d.next(L::kD); x.next(L::kX);
                 }
-                if (++unit == U) unit = 0;
+                __syncwarp();
             }
         }
-        __syncwarp();
     } else if (warp >= kStEpiWarps) {
-        /* ---------------- conversion: one group per team in turn ---------------- */
+        /* ---------------- conversion: one unit per team in turn ---------------- */
         const uint32_t team = (uint32_t)((warp - kStEpiWarps) >> 2);
         /* lane of tensor memory -> row of the stage: plain, or pair 16q + l in lanes l (gate) and l + 16 (up) */
         const int q4 = warp & 3;
         const int row = PAIRS ? q4 * 16 + (lane & 15) + (lane >> 4) * 64 : q4 * 32 + lane;
         const uint32_t a_lane = tmem + ((uint32_t)(q4 * 32) << 16) + (uint32_t)L::kAFirst;
-        StRing w, a;
-        uint32_t turn = 0, groups = 0;
+        uint32_t round = 0;
         bool ok = true;
-        for (int i = 0; i < count && ok; ++i) {
-            const int ng = min(2, G - 2 * unit);
-            for (int k = 0; k < ng; ++k, ++groups) {
-                if (turn == team) {
-                    ok = tc_warp_wait(&sm->w_full[w.slot], w.phase, abort_flag, lane); /* tcgen05.st is warp-wide: the warp goes on together or not at all */
-                    if (!ok) { if (lane == 0) st_give_up(sm, P.status, ST_ST_STAGE_FULL); break; }
-                    const uint32_t src = smem_u32(w_ring + (size_t)w.slot * kStUnitBytes) + (uint32_t)(row * 128);
-                    uint4 packed[4];
+        for (int i = (int)team; i < count && ok; i += L::kConvTeams, ++round) {
+            const uint32_t slot = (uint32_t)i % L::kW;
+            ok = st_warp_wait(&sm->w_full[slot], (uint32_t)(i / L::kW) & 1u, abort_flag); /* tcgen05.st is warp-wide: the warp goes on together or not at all */
+            if (!ok) { if (lane == 0) st_give_up(sm, P.status, ST_ST_STAGE_FULL); break; }
+            const uint32_t src = smem_u32(w_ring + (size_t)slot * kStUnitBytes) + (uint32_t)(row * 128);
 #pragma unroll
-                    for (int q = 0; q < 4; ++q) packed[q] = lds16_at(src + (uint32_t)(((k * 4 + q) ^ (row & 7)) << 4));
-                    if (groups >= (uint32_t)L::kA) {
-                        ok = tc_warp_wait(&sm->a_empty[a.slot], a.phase ^ 1u, abort_flag, lane);
-                        if (!ok) { if (lane == 0) st_give_up(sm, P.status, ST_ST_A_EMPTY); break; }
-                        tc_fence_after();
-                    }
+            for (int k = 0; k < 2; ++k) {
+                const uint32_t mine = team * 2u + (uint32_t)k;
+                uint4 packed[4];
 #pragma unroll
-                    for (int q = 0; q < 4; ++q) {
-                        uint32_t v[16];
-                        st_codes(packed[q].x, v); st_codes(packed[q].y, v + 4); st_codes(packed[q].z, v + 8); st_codes(packed[q].w, v + 12);
-                        tmem_st16(a_lane + a.slot * 64u + (uint32_t)(q * 16), v);
-                    }
-                    tmem_st_wait();
-                    tc_fence_before();
-                    __syncwarp();
-                    if (lane == 0) {
-                        mbar_arrive(&sm->a_ready[a.slot]);
-                        /* eight arrivals free a unit: four per group, and at an odd tail the missing group's too */
-                        mbar_arrive(&sm->w_empty[w.slot]);
-                        if (ng == 1) mbar_arrive(&sm->w_empty[w.slot]);
-                    }
+                for (int q = 0; q < 4; ++q) packed[q] = lds16_at(src + (uint32_t)(((k * 4 + q) ^ (row & 7)) << 4));
+                if (round > 0) {
+                    ok = st_warp_wait(&sm->a_empty[mine], (round - 1u) & 1u, abort_flag);
+                    if (!ok) { if (lane == 0) st_give_up(sm, P.status, ST_ST_A_EMPTY); break; }
+                    tc_fence_after();
                 }
-                a.next(L::kA);
-                if (++turn == (uint32_t)L::kConvTeams) turn = 0;
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    uint32_t v[16];
+                    st_codes(packed[q].x, v); st_codes(packed[q].y, v + 4); st_codes(packed[q].z, v + 8); st_codes(packed[q].w, v + 12);
+                    tmem_st16(a_lane + mine * 64u + (uint32_t)(q * 16), v);
+                }
+                tmem_st_wait();
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) {
+                    mbar_arrive(&sm->a_ready[mine]);
+                    if (k == 1) mbar_arrive(&sm->w_empty[slot]);
+                }
             }
-            w.next(L::kW);
-            if (++unit == U) unit = 0;
         }
     } else {
         /* ---------------- epilogue ---------------- */
@@ -379,10 +396,10 @@ __global__ void __launch_bounds__(StPlan<NP>::kThreads, 1) stream_tc_kernel(cons
                 fetch(sc[par]);
 #pragma unroll
                 for (int k = 0; k < 2; ++k) {
-                    if (2 * unit + k >= G) break;
-                    ok = tc_warp_wait(&sm->d_full[d.slot], d.phase, abort_flag, lane); /* tcgen05.ld is warp-wide: the warp goes on together or not at all */
+                    ok = st_warp_wait(&sm->d_full[d.slot], d.phase, abort_flag); /* tcgen05.ld is warp-wide: the warp goes on together or not at all */
                     if (!ok) { if (lane == 0) st_give_up(sm, P.status, ST_ST_D_FULL); break; }
                     tc_fence_after();
+                    if (2 * unit + k < G) /* an odd tail's second group is zeros times the first one's activations: not added */
 #pragma unroll
                     for (int c = 0; c < HALF; c += 16) {
                         uint32_t v[16];
