@@ -20,11 +20,13 @@
  *
  * Roles of a CTA (one per SM):
  *   producer   one thread: per unit a tiled TMA load of 128 bytes of 128 rows (gate/up: 64 gate and 64 up
- *              rows) into the weight ring, per group one bulk copy of the activations into theirs.  Alone,
- *              boxes of 128 bytes stream at 6.4 to 6.75 TB/s; 16-byte loads by the warps, eight rows an
- *              instruction, at 4.6; bulk copies of 512 bytes of a row at 2.3.
+ *              rows) into the weight ring.  Alone, boxes of 128 bytes stream at 6.4 to 6.75 TB/s; 16-byte
+ *              loads by the warps, eight rows an instruction, at 4.6; bulk copies of 512 bytes of a row at
+ *              2.3.
  *   conversion teams of four warps, one unit each in turn: codes -> BF16, from registers straight into
- *              tensor memory, where the MMA reads its A operand.
+ *              tensor memory, where the MMA reads its A operand.  A team that has waited for its unit before
+ *              also asks for the activations that take that unit's place (one bulk copy per group): a
+ *              thread that served both rings spent 800 cycles a group on its waits and copies.
  *   MMA        three warps, one group each in turn, one elected thread issues: a group costs a warp some
  *              1000 cycles of waits, issue and commits among 20 other warps, whatever its MMAs take.
  *   epilogue   eight warps: warp = lane quadrant and half of the token columns.
@@ -82,25 +84,26 @@ struct StPlan {
     static constexpr int kD = NP <= 64 ? 4 : 2;                        /* accumulators */
     static constexpr int kA = 2 * kConvTeams;                          /* operand buffers of 64 columns: a team has two of its own */
     static constexpr int kAFirst = 512 - kA * 64;
-    /* weight ring: at least 64 KB in flight; the rest of shared memory holds activation slices, two or more units' worth */
-    static constexpr int kX = NP <= 32 ? 8 : NP <= 64 ? 6 : 4;
+    /* activation slices: two turns of every team's units where they fit, one beyond; the weight ring takes the rest */
+    static constexpr int kX = NP <= 64 ? 2 * kA : kA;
     static constexpr int kWFree = (kStSmem - kStHeader - kX * kSlice) / kStUnitBytes;
     static constexpr int kW = kWFree < kStMaxRing ? kWFree : kStMaxRing;
     static constexpr int kSmem = kStHeader + kX * kSlice + kW * kStUnitBytes;
     static_assert(kW >= 4 && kSmem <= kStSmem && kD * NP <= kAFirst, "geometry");
     /* A waiter tells rounds of a slot apart by one bit, so none may run a whole ring ahead of another:
      * an MMA warp at group v has waited for the accumulator of group v - kMmaWarps, so the epilogue, which
-     * goes in order, is past v - kMmaWarps - kD >= v - 2 kD; that wait comes before the operand's, so the
-     * operand of v - kA <= v - kD has been used; a team at unit i has had the MMAs of its unit i - 2
-     * kConvTeams, so every team is past unit i - 2 kConvTeams - kD / 2, i.e. past i - kW. */
-    static_assert(kMmaWarps <= kD && kD <= kA && kW >= 2 * kConvTeams + kD / 2, "no role runs a ring ahead");
+     * goes in order, is past v - kMmaWarps - kD >= v - 2 kD; that wait comes before the operand's and the
+     * activations', whose last rounds v - kA and v - kX are <= v - kD; a team at unit i has had the MMAs of
+     * its unit i - 2 kConvTeams, so every team is past unit i - 2 kConvTeams - kD / 2, i.e. past i - kW. */
+    static_assert(kMmaWarps <= kD && kD <= kA && kA <= kX && kW >= 2 * kConvTeams + kD / 2, "no role runs a ring ahead");
 };
 
 struct StSmem {
     uint64_t w_full[kStMaxRing], w_empty[kStMaxRing];
-    uint64_t x_full[8], x_empty[8];
-    uint64_t a_ready[kStMaxA], a_empty[kStMaxA];
-    uint64_t d_full[kStMaxD], d_empty[kStMaxD];
+    uint64_t x_full[2 * kStMaxA];
+    uint64_t a_ready[kStMaxA];  /* a group's operand is complete (one arrival per warp of the team) */
+    uint64_t done[kStMaxA];     /* its MMAs are: operand buffer and activations are free, the sums can be read */
+    uint64_t d_empty[kStMaxD];  /* the epilogue has read the accumulator out */
     uint32_t tmem_base;
     int abort_flag;
 };
@@ -201,9 +204,9 @@ __global__ void __launch_bounds__(StPlan<NP>::kThreads, 1) stream_tc_kernel(cons
     griddep_launch();
     if (threadIdx.x == 0) {
         for (int i = 0; i < L::kW; ++i) { mbar_init(&sm->w_full[i], 1); mbar_init(&sm->w_empty[i], 4); }
-        for (int i = 0; i < L::kX; ++i) { mbar_init(&sm->x_full[i], 1); mbar_init(&sm->x_empty[i], 1); }
-        for (int i = 0; i < L::kA; ++i) { mbar_init(&sm->a_ready[i], 4); mbar_init(&sm->a_empty[i], 1); }
-        for (int i = 0; i < L::kD; ++i) { mbar_init(&sm->d_full[i], 1); mbar_init(&sm->d_empty[i], kStEpiWarps); }
+        for (int i = 0; i < L::kX; ++i) mbar_init(&sm->x_full[i], 1);
+        for (int i = 0; i < L::kA; ++i) { mbar_init(&sm->a_ready[i], 4); mbar_init(&sm->done[i], 1); }
+        for (int i = 0; i < L::kD; ++i) mbar_init(&sm->d_empty[i], kStEpiWarps);
         sm->abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -216,68 +219,56 @@ __global__ void __launch_bounds__(StPlan<NP>::kThreads, 1) stream_tc_kernel(cons
     tc_fence_after();
     const uint32_t tmem = sm->tmem_base;
 
+    /* The activations of unit u of block b, group k (an odd tail's second group: the first one's again),
+     * into the slot of group v of this CTA's line */
+    auto x_copy = [&](uint32_t v, int b, int u, int k) {
+        const uint32_t slot = v % L::kX;
+        const int tb = P.token_blocks == 1 ? 0 : b % P.token_blocks;
+        const uint8_t *from = P.xt + (size_t)(uint32_t)(tb * G + min(2 * u + k, G - 1)) * L::kSlice;
+        mbar_expect_tx(&sm->x_full[slot], L::kSlice);
+        bulk_g2s(x_ring + (size_t)slot * L::kSlice, from, L::kSlice, &sm->x_full[slot]);
+    };
+
     if (warp == L::kProducerWarp) {
-        /* ---------------- producer ---------------- */
+        /* ---------------- weights, and the first turns' activations ---------------- */
         if (elect_one()) {
-            auto w_copy = [&](int slot, int b, int u) {
-                const int rb = b / P.token_blocks;
+            int i = 0;
+            bool ok = true;
+            for (; i < count && ok; ++i) {
+                const uint32_t slot = (uint32_t)i % L::kW;
+                /* The weights never change: a ring of them is on its way before the launch this one depends
+                 * on, which writes the activations, is over. */
+                if (i == min(L::kW, count - 1)) {
+                    griddep_wait();
+                    int b = (int)(it0 / U), u = (int)(it0 % U);
+                    for (int j = 0; j < min(L::kX / 2, count); ++j) {
+                        x_copy((uint32_t)(2 * j), b, u, 0);
+                        x_copy((uint32_t)(2 * j + 1), b, u, 1);
+                        if (++u == U) { u = 0; ++b; }
+                    }
+                }
+                if (i >= L::kW && !st_wait(&sm->w_empty[slot], (uint32_t)(i / L::kW - 1) & 1u, abort_flag)) {
+                    st_give_up(sm, P.status, ST_ST_STAGE_EMPTY);
+                    ok = false;
+                    break;
+                }
+                const int rb = block / P.token_blocks;
                 uint8_t *to = w_ring + (size_t)slot * kStUnitBytes;
                 mbar_expect_tx(&sm->w_full[slot], kStUnitBytes);
                 /* rows and bytes past the matrix (a ragged last block, an odd tail's second group) arrive as zeros */
                 if (PAIRS) {
-                    tma_load_2d(to, &P.wmap, u * 128, rb * 64, &sm->w_full[slot]);
-                    tma_load_2d(to + kStUnitBytes / 2, &P.wmap, u * 128, P.up_offset + rb * 64, &sm->w_full[slot]);
+                    tma_load_2d(to, &P.wmap, unit * 128, rb * 64, &sm->w_full[slot]);
+                    tma_load_2d(to + kStUnitBytes / 2, &P.wmap, unit * 128, P.up_offset + rb * 64, &sm->w_full[slot]);
                 } else {
-                    tma_load_2d(to, &P.wmap, u * 128, rb * kTcRows, &sm->w_full[slot]);
-                }
-            };
-            /* The weights never change: the first of them are on their way before the launch this one
-             * depends on, which writes the activations, is over. */
-            int w_block = block, w_unit = unit, w_done = 0;
-            uint32_t x_done = 0;
-            bool ok = true;
-            for (int i = 0; i < count && ok; ++i) {
-                for (; w_done < count && w_done < i + L::kW; ++w_done) {
-                    const int slot = w_done % L::kW;
-                    if (w_done >= L::kW) {
-                        /* the slot's unit before: waited for only when it is the next one needed */
-                        const uint32_t parity = (uint32_t)(w_done / L::kW - 1) & 1u;
-                        if (w_done > i) {
-                            if (!mbar_test_wait(&sm->w_empty[slot], parity)) break;
-                        } else if (!st_wait(&sm->w_empty[slot], parity, abort_flag)) {
-                            st_give_up(sm, P.status, ST_ST_STAGE_EMPTY);
-                            ok = false;
-                            break;
-                        }
-                    }
-                    w_copy(slot, w_block, w_unit);
-                    if (++w_unit == U) { w_unit = 0; ++w_block; }
-                }
-                if (!ok) break;
-                if (i == 0) griddep_wait();
-                const uint8_t *from = P.xt + (size_t)(block % P.token_blocks) * G * L::kSlice;
-                for (int k = 0; k < 2; ++k, ++x_done) {
-                    const uint32_t slot = x_done % L::kX;
-                    if (x_done >= (uint32_t)L::kX && !st_wait(&sm->x_empty[slot], (x_done / L::kX - 1) & 1u, abort_flag)) {
-                        st_give_up(sm, P.status, ST_ST_STAGE_EMPTY);
-                        ok = false;
-                        break;
-                    }
-                    mbar_expect_tx(&sm->x_full[slot], L::kSlice);
-                    bulk_g2s(x_ring + (size_t)slot * L::kSlice, from + (size_t)min(2 * unit + k, G - 1) * L::kSlice, L::kSlice, &sm->x_full[slot]);
+                    tma_load_2d(to, &P.wmap, unit * 128, rb * kTcRows, &sm->w_full[slot]);
                 }
                 if (++unit == U) { unit = 0; ++block; }
             }
             /* never leave with a copy in flight: wait (bounded) for the last fill of every slot */
             bool drained = true;
-            for (int f = w_done > L::kW ? w_done - L::kW : 0; f < w_done; ++f) {
+            for (int f = i > L::kW ? i - L::kW : 0; f < i; ++f) {
                 bool done = false;
                 for (uint32_t q = 0; q < kSpinLimit && !done; ++q) done = mbar_try_wait(&sm->w_full[f % L::kW], (uint32_t)(f / L::kW) & 1u);
-                drained = drained && done;
-            }
-            for (uint32_t f = x_done > (uint32_t)L::kX ? x_done - L::kX : 0u; f < x_done; ++f) {
-                bool done = false;
-                for (uint32_t q = 0; q < kSpinLimit && !done; ++q) done = mbar_try_wait(&sm->x_full[f % L::kX], (f / L::kX) & 1u);
                 drained = drained && done;
             }
             if (!drained) atomicCAS(P.status, 0u, (unsigned)ST_DRAIN | ((unsigned)blockIdx.x << 8));
@@ -295,12 +286,12 @@ __global__ void __launch_bounds__(StPlan<NP>::kThreads, 1) stream_tc_kernel(cons
             for (int k = 0; k < 2; ++k, ++d_used, a.next(L::kA), d.next(L::kD), x.next(L::kX)) {
                 if (turn-- != 0) continue;
                 turn = L::kMmaWarps - 1;
-                ok = st_warp_wait(&sm->x_full[x.slot], x.phase, abort_flag);
-                if (!ok) { if (lane == 0) st_give_up(sm, P.status, ST_ST_STAGE_FULL); break; }
                 if (d_used >= (uint32_t)L::kD) {
                     ok = st_warp_wait(&sm->d_empty[d.slot], d.phase ^ 1u, abort_flag);
                     if (!ok) { if (lane == 0) st_give_up(sm, P.status, ST_ST_D_EMPTY); break; }
                 }
+                ok = st_warp_wait(&sm->x_full[x.slot], x.phase, abort_flag);
+                if (!ok) { if (lane == 0) st_give_up(sm, P.status, ST_ST_STAGE_FULL); break; }
                 ok = st_warp_wait(&sm->a_ready[a.slot], a.phase, abort_flag);
                 if (!ok) { if (lane == 0) st_give_up(sm, P.status, ST_ST_A_READY); break; }
                 tc_fence_after();
@@ -310,9 +301,7 @@ __global__ void __launch_bounds__(StPlan<NP>::kThreads, 1) stream_tc_kernel(cons
 #pragma unroll
                     for (int q = 0; q < FFN_INT4_GROUP / 16; ++q)
                         tc_mma_ts(dcol, acol + (uint32_t)(q * 8), bdesc + (uint64_t)(((q >> 2) * NP * 128 + (q & 3) * 32) >> 4), idesc, q > 0 ? 1u : 0u);
-                    tc_commit(&sm->x_empty[x.slot]);
-                    tc_commit(&sm->a_empty[a.slot]);
-                    tc_commit(&sm->d_full[d.slot]);
+                    tc_commit(&sm->done[a.slot]);
                 }
                 __syncwarp();
             }
@@ -325,6 +314,9 @@ __global__ void __launch_bounds__(StPlan<NP>::kThreads, 1) stream_tc_kernel(cons
         const int row = PAIRS ? q4 * 16 + (lane & 15) + (lane >> 4) * 64 : q4 * 32 + lane;
         const uint32_t a_lane = tmem + ((uint32_t)(q4 * 32) << 16) + (uint32_t)L::kAFirst;
         uint32_t round = 0;
+        int x_last[2] = {-1, -1};
+        int x_block = block, x_unit = unit + (int)team + L::kX / 2; /* of the unit whose activations are asked for next */
+        while (x_unit >= U) { x_unit -= U; ++x_block; }
         bool ok = true;
         for (int i = (int)team; i < count && ok; i += L::kConvTeams, ++round) {
             const uint32_t slot = (uint32_t)i % L::kW;
@@ -338,9 +330,16 @@ __global__ void __launch_bounds__(StPlan<NP>::kThreads, 1) stream_tc_kernel(cons
 #pragma unroll
                 for (int q = 0; q < 4; ++q) packed[q] = lds16_at(src + (uint32_t)(((k * 4 + q) ^ (row & 7)) << 4));
                 if (round > 0) {
-                    ok = st_warp_wait(&sm->a_empty[mine], (round - 1u) & 1u, abort_flag);
+                    ok = st_warp_wait(&sm->done[mine], (round - 1u) & 1u, abort_flag);
                     if (!ok) { if (lane == 0) st_give_up(sm, P.status, ST_ST_A_EMPTY); break; }
                     tc_fence_after();
+                    /* the activations' slot of the team's unit before is free as well */
+                    const int next = i + L::kX / 2 - L::kConvTeams;
+                    if (q4 == 0 && next < count && elect_one()) { x_copy((uint32_t)(2 * next + k), x_block, x_unit, k); x_last[k] = next; }
+                    if (k == 1) {
+                        x_unit += L::kConvTeams;
+                        while (x_unit >= U) { x_unit -= U; ++x_block; }
+                    }
                 }
 #pragma unroll
                 for (int q = 0; q < 4; ++q) {
@@ -356,6 +355,16 @@ __global__ void __launch_bounds__(StPlan<NP>::kThreads, 1) stream_tc_kernel(cons
                     if (k == 1) mbar_arrive(&sm->w_empty[slot]);
                 }
             }
+        }
+        if (!ok && q4 == 0) {
+            /* given up: never leave with a copy in flight (those that the MMAs have not waited for) */
+#pragma unroll
+            for (int k = 0; k < 2; ++k)
+                if (x_last[k] >= 0) {
+                    const uint32_t v = (uint32_t)(2 * x_last[k] + k);
+                    for (uint32_t q = 0; q < kSpinLimit; ++q)
+                        if (mbar_try_wait(&sm->x_full[v % L::kX], (v / L::kX) & 1u)) break;
+                }
         }
     } else {
         /* ---------------- epilogue ---------------- */
@@ -385,7 +394,7 @@ __global__ void __launch_bounds__(StPlan<NP>::kThreads, 1) stream_tc_kernel(cons
         float acc[HALF];
 #pragma unroll
         for (int c = 0; c < HALF; ++c) acc[c] = 0.0f;
-        StRing d;
+        StRing d, a;
         bool ok = true;
         for (int i0 = 0; i0 < count && ok; i0 += 2) {
 #pragma unroll
@@ -396,7 +405,7 @@ __global__ void __launch_bounds__(StPlan<NP>::kThreads, 1) stream_tc_kernel(cons
                 fetch(sc[par]);
 #pragma unroll
                 for (int k = 0; k < 2; ++k) {
-                    ok = st_warp_wait(&sm->d_full[d.slot], d.phase, abort_flag); /* tcgen05.ld is warp-wide: the warp goes on together or not at all */
+                    ok = st_warp_wait(&sm->done[a.slot], a.phase, abort_flag); /* tcgen05.ld is warp-wide: the warp goes on together or not at all */
                     if (!ok) { if (lane == 0) st_give_up(sm, P.status, ST_ST_D_FULL); break; }
                     tc_fence_after();
                     if (2 * unit + k < G) /* an odd tail's second group is zeros times the first one's activations: not added */
@@ -413,7 +422,7 @@ __global__ void __launch_bounds__(StPlan<NP>::kThreads, 1) stream_tc_kernel(cons
                     tc_fence_before();
                     __syncwarp();
                     if (lane == 0) mbar_arrive(&sm->d_empty[d.slot]);
-                    d.next(L::kD);
+                    d.next(L::kD); a.next(L::kA);
                 }
                 if (!ok) break;
                 if (++unit == U || i + 1 == count) {
