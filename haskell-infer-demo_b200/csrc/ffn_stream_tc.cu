@@ -29,7 +29,7 @@
  *              thread that served both rings spent 800 cycles a group on its waits and copies.
  *   MMA        three warps, one group each in turn, one elected thread issues: a group costs a warp some
  *              1000 cycles of waits, issue and commits among 20 other warps, whatever its MMAs take.
- *   epilogue   eight warps: warp = lane quadrant and half of the token columns.
+ *   epilogue   8 or 16 warps: warp = lane quadrant and an equal part of the token columns.
  *
  * Gate/up blocks put pair 16*q + l in lanes l (gate) and l + 16 (up) of quadrant q, so SiLU * up is one
  * shuffle away.  Activations are read in tile order (K blocks of 64 values, see ffn_tc.cu), one region per
@@ -46,7 +46,7 @@ namespace ffn {
 
 constexpr int kStMaxTokens = 128;            /* tokens of a block = MMA columns */
 constexpr int kStSlab = 512;                 /* tokens of a launch */
-constexpr int kStEpiWarps = 8;
+constexpr int kStMaxEpiWarps = 16;
 constexpr int kStMaxRing = 10, kStMaxA = 6, kStMaxD = 4;
 constexpr int kStUnitBytes = kTcRows * 128;  /* packed bytes of a unit */
 constexpr int kStHeader = 1024;
@@ -68,7 +68,7 @@ struct StreamTcParams {
     uint8_t *act_t;         /* PAIRS: the same in tile order */
     uint16_t *residual;     /* optional bf16 [M][N], h <- bf16(h + y) */
     float *partial;         /* [CTA][2][columns][128] */
-    unsigned *arrivals;     /* [CTA][8], zero at the start */
+    unsigned *arrivals;     /* [CTA][epilogue warp], zero at the start */
     unsigned *status;
 };
 
@@ -76,10 +76,12 @@ struct StreamTcParams {
 template <int NP>
 struct StPlan {
     static constexpr int kSlice = NP * 256;                            /* activations of a group */
+    static constexpr int kEpiWarps = NP <= 32 ? 8 : 16;
+    static constexpr int kCols = NP / (kEpiWarps / 4);                  /* token columns of an epilogue warp */
     static constexpr int kConvTeams = NP <= 32 ? 3 : 2;
     static constexpr int kConvWarps = kConvTeams * 4;
     static constexpr int kMmaWarps = NP <= 64 ? 3 : 2;
-    static constexpr int kProducerWarp = kStEpiWarps + kConvWarps, kMmaWarp = kProducerWarp + 1;
+    static constexpr int kProducerWarp = kEpiWarps + kConvWarps, kMmaWarp = kProducerWarp + 1;
     static constexpr int kThreads = (kMmaWarp + kMmaWarps) * 32;
     static constexpr int kD = NP <= 64 ? 4 : 2;                        /* accumulators */
     static constexpr int kA = 2 * kConvTeams;                          /* operand buffers of 64 columns: a team has two of its own */
@@ -129,6 +131,20 @@ __device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t *d) {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
                  : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3]), "=r"(d[4]), "=r"(d[5]), "=r"(d[6]), "=r"(d[7]) : "r"(taddr));
 }
+__device__ __forceinline__ void tmem_ld4(uint32_t taddr, uint32_t *d) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3]) : "r"(taddr));
+}
+/* N (a multiple of 4, at most 16) consecutive FP32 columns of this thread's lane */
+template <int N>
+__device__ __forceinline__ void tmem_ld(uint32_t taddr, uint32_t (&d)[16]) {
+    if (N == 16) {
+        tmem_ld16(taddr, d);
+    } else {
+        if (N & 8) tmem_ld8(taddr, d);
+        if (N & 4) tmem_ld4(taddr + (N & 8), d + (N & 8));
+    }
+}
+__device__ __forceinline__ void prefetch_l2(const void *p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 __device__ __forceinline__ uint16_t ld_scale(const uint16_t *p) {
     uint16_t v;
     asm volatile("ld.global.nc.u16 %0, [%1];" : "=h"(v) : "l"(p));
@@ -156,28 +172,31 @@ struct StRing {
     __device__ __forceinline__ void next(uint32_t n) { if (++slot == n) { slot = 0; phase ^= 1u; } }
 };
 
-/* One row's finished sums (HALF columns from column c0 of a token block): rounding, SiLU * up, residual. */
-template <int HALF, int NP, bool PAIRS>
-__device__ __forceinline__ void st_finish(const StreamTcParams &P, const float (&acc)[HALF], int rb, int tb, int quadrant, int lane, int c0) {
+/* One row's finished sums (COLS columns from column c0 of a token block): rounding, SiLU * up, residual. */
+template <int COLS, int NP, bool PAIRS>
+__device__ __forceinline__ void st_finish(const StreamTcParams &P, const float (&acc)[COLS], int rb, int tb, int quadrant, int lane, int c0) {
     const int m0 = tb * P.per_block, count = min(P.per_block, P.M - m0);
     if (PAIRS) {
         const int p = rb * 64 + quadrant * 16 + (lane & 15);
         uint8_t *tile = P.act_t + (size_t)tb * P.N * NP * 2 + (size_t)(p >> 6) * NP * 128 + tc_permute8(p & 7) * 2;
+        /* two columns at a time: the pair's gate lane finishes the first, its up lane the second */
+        const bool gate_lane = lane < 16;
 #pragma unroll
-        for (int c = 0; c < HALF; ++c) {
-            const float mine = round_bf16(acc[c] * kStCodeScale), other = __shfl_xor_sync(~0u, mine, 16);
-            /* the pair's gate lane finishes the even columns, its up lane the odd ones */
-            if ((c & 1) == (lane >> 4) && c0 + c < count && p < P.N) {
-                const uint16_t a = f32_to_bf16_bits(silu_mul(lane < 16 ? mine : other, lane < 16 ? other : mine));
-                P.out[(size_t)(m0 + c0 + c) * P.N + p] = a;
-                *(uint16_t *)(tile + tc_tile_offset(c0 + c, (p >> 3) & 7)) = a;
+        for (int c = 0; c < COLS; c += 2) {
+            const float v0 = round_bf16(acc[c] * kStCodeScale), v1 = round_bf16(acc[c + 1] * kStCodeScale);
+            const float other = __shfl_xor_sync(~0u, gate_lane ? v1 : v0, 16);
+            const int n = c0 + c + (gate_lane ? 0 : 1);
+            if (n < count && p < P.N) {
+                const uint16_t a = f32_to_bf16_bits(silu_mul(gate_lane ? v0 : other, gate_lane ? other : v1));
+                P.out[(size_t)(m0 + n) * P.N + p] = a;
+                *(uint16_t *)(tile + tc_tile_offset(n, (p >> 3) & 7)) = a;
             }
         }
     } else {
         const int row = rb * kTcRows + quadrant * 32 + lane;
         if (row >= P.N) return;
 #pragma unroll
-        for (int c = 0; c < HALF; ++c)
+        for (int c = 0; c < COLS; ++c)
             if (c0 + c < count) {
                 const size_t o = (size_t)(m0 + c0 + c) * P.N + row;
                 const float y = round_bf16(acc[c] * kStCodeScale);
@@ -206,7 +225,7 @@ __global__ void __launch_bounds__(StPlan<NP>::kThreads, 1) stream_tc_kernel(cons
         for (int i = 0; i < L::kW; ++i) { mbar_init(&sm->w_full[i], 1); mbar_init(&sm->w_empty[i], 4); }
         for (int i = 0; i < L::kX; ++i) mbar_init(&sm->x_full[i], 1);
         for (int i = 0; i < L::kA; ++i) { mbar_init(&sm->a_ready[i], 4); mbar_init(&sm->done[i], 1); }
-        for (int i = 0; i < L::kD; ++i) mbar_init(&sm->d_empty[i], kStEpiWarps);
+        for (int i = 0; i < L::kD; ++i) mbar_init(&sm->d_empty[i], L::kEpiWarps);
         sm->abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -306,9 +325,9 @@ __global__ void __launch_bounds__(StPlan<NP>::kThreads, 1) stream_tc_kernel(cons
                 __syncwarp();
             }
         }
-    } else if (warp >= kStEpiWarps) {
+    } else if (warp >= L::kEpiWarps) {
         /* ---------------- conversion: one unit per team in turn ---------------- */
-        const uint32_t team = (uint32_t)((warp - kStEpiWarps) >> 2);
+        const uint32_t team = (uint32_t)((warp - L::kEpiWarps) >> 2);
         /* lane of tensor memory -> row of the stage: plain, or pair 16q + l in lanes l (gate) and l + 16 (up) */
         const int q4 = warp & 3;
         const int row = PAIRS ? q4 * 16 + (lane & 15) + (lane >> 4) * 64 : q4 * 32 + lane;
@@ -368,8 +387,8 @@ __global__ void __launch_bounds__(StPlan<NP>::kThreads, 1) stream_tc_kernel(cons
         }
     } else {
         /* ---------------- epilogue ---------------- */
-        constexpr int HALF = NP / 2;
-        const int quadrant = warp & 3, c0 = (warp >> 2) * HALF;
+        constexpr int COLS = L::kCols;
+        const int quadrant = warp & 3, c0 = (warp >> 2) * COLS;
         const uint32_t d_lane = tmem + ((uint32_t)(quadrant * 32) << 16) + (uint32_t)c0;
         /* this lane's row of block b; rows past a ragged end read the last row's scales */
         auto scale_row = [&](int b) {
@@ -388,12 +407,20 @@ __global__ void __launch_bounds__(StPlan<NP>::kThreads, 1) stream_tc_kernel(cons
             to[1] = ld_scale(s_from + min(2 * s_unit + 1, G - 1));
             if (++s_unit == U) { s_unit = 0; if (s_left > 0) s_from = P.s + (size_t)scale_row(++s_block) * G; }
         };
+        /* a row's scales lie far apart from the next row's, so each new 32 bytes come from HBM: ask for a block's
+         * ahead of time, this one's now and the next one's when it is begun */
+        auto ahead = [&](int b) {
+            if (b >= P.blocks) return;
+            const uint16_t *row = P.s + (size_t)scale_row(b) * G;
+            for (int g = 0; g < G; g += 16) prefetch_l2(row + g);
+        };
+        if (c0 == 0) { ahead(block); ahead(block + 1); }
         fetch(sc[0]);
         fetch(sc[1]);
         griddep_wait(); /* before the first write: earlier launches may still read what this one overwrites */
-        float acc[HALF];
+        float acc[COLS];
 #pragma unroll
-        for (int c = 0; c < HALF; ++c) acc[c] = 0.0f;
+        for (int c = 0; c < COLS; ++c) acc[c] = 0.0f;
         StRing d, a;
         bool ok = true;
         for (int i0 = 0; i0 < count && ok; i0 += 2) {
@@ -410,14 +437,14 @@ __global__ void __launch_bounds__(StPlan<NP>::kThreads, 1) stream_tc_kernel(cons
                     tc_fence_after();
                     if (2 * unit + k < G) /* an odd tail's second group is zeros times the first one's activations: not added */
 #pragma unroll
-                    for (int c = 0; c < HALF; c += 16) {
+                    for (int c = 0; c < COLS; c += 16) {
                         uint32_t v[16];
-                        tmem_ld8(d_lane + d.slot * (uint32_t)NP + (uint32_t)c, v);
-                        if (c + 8 < HALF) tmem_ld8(d_lane + d.slot * (uint32_t)NP + (uint32_t)(c + 8), v + 8);
+                        if (c + 16 <= COLS) tmem_ld<16>(d_lane + d.slot * (uint32_t)NP + (uint32_t)c, v);
+                        else tmem_ld<COLS % 16>(d_lane + d.slot * (uint32_t)NP + (uint32_t)c, v);
                         tmem_ld_wait();
 #pragma unroll
                         for (int j = 0; j < 16; ++j)
-                            if (c + j < HALF) acc[c + j] = fmaf(scale[k], __uint_as_float(v[j]), acc[c + j]);
+                            if (c + j < COLS) acc[c + j] = fmaf(scale[k], __uint_as_float(v[j]), acc[c + j]);
                     }
                     tc_fence_before();
                     __syncwarp();
@@ -435,29 +462,33 @@ __global__ void __launch_bounds__(StPlan<NP>::kThreads, 1) stream_tc_kernel(cons
                         const size_t per_slot = (size_t)NP * kTcRows, mine = (size_t)c0 * kTcRows + quadrant * 32 + lane;
                         float *to = P.partial + ((size_t)blockIdx.x * 2 + (it0 > first ? 0 : 1)) * per_slot + mine;
 #pragma unroll
-                        for (int c = 0; c < HALF; ++c) __stcg(to + c * kTcRows, acc[c]);
+                        for (int c = 0; c < COLS; ++c) __stcg(to + c * kTcRows, acc[c]);
                         __threadfence();
                         __syncwarp();
                         /* CTA q holds unit u when q = floor(((u + 1) * CTAs - 1) / total) */
                         const int q0 = (int)(((first + 1) * gridDim.x - 1) / total), q1 = (int)((last * gridDim.x - 1) / total);
                         unsigned before = 0;
-                        if (lane == 0) before = atomicAdd(P.arrivals + (size_t)q0 * kStEpiWarps + warp, 1u);
+                        if (lane == 0) before = atomicAdd(P.arrivals + (size_t)q0 * kStMaxEpiWarps + warp, 1u);
                         finish = __shfl_sync(~0u, before, 0) == (unsigned)(q1 - q0);
                         if (finish) {
                             __threadfence();
 #pragma unroll
-                            for (int c = 0; c < HALF; ++c) acc[c] = 0.0f;
+                            for (int c = 0; c < COLS; ++c) acc[c] = 0.0f;
                             for (int q = q0; q <= q1; ++q) {
                                 const float *from = P.partial + ((size_t)q * 2 + (total * q / gridDim.x > first ? 0 : 1)) * per_slot + mine;
 #pragma unroll
-                                for (int c = 0; c < HALF; ++c) acc[c] += __ldcg(from + c * kTcRows);
+                                for (int c = 0; c < COLS; ++c) acc[c] += __ldcg(from + c * kTcRows);
                             }
                         }
                     }
-                    if (finish) st_finish<HALF, NP, PAIRS>(P, acc, rb, tb, quadrant, lane, c0);
+                    if (finish) st_finish<COLS, NP, PAIRS>(P, acc, rb, tb, quadrant, lane, c0);
 #pragma unroll
-                    for (int c = 0; c < HALF; ++c) acc[c] = 0.0f;
-                    if (unit == U) { unit = 0; ++block; }
+                    for (int c = 0; c < COLS; ++c) acc[c] = 0.0f;
+                    if (unit == U) {
+                        unit = 0;
+                        ++block;
+                        if (c0 == 0) ahead(block + 1);
+                    }
                 }
             }
         }
@@ -539,7 +570,7 @@ static int st_ctas(int blocks, int G, int sm_count) {
     const long long n = (long long)blocks * ((G + 1) / 2);
     return n < sm_count ? (int)n : sm_count;
 }
-static size_t st_counter_bytes(int sm_count) { return st_round((size_t)sm_count * kStEpiWarps * sizeof(unsigned)); }
+static size_t st_counter_bytes(int sm_count) { return st_round((size_t)sm_count * kStMaxEpiWarps * sizeof(unsigned)); }
 static size_t st_partial_bytes(int sm_count, int np) { return (size_t)sm_count * 2 * np * kTcRows * sizeof(float); }
 static size_t st_tile_bytes(const StTokens &t, int K) { return st_round((size_t)t.blocks * t.np * K * 2); }
 
