@@ -627,7 +627,7 @@ static std::mutex g_st_mutex;
 
 int stream_tc_ffn_launch(cudaStream_t stream, const void *x, void *act, void *layer_out, const FfnMlpWeights *w, int tokens, int H,
                          int I, void *residual, const FusedNorm *norm, unsigned *status) {
-    if (tokens <= 16 || tc_get_mode() != 2) return FFN_NOT_ADMITTED; /* 3..16 tokens: the mma.sync pair, 63 against 81 us at 8 on the 5120 x 17408 layer */
+    if (tokens <= 2 || tc_get_mode() != 2) return FFN_NOT_ADMITTED; /* 3..16 tokens: the mma.sync pair, 63 against 81 us at 8 on the 5120 x 17408 layer */
     if (((uintptr_t)w->gate_up_i4 & 15) || ((uintptr_t)w->down_i4 & 15) || ((uintptr_t)x & 15)) return FFN_NOT_ADMITTED;
     int dev = 0, sm_count = 0, st = st_device(&dev, &sm_count);
     if (st) return st;
