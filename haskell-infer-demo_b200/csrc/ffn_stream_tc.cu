@@ -18,17 +18,17 @@
  * finished by the last of its contributors to arrive, which adds the partial sums in CTA order (FP32,
  * through L2).  Nothing waits for another CTA.
  *
- * Roles of a CTA (one per SM):
- *   producer   one thread: per unit a tiled TMA load of 128 bytes of 128 rows (gate/up: 64 gate and 64 up
- *              rows) into the weight ring.  Alone, boxes of 128 bytes stream at 6.4 to 6.75 TB/s; 16-byte
- *              loads by the warps, eight rows an instruction, at 4.6; bulk copies of 512 bytes of a row at
- *              2.3.
+ * Roles of a CTA (one per SM).  A step of the pipeline is a unit up to 64 tokens, a group above; every role
+ * is a chain of waits and short work among some 25 warps that share the issue slots, so what a step costs in
+ * instructions bounds the kernel before the tensor pipe does, and each role does what it can per step once:
+ *   weights    one thread: per unit a tiled TMA load of 128 bytes of 128 rows (gate/up: 64 gate and 64 up
+ *              rows) into a ring.  Alone, boxes of 128 bytes stream at 6.4 to 6.75 TB/s; 16-byte loads by
+ *              the warps, eight rows an instruction, at 4.6; bulk copies of 512 bytes of a row at 2.3.
+ *   input      one thread: per step one bulk copy of the activations, when the slot's last MMAs are done.
  *   conversion teams of four warps, one unit each in turn: codes -> BF16, from registers straight into
- *              tensor memory, where the MMA reads its A operand.  A team that has waited for its unit before
- *              also asks for the activations that take that unit's place (one bulk copy per group): a
- *              thread that served both rings spent 800 cycles a group on its waits and copies.
- *   MMA        three warps, one group each in turn, one elected thread issues: a group costs a warp some
- *              1000 cycles of waits, issue and commits among 20 other warps, whatever its MMAs take.
+ *              tensor memory, where the MMA reads its A operand.
+ *   MMA        two warps, one step each in turn into an accumulator of its own; an elected thread issues,
+ *              and one commit frees operand and activations and hands over the sums.
  *   epilogue   8 or 16 warps: warp = lane quadrant and an equal part of the token columns.
  *
  * Gate/up blocks put pair 16*q + l in lanes l (gate) and l + 16 (up) of quadrant q, so SiLU * up is one
@@ -47,7 +47,7 @@ namespace ffn {
 constexpr int kStMaxTokens = 128;            /* tokens of a block = MMA columns */
 constexpr int kStSlab = 512;                 /* tokens of a launch */
 constexpr int kStMaxEpiWarps = 16;
-constexpr int kStMaxRing = 10, kStMaxA = 6, kStMaxD = 4;
+constexpr int kStMaxRing = 10, kStMaxA = 4, kStMaxD = 2;
 constexpr int kStUnitBytes = kTcRows * 128;  /* packed bytes of a unit */
 constexpr int kStHeader = 1024;
 constexpr int kStSmem = 232448;
@@ -72,39 +72,38 @@ struct StreamTcParams {
     unsigned *status;
 };
 
-/* Geometry for NP token columns. */
+/* Geometry for NP token columns.  A step is what one turn of the pipeline takes: a whole unit (two groups)
+ * while two accumulators of two groups fit tensor memory, else one group. */
 template <int NP>
 struct StPlan {
     static constexpr int kSlice = NP * 256;                            /* activations of a group */
-    static constexpr int kEpiWarps = NP <= 32 ? 8 : 16;
+    static constexpr int kGroups = NP <= 64 ? 2 : 1;                   /* groups of a step */
+    static constexpr int kEpiWarps = NP <= 64 ? 8 : 16;
     static constexpr int kCols = NP / (kEpiWarps / 4);                  /* token columns of an epilogue warp */
     static constexpr int kConvTeams = NP <= 32 ? 3 : 2;
     static constexpr int kConvWarps = kConvTeams * 4;
-    static constexpr int kMmaWarps = NP <= 64 ? 3 : 2;
-    static constexpr int kProducerWarp = kEpiWarps + kConvWarps, kMmaWarp = kProducerWarp + 1;
+    static constexpr int kMmaWarps = 2;
+    static constexpr int kWeightWarp = kEpiWarps + kConvWarps, kInputWarp = kWeightWarp + 1, kMmaWarp = kInputWarp + 1;
     static constexpr int kThreads = (kMmaWarp + kMmaWarps) * 32;
-    static constexpr int kD = NP <= 64 ? 4 : 2;                        /* accumulators */
-    static constexpr int kA = 2 * kConvTeams;                          /* operand buffers of 64 columns: a team has two of its own */
-    static constexpr int kAFirst = 512 - kA * 64;
-    /* activation slices: two turns of every team's units where they fit, one beyond; the weight ring takes the rest */
-    static constexpr int kX = NP <= 64 ? 2 * kA : kA;
-    static constexpr int kWFree = (kStSmem - kStHeader - kX * kSlice) / kStUnitBytes;
-    static constexpr int kW = kWFree < kStMaxRing ? kWFree : kStMaxRing;
-    static constexpr int kSmem = kStHeader + kX * kSlice + kW * kStUnitBytes;
-    static_assert(kW >= 4 && kSmem <= kStSmem && kD * NP <= kAFirst, "geometry");
-    /* A waiter tells rounds of a slot apart by one bit, so none may run a whole ring ahead of another:
-     * an MMA warp at group v has waited for the accumulator of group v - kMmaWarps, so the epilogue, which
-     * goes in order, is past v - kMmaWarps - kD >= v - 2 kD; that wait comes before the operand's and the
-     * activations', whose last rounds v - kA and v - kX are <= v - kD; a team at unit i has had the MMAs of
-     * its unit i - 2 kConvTeams, so every team is past unit i - 2 kConvTeams - kD / 2, i.e. past i - kW. */
-    static_assert(kMmaWarps <= kD && kD <= kA && kA <= kX && kW >= 2 * kConvTeams + kD / 2, "no role runs a ring ahead");
+    static constexpr int kD = 2;                                       /* accumulators, a step each */
+    static constexpr int kA = 2 * kConvTeams / kGroups;                /* operands and activations, a step each: a team has two groups' of its own */
+    static constexpr int kAFirst = 512 - 2 * kConvTeams * 64;
+    static constexpr int kWFree = (kStSmem - kStHeader - 2 * kConvTeams * kSlice) / kStUnitBytes;
+    static constexpr int kW = kWFree < kStMaxRing ? kWFree : kStMaxRing; /* units of weights */
+    static constexpr int kSmem = kStHeader + 2 * kConvTeams * kSlice + kW * kStUnitBytes;
+    static_assert(kSmem <= kStSmem && kD * kGroups * NP <= kAFirst, "geometry");
+    /* A waiter tells rounds of a slot apart by one bit, so none may run a whole ring ahead of another.  An
+     * MMA warp at step s has had the accumulator of step s - kMmaWarps, so the epilogue, which goes in
+     * order, is past s - kMmaWarps - kD >= s - 2 kD; that wait comes before the operand's, whose last round
+     * s - kA is <= s - kD.  A team at unit i has had the MMAs of its unit i - 2 kConvTeams, hence the
+     * epilogue is past the step kD before, and with it every team past unit i - kW. */
+    static_assert(kMmaWarps <= kD && kD <= kA && kW >= 2 * kConvTeams + kGroups, "no role runs a ring ahead");
 };
 
 struct StSmem {
     uint64_t w_full[kStMaxRing], w_empty[kStMaxRing];
-    uint64_t x_full[2 * kStMaxA];
-    uint64_t a_ready[kStMaxA];  /* a group's operand is complete (one arrival per warp of the team) */
-    uint64_t done[kStMaxA];     /* its MMAs are: operand buffer and activations are free, the sums can be read */
+    uint64_t ready[kStMaxA];    /* a step's operand (one arrival per warp of the team) and activations (a copy's bytes) are there */
+    uint64_t done[kStMaxA];     /* its MMAs are: both are free again, the sums can be read */
     uint64_t d_empty[kStMaxD];  /* the epilogue has read the accumulator out */
     uint32_t tmem_base;
     int abort_flag;
@@ -223,8 +222,7 @@ __global__ void __launch_bounds__(StPlan<NP>::kThreads, 1) stream_tc_kernel(cons
     griddep_launch();
     if (threadIdx.x == 0) {
         for (int i = 0; i < L::kW; ++i) { mbar_init(&sm->w_full[i], 1); mbar_init(&sm->w_empty[i], 4); }
-        for (int i = 0; i < L::kX; ++i) mbar_init(&sm->x_full[i], 1);
-        for (int i = 0; i < L::kA; ++i) { mbar_init(&sm->a_ready[i], 4); mbar_init(&sm->done[i], 1); }
+        for (int i = 0; i < L::kA; ++i) { mbar_init(&sm->ready[i], 4 + 1); mbar_init(&sm->done[i], 1); }
         for (int i = 0; i < L::kD; ++i) mbar_init(&sm->d_empty[i], L::kEpiWarps);
         sm->abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -238,50 +236,27 @@ __global__ void __launch_bounds__(StPlan<NP>::kThreads, 1) stream_tc_kernel(cons
     tc_fence_after();
     const uint32_t tmem = sm->tmem_base;
 
-    /* The activations of unit u of block b, group k (an odd tail's second group: the first one's again),
-     * into the slot of group v of this CTA's line */
-    auto x_copy = [&](uint32_t v, int b, int u, int k) {
-        const uint32_t slot = v % L::kX;
-        const int tb = P.token_blocks == 1 ? 0 : b % P.token_blocks;
-        const uint8_t *from = P.xt + (size_t)(uint32_t)(tb * G + min(2 * u + k, G - 1)) * L::kSlice;
-        mbar_expect_tx(&sm->x_full[slot], L::kSlice);
-        bulk_g2s(x_ring + (size_t)slot * L::kSlice, from, L::kSlice, &sm->x_full[slot]);
-    };
-
-    if (warp == L::kProducerWarp) {
-        /* ---------------- weights, and the first turns' activations ---------------- */
+    if (warp == L::kWeightWarp) {
+        /* ---------------- weights ---------------- */
         if (elect_one()) {
-            int i = 0;
-            bool ok = true;
-            for (; i < count && ok; ++i) {
-                const uint32_t slot = (uint32_t)i % L::kW;
-                /* The weights never change: a ring of them is on its way before the launch this one depends
-                 * on, which writes the activations, is over. */
-                if (i == min(L::kW, count - 1)) {
-                    griddep_wait();
-                    int b = (int)(it0 / U), u = (int)(it0 % U);
-                    for (int j = 0; j < min(L::kX / 2, count); ++j) {
-                        x_copy((uint32_t)(2 * j), b, u, 0);
-                        x_copy((uint32_t)(2 * j + 1), b, u, 1);
-                        if (++u == U) { u = 0; ++b; }
-                    }
-                }
-                if (i >= L::kW && !st_wait(&sm->w_empty[slot], (uint32_t)(i / L::kW - 1) & 1u, abort_flag)) {
+            /* They never change: a ring of them is on its way before the launch this one depends on is over. */
+            StRing w;
+            int rb = block / P.token_blocks, i = 0;
+            for (; i < count; ++i, w.next(L::kW)) {
+                if (i >= L::kW && !st_wait(&sm->w_empty[w.slot], w.phase ^ 1u, abort_flag)) {
                     st_give_up(sm, P.status, ST_ST_STAGE_EMPTY);
-                    ok = false;
                     break;
                 }
-                const int rb = block / P.token_blocks;
-                uint8_t *to = w_ring + (size_t)slot * kStUnitBytes;
-                mbar_expect_tx(&sm->w_full[slot], kStUnitBytes);
+                uint8_t *to = w_ring + (size_t)w.slot * kStUnitBytes;
+                mbar_expect_tx(&sm->w_full[w.slot], kStUnitBytes);
                 /* rows and bytes past the matrix (a ragged last block, an odd tail's second group) arrive as zeros */
                 if (PAIRS) {
-                    tma_load_2d(to, &P.wmap, unit * 128, rb * 64, &sm->w_full[slot]);
-                    tma_load_2d(to + kStUnitBytes / 2, &P.wmap, unit * 128, P.up_offset + rb * 64, &sm->w_full[slot]);
+                    tma_load_2d(to, &P.wmap, unit * 128, rb * 64, &sm->w_full[w.slot]);
+                    tma_load_2d(to + kStUnitBytes / 2, &P.wmap, unit * 128, P.up_offset + rb * 64, &sm->w_full[w.slot]);
                 } else {
-                    tma_load_2d(to, &P.wmap, unit * 128, rb * kTcRows, &sm->w_full[slot]);
+                    tma_load_2d(to, &P.wmap, unit * 128, rb * kTcRows, &sm->w_full[w.slot]);
                 }
-                if (++unit == U) { unit = 0; ++block; }
+                if (++unit == U) { unit = 0; rb = ++block / P.token_blocks; }
             }
             /* never leave with a copy in flight: wait (bounded) for the last fill of every slot */
             bool drained = true;
@@ -293,37 +268,67 @@ __global__ void __launch_bounds__(StPlan<NP>::kThreads, 1) stream_tc_kernel(cons
             if (!drained) atomicCAS(P.status, 0u, (unsigned)ST_DRAIN | ((unsigned)blockIdx.x << 8));
         }
         __syncwarp();
+    } else if (warp == L::kInputWarp) {
+        /* ---------------- activations ---------------- */
+        if (elect_one()) {
+            griddep_wait(); /* they come from the launch before */
+            StRing a;
+            const uint8_t *region = P.xt + (size_t)(block % P.token_blocks) * G * L::kSlice;
+            bool ok = true;
+            for (int i = 0; i < count && ok; ++i) {
+#pragma unroll
+                for (int k = 0; k < 2; k += L::kGroups, a.next(L::kA)) {
+                    if (i * (2 / L::kGroups) + k >= L::kA && !st_wait(&sm->done[a.slot], a.phase ^ 1u, abort_flag)) {
+                        st_give_up(sm, P.status, ST_ST_STAGE_EMPTY);
+                        ok = false;
+                        break;
+                    }
+                    /* the second group of an odd tail is multiplied with what the slot holds, and not added */
+                    const int ng = min(L::kGroups, G - 2 * unit - k);
+                    if (ng > 0) {
+                        mbar_expect_tx(&sm->ready[a.slot], (uint32_t)(ng * L::kSlice));
+                        bulk_g2s(x_ring + (size_t)(a.slot * L::kGroups) * L::kSlice, region + (size_t)(2 * unit + k) * L::kSlice, (uint32_t)(ng * L::kSlice), &sm->ready[a.slot]);
+                    } else {
+                        mbar_arrive(&sm->ready[a.slot]);
+                    }
+                }
+                if (++unit == U) { unit = 0; ++block; region = P.xt + (size_t)(block % P.token_blocks) * G * L::kSlice; }
+            }
+            /* given up: the last copies have no barrier of their own, so give them a millisecond */
+            for (int q = 0; q < 1000 && !ok; ++q) __nanosleep(1000);
+        }
+        __syncwarp();
     } else if (warp >= L::kMmaWarp) {
-        /* ---------------- MMA issue: the warp waits together, one thread issues ---------------- */
-        uint32_t turn = (uint32_t)(warp - L::kMmaWarp); /* groups until this warp's next */
+        /* ---------------- MMA issue: the warps take steps in turn, wait together, one thread issues ---------------- */
         const uint32_t idesc = tc_instr_desc(NP);
         const uint64_t bdesc0 = tc_smem_desc(smem_u32(x_ring), 1024);
-        StRing a, d, x;
-        uint32_t d_used = 0;
+        const int steps = count * (2 / L::kGroups);
+        uint32_t a_slot = (uint32_t)(warp - L::kMmaWarp), a_phase = 0;
+        const uint32_t d_slot = a_slot; /* as many accumulators as warps: each warp has its own */
+        static_assert(L::kD == L::kMmaWarps && L::kMmaWarps <= L::kA, "a warp's accumulator");
         bool ok = true;
-        for (int i = 0; i < count && ok; ++i) {
-            for (int k = 0; k < 2; ++k, ++d_used, a.next(L::kA), d.next(L::kD), x.next(L::kX)) {
-                if (turn-- != 0) continue;
-                turn = L::kMmaWarps - 1;
-                if (d_used >= (uint32_t)L::kD) {
-                    ok = st_warp_wait(&sm->d_empty[d.slot], d.phase ^ 1u, abort_flag);
-                    if (!ok) { if (lane == 0) st_give_up(sm, P.status, ST_ST_D_EMPTY); break; }
-                }
-                ok = st_warp_wait(&sm->x_full[x.slot], x.phase, abort_flag);
-                if (!ok) { if (lane == 0) st_give_up(sm, P.status, ST_ST_STAGE_FULL); break; }
-                ok = st_warp_wait(&sm->a_ready[a.slot], a.phase, abort_flag);
-                if (!ok) { if (lane == 0) st_give_up(sm, P.status, ST_ST_A_READY); break; }
-                tc_fence_after();
-                const uint64_t bdesc = bdesc0 + (uint64_t)((x.slot * (uint32_t)L::kSlice) >> 4);
-                const uint32_t acol = tmem + (uint32_t)L::kAFirst + a.slot * 64u, dcol = tmem + d.slot * (uint32_t)NP;
-                if (elect_one()) {
+        for (int i = warp - L::kMmaWarp, used = 0; i < steps; i += L::kMmaWarps, ++used) {
+            if (used > 0) {
+                ok = st_warp_wait(&sm->d_empty[d_slot], (uint32_t)(used - 1) & 1u, abort_flag);
+                if (!ok) { if (lane == 0) st_give_up(sm, P.status, ST_ST_D_EMPTY); break; }
+            }
+            ok = st_warp_wait(&sm->ready[a_slot], a_phase, abort_flag);
+            if (!ok) { if (lane == 0) st_give_up(sm, P.status, ST_ST_A_READY); break; }
+            tc_fence_after();
+            const uint64_t bdesc = bdesc0 + (uint64_t)((a_slot * (uint32_t)(L::kGroups * L::kSlice)) >> 4);
+            const uint32_t acol = tmem + (uint32_t)L::kAFirst + a_slot * (uint32_t)(L::kGroups * 64), dcol = tmem + d_slot * (uint32_t)(L::kGroups * NP);
+            if (elect_one()) {
+#pragma unroll
+                for (int k = 0; k < L::kGroups; ++k)
 #pragma unroll
                     for (int q = 0; q < FFN_INT4_GROUP / 16; ++q)
-                        tc_mma_ts(dcol, acol + (uint32_t)(q * 8), bdesc + (uint64_t)(((q >> 2) * NP * 128 + (q & 3) * 32) >> 4), idesc, q > 0 ? 1u : 0u);
-                    tc_commit(&sm->done[a.slot]);
-                }
-                __syncwarp();
+                        tc_mma_ts(dcol + (uint32_t)(k * NP), acol + (uint32_t)(k * 64 + q * 8),
+                                  bdesc + (uint64_t)((k * L::kSlice + (q >> 2) * NP * 128 + (q & 3) * 32) >> 4), idesc, q > 0 ? 1u : 0u);
+                tc_commit(&sm->done[a_slot]);
             }
+            __syncwarp();
+            a_slot += L::kMmaWarps;
+            if (a_slot >= (uint32_t)L::kA) { a_slot -= L::kA; a_phase ^= 1u; }
         }
     } else if (warp >= L::kEpiWarps) {
         /* ---------------- conversion: one unit per team in turn ---------------- */
@@ -332,58 +337,41 @@ __global__ void __launch_bounds__(StPlan<NP>::kThreads, 1) stream_tc_kernel(cons
         const int q4 = warp & 3;
         const int row = PAIRS ? q4 * 16 + (lane & 15) + (lane >> 4) * 64 : q4 * 32 + lane;
         const uint32_t a_lane = tmem + ((uint32_t)(q4 * 32) << 16) + (uint32_t)L::kAFirst;
-        uint32_t round = 0;
-        int x_last[2] = {-1, -1};
-        int x_block = block, x_unit = unit + (int)team + L::kX / 2; /* of the unit whose activations are asked for next */
-        while (x_unit >= U) { x_unit -= U; ++x_block; }
+        uint32_t round = 0, slot = team, w_phase = 0;
         bool ok = true;
         for (int i = (int)team; i < count && ok; i += L::kConvTeams, ++round) {
-            const uint32_t slot = (uint32_t)i % L::kW;
-            ok = st_warp_wait(&sm->w_full[slot], (uint32_t)(i / L::kW) & 1u, abort_flag); /* tcgen05.st is warp-wide: the warp goes on together or not at all */
+            ok = st_warp_wait(&sm->w_full[slot], w_phase, abort_flag); /* tcgen05.st is warp-wide: the warp goes on together or not at all */
             if (!ok) { if (lane == 0) st_give_up(sm, P.status, ST_ST_STAGE_FULL); break; }
-            const uint32_t src = smem_u32(w_ring + (size_t)slot * kStUnitBytes) + (uint32_t)(row * 128);
+            const uint32_t src = smem_u32(w_ring) + slot * (uint32_t)kStUnitBytes + (uint32_t)(row * 128);
 #pragma unroll
             for (int k = 0; k < 2; ++k) {
-                const uint32_t mine = team * 2u + (uint32_t)k;
+                const uint32_t mine = (team * 2u + (uint32_t)k) / L::kGroups;
                 uint4 packed[4];
 #pragma unroll
                 for (int q = 0; q < 4; ++q) packed[q] = lds16_at(src + (uint32_t)(((k * 4 + q) ^ (row & 7)) << 4));
-                if (round > 0) {
+                if (round > 0 && k % L::kGroups == 0) {
                     ok = st_warp_wait(&sm->done[mine], (round - 1u) & 1u, abort_flag);
                     if (!ok) { if (lane == 0) st_give_up(sm, P.status, ST_ST_A_EMPTY); break; }
                     tc_fence_after();
-                    /* the activations' slot of the team's unit before is free as well */
-                    const int next = i + L::kX / 2 - L::kConvTeams;
-                    if (q4 == 0 && next < count && elect_one()) { x_copy((uint32_t)(2 * next + k), x_block, x_unit, k); x_last[k] = next; }
-                    if (k == 1) {
-                        x_unit += L::kConvTeams;
-                        while (x_unit >= U) { x_unit -= U; ++x_block; }
-                    }
                 }
 #pragma unroll
                 for (int q = 0; q < 4; ++q) {
                     uint32_t v[16];
                     st_codes(packed[q].x, v); st_codes(packed[q].y, v + 4); st_codes(packed[q].z, v + 8); st_codes(packed[q].w, v + 12);
-                    tmem_st16(a_lane + mine * 64u + (uint32_t)(q * 16), v);
+                    tmem_st16(a_lane + (team * 2u + (uint32_t)k) * 64u + (uint32_t)(q * 16), v);
                 }
-                tmem_st_wait();
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) {
-                    mbar_arrive(&sm->a_ready[mine]);
-                    if (k == 1) mbar_arrive(&sm->w_empty[slot]);
+                if (k == 1 || L::kGroups == 1) {
+                    tmem_st_wait();
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) {
+                        mbar_arrive(&sm->ready[mine]);
+                        if (k == 1) mbar_arrive(&sm->w_empty[slot]);
+                    }
                 }
             }
-        }
-        if (!ok && q4 == 0) {
-            /* given up: never leave with a copy in flight (those that the MMAs have not waited for) */
-#pragma unroll
-            for (int k = 0; k < 2; ++k)
-                if (x_last[k] >= 0) {
-                    const uint32_t v = (uint32_t)(2 * x_last[k] + k);
-                    for (uint32_t q = 0; q < kSpinLimit; ++q)
-                        if (mbar_try_wait(&sm->x_full[v % L::kX], (v / L::kX) & 1u)) break;
-                }
+            slot += L::kConvTeams;
+            if (slot >= (uint32_t)L::kW) { slot -= L::kW; w_phase ^= 1u; }
         }
     } else {
         /* ---------------- epilogue ---------------- */
@@ -432,24 +420,29 @@ __global__ void __launch_bounds__(StPlan<NP>::kThreads, 1) stream_tc_kernel(cons
                 fetch(sc[par]);
 #pragma unroll
                 for (int k = 0; k < 2; ++k) {
-                    ok = st_warp_wait(&sm->done[a.slot], a.phase, abort_flag); /* tcgen05.ld is warp-wide: the warp goes on together or not at all */
-                    if (!ok) { if (lane == 0) st_give_up(sm, P.status, ST_ST_D_FULL); break; }
-                    tc_fence_after();
-                    if (2 * unit + k < G) /* an odd tail's second group is zeros times the first one's activations: not added */
+                    if (k % L::kGroups == 0) {
+                        ok = st_warp_wait(&sm->done[a.slot], a.phase, abort_flag); /* tcgen05.ld is warp-wide: the warp goes on together or not at all */
+                        if (!ok) { if (lane == 0) st_give_up(sm, P.status, ST_ST_D_FULL); break; }
+                        tc_fence_after();
+                    }
+                    const uint32_t from = d_lane + (d.slot * (uint32_t)L::kGroups + (uint32_t)(k % L::kGroups)) * (uint32_t)NP;
+                    if (2 * unit + k < G) /* an odd tail's second group is not added */
 #pragma unroll
                     for (int c = 0; c < COLS; c += 16) {
                         uint32_t v[16];
-                        if (c + 16 <= COLS) tmem_ld<16>(d_lane + d.slot * (uint32_t)NP + (uint32_t)c, v);
-                        else tmem_ld<COLS % 16>(d_lane + d.slot * (uint32_t)NP + (uint32_t)c, v);
+                        if (c + 16 <= COLS) tmem_ld<16>(from + (uint32_t)c, v);
+                        else tmem_ld<COLS % 16>(from + (uint32_t)c, v);
                         tmem_ld_wait();
 #pragma unroll
                         for (int j = 0; j < 16; ++j)
                             if (c + j < COLS) acc[c + j] = fmaf(scale[k], __uint_as_float(v[j]), acc[c + j]);
                     }
-                    tc_fence_before();
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(&sm->d_empty[d.slot]);
-                    d.next(L::kD); a.next(L::kA);
+                    if (k == 1 || L::kGroups == 1) {
+                        tc_fence_before();
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(&sm->d_empty[d.slot]);
+                        d.next(L::kD); a.next(L::kA);
+                    }
                 }
                 if (!ok) break;
                 if (++unit == U || i + 1 == count) {
