@@ -532,6 +532,7 @@ void fused_set_trace(long long *device_buffer) { g_trace = device_buffer; }
 long long *fused_get_trace() { return g_trace; }
 static std::mutex g_dev_mutex;
 static int g_launch_overlap = 1;
+bool fused_launch_overlap() { return g_launch_overlap != 0; }
 int fused_set_launch_overlap(int on) {
     const int old = g_launch_overlap;
     g_launch_overlap = on != 0;

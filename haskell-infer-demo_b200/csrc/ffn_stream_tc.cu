@@ -502,7 +502,8 @@ __global__ void __launch_bounds__(kTileThreads) stream_tile_input_kernel(uint8_t
                                                                         const uint16_t *__restrict__ norm_w, float eps, float gemma, int M,
                                                                         int per_block, int np, int K, unsigned *arrivals, int counters) {
     __shared__ float red[kTileThreads / 32];
-    griddep_launch();
+    griddep_wait();
+    griddep_launch(); /* only now: the launch that follows reads weights before its own wait, and what precedes this one may have written them */
     if (blockIdx.x == 0)
         for (int i = threadIdx.x; i < counters; i += kTileThreads) arrivals[i] = 0u;
     const int tb = blockIdx.x / np, n = blockIdx.x % np, m = tb * per_block + n;
@@ -576,7 +577,7 @@ static int st_launch(const StreamTcParams &P, int ctas, cudaStream_t stream) {
     attr.val.programmaticStreamSerializationAllowed = 1;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)ctas); cfg.blockDim = dim3(L::kThreads); cfg.dynamicSmemBytes = L::kSmem; cfg.stream = stream;
-    cfg.attrs = &attr; cfg.numAttrs = 1;
+    cfg.attrs = &attr; cfg.numAttrs = fused_launch_overlap() ? 1 : 0;
     FFN_CUDA_TRY(cudaLaunchKernelEx(&cfg, stream_tc_kernel<NP, PAIRS>, P), "streaming tcgen05 launch");
     return FFN_OK;
 }
@@ -594,10 +595,15 @@ static int st_launch_np(const StreamTcParams &P, int np, int ctas, cudaStream_t 
     }
 }
 static int st_tile_input(uint8_t *xt, const void *x, const FusedNorm *norm, int M, const StTokens &t, int K, unsigned *arrivals, size_t counter_bytes, cudaStream_t stream) {
-    stream_tile_input_kernel<<<t.blocks * t.np, kTileThreads, 0, stream>>>(xt, (const uint16_t *)x, norm ? (const uint16_t *)norm->weight : nullptr,
-                                                                           norm ? norm->eps : 1.0f, norm && norm->gemma ? 1.0f : 0.0f, M, t.per_block, t.np, K,
-                                                                           arrivals, (int)(counter_bytes / sizeof(unsigned)));
-    FFN_CUDA_TRY(cudaGetLastError(), "tile-order input launch");
+    cudaLaunchAttribute attr = {};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(t.blocks * t.np)); cfg.blockDim = dim3(kTileThreads); cfg.stream = stream;
+    cfg.attrs = &attr; cfg.numAttrs = fused_launch_overlap() ? 1 : 0;
+    FFN_CUDA_TRY(cudaLaunchKernelEx(&cfg, stream_tile_input_kernel, xt, (const uint16_t *)x, norm ? (const uint16_t *)norm->weight : (const uint16_t *)nullptr,
+                                    norm ? norm->eps : 1.0f, norm && norm->gemma ? 1.0f : 0.0f, M, t.per_block, t.np, K, arrivals, (int)(counter_bytes / sizeof(unsigned))),
+                 "tile-order input launch");
     return FFN_OK;
 }
 static int st_device(int *dev, int *sm_count) {

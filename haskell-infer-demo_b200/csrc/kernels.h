@@ -134,6 +134,7 @@ int kmajor_ffn_launch(cudaStream_t stream, const void *x, void *act, void *layer
                       int num_layers, int tokens, int H, int I, const FusedTp *tp, void *residual, int with_norm,
                       float eps, int gemma, unsigned *status);
 void kmajor_reset_sync();
+bool fused_launch_overlap();
 int fused_set_launch_overlap(int on); /* ffn_fused.cu: programmatic dependent launch on or off; returns the previous setting */
 /* ffn_imma.cu: the same contract for 1..4 tokens with the inner products on the INT8 tensor cores.
  * kmajor_ffn_launch tries it first only after kmajor_prefer_dp4a(0) (A/B measurements, tests): it measured
