@@ -58,7 +58,7 @@ static int mlp_common(cudaStream_t stream, const void *normed, void *ws, void *l
     if (g_fused_enabled) { /* 3..64 tokens per pass on the tensor cores; longer batches in blocks of 64 */
         unsigned *status = nullptr;
         if ((st = fused_status_word(&status))) return st;
-        if ((st = stream_tc_ffn_launch(stream, normed, act, layer_out, w, tokens, H, I, nullptr, nullptr, status)) != FFN_NOT_ADMITTED) return st;
+        if ((st = stream_tc_ffn_launch(stream, normed, act, layer_out, w, tokens, H, I, nullptr, nullptr, nullptr, status)) != FFN_NOT_ADMITTED) return st;
         bool taken = true;
         for (int m0 = 0; m0 < tokens && taken; m0 += 64) {
             const int m = tokens - m0 < 64 ? tokens - m0 : 64;
@@ -347,6 +347,16 @@ int ffn_forward_mlp(void *cublas, void *stream, const void *residual, void *ws, 
     const void *normed = residual;
     if (w->post_norm_w) {
         if (!(dims->rms_eps > 0.0f)) return fail(FFN_ERR_CONFIG, "ffn_forward_mlp: invalid shape or epsilon");
+        if (g_fused_enabled && tokens > 2) { /* the norm in the input stage of the FFN's own kernels */
+            const FusedNorm norm = {w->post_norm_w, dims->rms_eps, dims->norm_style == 0};
+            uint16_t *act = (uint16_t *)ws + (size_t)tokens * dims->hidden_size + (size_t)2 * tokens * dims->intermediate_size;
+            unsigned *status = nullptr;
+            int st = FFN_NOT_ADMITTED;
+            if (tc_get_mode() == 2 && (st = fused_status_word(&status))) return st;
+            if (status) st = stream_tc_ffn_launch((cudaStream_t)stream, residual, act, layer_out, w, tokens, dims->hidden_size,
+                                                  dims->intermediate_size, nullptr, &norm, ws, status);
+            if (st != FFN_NOT_ADMITTED) return st;
+        }
         const int st = gemma_rms_norm(ws, residual, w->post_norm_w, dims->hidden_size, tokens,
                                       dims->rms_eps, dims->norm_style == 0, (cudaStream_t)stream);
         if (st) return st;

@@ -5,8 +5,8 @@
  * what the operator-level entry points fall back on for shapes the fused kernels do not admit
  * (they are still CUDA kernels - there is no CPU path).
  */
-#include "common.cuh"
 #include "kernels.h"
+#include "stream_common.cuh"
 
 namespace ffn {
 
@@ -173,6 +173,9 @@ __global__ void __launch_bounds__(256)
 gemma_rms_norm_kernel(uint16_t *__restrict__ out, const uint16_t *__restrict__ x,
                       const uint16_t *__restrict__ w, int cols, float eps, int gemma) {
     __shared__ float red[8];
+    /* This kernel is launched without the overlap attribute, so whatever wrote the weights is complete: an FFN
+     * kernel behind it may start its weight stream now, and waits for this grid before it reads the output. */
+    griddep_launch();
     const size_t base = (size_t)blockIdx.x * cols;
     float ss = 0.0f;
     for (int i = threadIdx.x; i < cols; i += blockDim.x) {

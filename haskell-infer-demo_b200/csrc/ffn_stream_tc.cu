@@ -495,11 +495,12 @@ __global__ void __launch_bounds__(StPlan<NP>::kThreads, 1) stream_tc_kernel(cons
 }
 
 /* x bf16 [M][K] -> tile order, one region of np columns per token block, optionally through RMSNorm (the
- * reference's expression and its BF16 rounding); columns without a token become zeros.  One CTA per column;
+ * reference's expression and its BF16 rounding; `normed` then receives the rows in natural order as well);
+ * columns without a token become zeros.  One CTA per column;
  * the first clears the arrival counters of the launches that follow. */
 constexpr int kTileThreads = 512;
 __global__ void __launch_bounds__(kTileThreads) stream_tile_input_kernel(uint8_t *__restrict__ xt, const uint16_t *__restrict__ x,
-                                                                        const uint16_t *__restrict__ norm_w, float eps, float gemma, int M,
+                                                                        const uint16_t *__restrict__ norm_w, float eps, float gemma, uint16_t *__restrict__ normed, int M,
                                                                         int per_block, int np, int K, unsigned *arrivals, int counters) {
     __shared__ float red[kTileThreads / 32];
     griddep_wait();
@@ -539,6 +540,7 @@ __global__ void __launch_bounds__(kTileThreads) stream_tile_input_kernel(uint8_t
                     e[i] = (uint32_t)f32_to_bf16_bits(bf16_lo(e[i]) * inv * w0) | ((uint32_t)f32_to_bf16_bits(bf16_hi(e[i]) * inv * w1) << 16);
                 }
                 v = make_uint4(e[0], e[1], e[2], e[3]);
+                if (normed) *(uint4 *)(normed + (size_t)m * K + p * 8) = v;
             }
         }
         const uint4 o = make_uint4(prmt(v.x, v.z, 0x5410), prmt(v.x, v.z, 0x7632), prmt(v.y, v.w, 0x5410), prmt(v.y, v.w, 0x7632));
@@ -594,7 +596,7 @@ static int st_launch_np(const StreamTcParams &P, int np, int ctas, cudaStream_t 
         default: return st_launch<128, PAIRS>(P, ctas, stream);
     }
 }
-static int st_tile_input(uint8_t *xt, const void *x, const FusedNorm *norm, int M, const StTokens &t, int K, unsigned *arrivals, size_t counter_bytes, cudaStream_t stream) {
+static int st_tile_input(uint8_t *xt, const void *x, const FusedNorm *norm, void *normed, int M, const StTokens &t, int K, unsigned *arrivals, size_t counter_bytes, cudaStream_t stream) {
     cudaLaunchAttribute attr = {};
     attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr.val.programmaticStreamSerializationAllowed = 1;
@@ -602,7 +604,7 @@ static int st_tile_input(uint8_t *xt, const void *x, const FusedNorm *norm, int 
     cfg.gridDim = dim3((unsigned)(t.blocks * t.np)); cfg.blockDim = dim3(kTileThreads); cfg.stream = stream;
     cfg.attrs = &attr; cfg.numAttrs = fused_launch_overlap() ? 1 : 0;
     FFN_CUDA_TRY(cudaLaunchKernelEx(&cfg, stream_tile_input_kernel, xt, (const uint16_t *)x, norm ? (const uint16_t *)norm->weight : (const uint16_t *)nullptr,
-                                    norm ? norm->eps : 1.0f, norm && norm->gemma ? 1.0f : 0.0f, M, t.per_block, t.np, K, arrivals, (int)(counter_bytes / sizeof(unsigned))),
+                                    norm ? norm->eps : 1.0f, norm && norm->gemma ? 1.0f : 0.0f, (uint16_t *)normed, M, t.per_block, t.np, K, arrivals, (int)(counter_bytes / sizeof(unsigned))),
                  "tile-order input launch");
     return FFN_OK;
 }
@@ -625,9 +627,9 @@ static StScratch g_st_scratch[64];
 static std::mutex g_st_mutex;
 
 int stream_tc_ffn_launch(cudaStream_t stream, const void *x, void *act, void *layer_out, const FfnMlpWeights *w, int tokens, int H,
-                         int I, void *residual, const FusedNorm *norm, unsigned *status) {
+                         int I, void *residual, const FusedNorm *norm, void *normed, unsigned *status) {
     if (tokens <= 2 || tc_get_mode() != 2) return FFN_NOT_ADMITTED; /* 3..16 tokens: the mma.sync pair, 63 against 81 us at 8 on the 5120 x 17408 layer */
-    if (((uintptr_t)w->gate_up_i4 & 15) || ((uintptr_t)w->down_i4 & 15) || ((uintptr_t)x & 15)) return FFN_NOT_ADMITTED;
+    if (((uintptr_t)w->gate_up_i4 & 15) || ((uintptr_t)w->down_i4 & 15) || ((uintptr_t)x & 15) || ((uintptr_t)normed & 15)) return FFN_NOT_ADMITTED;
     int dev = 0, sm_count = 0, st = st_device(&dev, &sm_count);
     if (st) return st;
     /* layout: [arrivals of both launches | partial sums | input | act] */
@@ -649,7 +651,7 @@ int stream_tc_ffn_launch(cudaStream_t stream, const void *x, void *act, void *la
         const int m = tokens - m0 < kStSlab ? tokens - m0 : kStSlab;
         const StTokens t = st_tokens(m);
         uint8_t *xt = sc.base + 2 * counters + partial, *act_t = xt + st_tile_bytes(most, H);
-        if ((st = st_tile_input(xt, (const uint16_t *)x + (size_t)m0 * H, norm, m, t, H, (unsigned *)sc.base, 2 * counters, stream))) return st;
+        if ((st = st_tile_input(xt, (const uint16_t *)x + (size_t)m0 * H, norm, normed ? (uint16_t *)normed + (size_t)m0 * H : nullptr, m, t, H, (unsigned *)sc.base, 2 * counters, stream))) return st;
         A.s = (const uint16_t *)w->gate_up_i4_scales; A.xt = xt;
         A.M = m; A.per_block = t.per_block; A.token_blocks = t.blocks;
         A.N = I; A.K = H; A.up_offset = I; A.blocks = (I / 64) * t.blocks;
@@ -711,7 +713,7 @@ int stream_tc_gemm(const void *a, const void *packed, const void *scales, void *
         const int m = M - m0 < kStSlab ? M - m0 : kStSlab;
         const StTokens t = st_tokens(m);
         uint8_t *xt = base + counters + partial;
-        if ((st = st_tile_input(xt, (const uint16_t *)a + (size_t)m0 * K, nullptr, m, t, K, (unsigned *)base, counters, stream))) break;
+        if ((st = st_tile_input(xt, (const uint16_t *)a + (size_t)m0 * K, nullptr, nullptr, m, t, K, (unsigned *)base, counters, stream))) break;
         P.s = (const uint16_t *)scales; P.xt = xt;
         P.M = m; P.per_block = t.per_block; P.token_blocks = t.blocks;
         P.N = N; P.K = K; P.blocks = ((N + kTcRows - 1) / kTcRows) * t.blocks;

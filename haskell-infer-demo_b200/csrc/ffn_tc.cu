@@ -711,7 +711,7 @@ long long tc_tile_order_offset(int token, int k, int npad) {
 int batched_ffn_launch(cudaStream_t stream, const void *normed, void *act, void *layer_out,
                        const FfnMlpWeights *w, int tokens, int H, int I, const FusedTp *tp, void *residual, unsigned *status) {
     int st = FFN_NOT_ADMITTED;
-    if (!tp || tp->tp < 2) st = stream_tc_ffn_launch(stream, normed, act, layer_out, w, tokens, H, I, residual, nullptr, status);
+    if (!tp || tp->tp < 2) st = stream_tc_ffn_launch(stream, normed, act, layer_out, w, tokens, H, I, residual, nullptr, nullptr, status);
     if (st == FFN_NOT_ADMITTED) st = tc_ffn_launch(stream, normed, act, layer_out, w, tokens, H, I, tp, residual, status);
     if (st != FFN_NOT_ADMITTED) return st;
     return mma_ffn_launch(stream, normed, act, layer_out, w, tokens, H, I, tp, residual, status);

@@ -165,9 +165,10 @@ int mma_ffn_launch(cudaStream_t stream, const void *normed, void *act, void *lay
  * rows, written to shared memory with the 128-byte swizzle (ffn_tc.cu). */
 int weight_tile_map(CUtensorMap_st *map, const void *w, int rows, int K, int box_rows);
 /* ffn_stream_tc.cu: one rank's batched FFN for any number of tokens (optional RMSNorm in its input stage,
- * optional residual update) and the GEMM for any number of rows. */
+ * which also leaves the normalized rows in `normed`; optional residual update) and the GEMM for any number of
+ * rows. */
 int stream_tc_ffn_launch(cudaStream_t stream, const void *x, void *act, void *layer_out, const FfnMlpWeights *w, int tokens, int H,
-                         int I, void *residual, const FusedNorm *norm, unsigned *status);
+                         int I, void *residual, const FusedNorm *norm, void *normed, unsigned *status);
 int stream_tc_gemm(const void *a, const void *packed, const void *scales, void *out, int M, int N, int K, cudaStream_t stream);
 /* Device address of the status word shared by the kernels of this library (allocating it on first use). */
 int fused_status_word(unsigned **out);

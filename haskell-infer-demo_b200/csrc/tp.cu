@@ -363,10 +363,11 @@ static int decode_layer(TpComm *c, cudaStream_t stream, void *h, void *ws, void 
     int st = fused_ffn_launch(stream, h, act, layer_out, w, tokens, H, I, tp, h, &norm);
     if (st != FFN_NOT_ADMITTED) return st;
     if (tokens > 64) return fail(FFN_ERR_CONFIG, "ffn_decode_layer: at most 64 tokens per call");
-    st = gemma_rms_norm(normed, h, w->post_norm_w, H, tokens, dims->rms_eps, dims->norm_style == 0, stream);
-    if (st) return st;
     unsigned *status = nullptr;
     if ((st = fused_status_word(&status))) return st;
+    if (!tp && (st = stream_tc_ffn_launch(stream, h, act, layer_out, w, tokens, H, I, h, &norm, normed, status)) != FFN_NOT_ADMITTED) return st;
+    st = gemma_rms_norm(normed, h, w->post_norm_w, H, tokens, dims->rms_eps, dims->norm_style == 0, stream);
+    if (st) return st;
     st = batched_ffn_launch(stream, normed, act, layer_out, w, tokens, H, I, tp, h, status);
     if (st == FFN_NOT_ADMITTED) return fail(FFN_ERR_CONFIG, "ffn_decode_layer: no kernel takes tokens=%d H=%d I=%d", tokens, H, I);
     return st;
