@@ -668,8 +668,9 @@ int stream_tc_ffn_launch(cudaStream_t stream, const void *x, void *act, void *la
     return FFN_OK;
 }
 
-/* The GEMM's scratch comes from a stream-ordered pool of its own, so calls on different streams and threads
- * never share it; the pool keeps at most 64 MiB between calls. */
+/* Scratch of a call that any stream and thread may make at any time (the GEMM, the quantizer) comes from a
+ * stream-ordered pool of the library's own and goes back with cudaFreeAsync on the same stream; the pool keeps
+ * at most 64 MiB between calls. */
 constexpr unsigned long long kStPoolKeep = 64ull << 20;
 static cudaMemPool_t g_st_pool[64];
 static std::mutex g_st_pool_mutex;
@@ -692,23 +693,29 @@ static int st_pool(int dev, cudaMemPool_t *out) {
     return FFN_OK;
 }
 
+int scratch_alloc(void **out, size_t bytes, cudaStream_t stream) {
+    int dev = 0;
+    FFN_CUDA_TRY(cudaGetDevice(&dev), "cudaGetDevice");
+    if (dev < 0 || dev >= 64) return FFN_NOT_ADMITTED;
+    cudaMemPool_t pool;
+    if (st_pool(dev, &pool) != FFN_OK) return FFN_NOT_ADMITTED;
+    if (cudaMallocFromPoolAsync(out, bytes, pool, stream) == cudaSuccess) return FFN_OK;
+    (void)cudaGetLastError();
+    return FFN_NOT_ADMITTED;
+}
+
 int stream_tc_gemm(const void *a, const void *packed, const void *scales, void *out, int M, int N, int K, cudaStream_t stream) {
     int dev = 0, sm_count = 0, st = st_device(&dev, &sm_count);
     if (st) return st;
     unsigned *status = nullptr;
     if ((st = fused_status_word(&status))) return st;
-    cudaMemPool_t pool;
-    if (st_pool(dev, &pool) != FFN_OK) return FFN_NOT_ADMITTED;
     const StTokens most = st_tokens(M < kStSlab ? M : kStSlab);
     const size_t counters = st_counter_bytes(sm_count), partial = st_partial_bytes(sm_count, M <= kStSlab ? most.np : kStMaxTokens);
     const size_t tiles = M <= kStSlab ? st_tile_bytes(most, K) : st_round((size_t)kStSlab * K * 2);
     StreamTcParams P = {};
     if ((st = weight_tile_map(&P.wmap, packed, N, K, kTcRows))) return st;
     uint8_t *base = nullptr;
-    if (cudaMallocFromPoolAsync((void **)&base, counters + partial + tiles, pool, stream) != cudaSuccess) {
-        (void)cudaGetLastError();
-        return FFN_NOT_ADMITTED;
-    }
+    if ((st = scratch_alloc((void **)&base, counters + partial + tiles, stream))) return st;
     for (int m0 = 0; m0 < M && st == FFN_OK; m0 += kStSlab) {
         const int m = M - m0 < kStSlab ? M - m0 : kStSlab;
         const StTokens t = st_tokens(m);

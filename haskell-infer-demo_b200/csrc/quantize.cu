@@ -11,8 +11,15 @@
  * positive finite BF16 (e.g. a group of 1e-40).  The reference validates everything before it
  * writes anything; so does this file (one checking pass, then the writing pass).
  *
- * One warp per group: a lane loads four consecutive elements (one 16-byte load, 512 contiguous bytes
- * per warp), the maximum is a five-step shuffle, and each lane stores its two packed bytes.
+ * HBM bound: the FP32 input is read once.  The checking pass quantizes into scratch as it goes, and a second
+ * launch moves the bytes to the caller once nothing was refused - it looks at the verdict itself, so the host
+ * waits once, at the end.  5120 x 17408: 221 us with a checking and a writing pass over the input, a wait
+ * between them and cudaMalloc / cudaFree around them; MEASURED now.  Where the bytes exceed the scratch that
+ * the library keeps (kScratchMost) the second launch quantizes again instead.
+ *
+ * One warp per group, four groups in flight: a lane loads four consecutive elements of each (16-byte loads,
+ * 512 contiguous bytes per warp), the maximum is a five-step shuffle, and each lane stores its two packed
+ * bytes.
  */
 #include "common.cuh"
 #include "kernels.h"
@@ -32,48 +39,85 @@ struct QuantStatus {
     unsigned long long bad_group;   /* 1 + (row * groups + group) of an unrepresentable scale, 0 = none */
 };
 
-template <bool WRITE>
-__global__ void __launch_bounds__(256) quantize_int4_kernel(const float *__restrict__ w, uint8_t *__restrict__ packed,
-                                                            uint16_t *__restrict__ scales, long long groups_total,
-                                                            QuantStatus *status) {
+constexpr int kGroupsInFlight = 4;
+constexpr int kQuantThreads = 256;
+constexpr size_t kScratchMost = 56ull << 20; /* of the 64 MiB that the library's pool keeps between calls */
+
+/* CHECK: looks for what the format cannot hold (and writes the bytes where `packed` is given); else nothing is
+ * written when a check before this launch found something. */
+template <bool CHECK>
+__global__ void __launch_bounds__(kQuantThreads) quantize_int4_kernel(const float *__restrict__ w, uint8_t *__restrict__ packed,
+                                                                     uint16_t *__restrict__ scales, long long groups_total,
+                                                                     QuantStatus *status) {
+    if (!CHECK && (status->bad_element != ~0ull || status->bad_group != ~0ull)) return;
     const int lane = threadIdx.x & 31;
     const long long warp = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     const long long nwarps = (long long)gridDim.x * (blockDim.x >> 5);
-    for (long long grp = warp; grp < groups_total; grp += nwarps) {
-        const long long base = grp * FFN_INT4_GROUP + lane * 4;
-        const float4 v = *(const float4 *)(w + base);
-        const float e[4] = {v.x, v.y, v.z, v.w};
-        float max_abs = 0.0f;
-        bool finite = true;
+    for (long long first = warp * kGroupsInFlight; first < groups_total; first += nwarps * kGroupsInFlight) {
+        float4 v[kGroupsInFlight];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            finite = finite && isfinite(e[i]);
-            max_abs = fmaxf(max_abs, fabsf(e[i]));
-        }
-        if (!WRITE && !finite) {
+        for (int j = 0; j < kGroupsInFlight; ++j)
+            v[j] = first + j < groups_total ? __ldcs((const float4 *)(w + (first + j) * FFN_INT4_GROUP) + lane) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 #pragma unroll
-            for (int i = 0; i < 4; ++i)
-                if (!isfinite(e[i])) atomicMin(&status->bad_element, (unsigned long long)(base + i) + 1ull);
-        }
+        for (int j = 0; j < kGroupsInFlight; ++j) {
+            const long long grp = first + j;
+            if (grp >= groups_total) break;
+            const long long base = grp * FFN_INT4_GROUP + lane * 4;
+            const float e[4] = {v[j].x, v[j].y, v[j].z, v[j].w};
+            /* magnitudes compare like their bits, with Inf and NaN above every finite one */
+            unsigned top = 0;
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) max_abs = fmaxf(max_abs, __shfl_xor_sync(0xFFFFFFFFu, max_abs, o));
-        const uint16_t scale_bits = max_abs == 0.0f ? (uint16_t)0x3F80u : bf16_rne_bits(__fdiv_rn(max_abs, 7.0f));
-        const float scale = bf16_bits_to_f32(scale_bits);
-        if (!WRITE) {
-            if (lane == 0 && (!(scale > 0.0f) || !isfinite(scale))) atomicMin(&status->bad_group, (unsigned long long)grp + 1ull);
-            continue;
-        }
-        if (lane == 0) scales[grp] = scale_bits;
-        uint32_t nib[4];
+            for (int i = 0; i < 4; ++i) top = max(top, __float_as_uint(e[i]) & 0x7FFFFFFFu);
+            top = __reduce_max_sync(0xFFFFFFFFu, top);
+            if (top >= 0x7F800000u) { /* a group with an Inf or a NaN */
+                if (CHECK) {
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            float q = rintf(__fdiv_rn(e[i], scale)); /* nearest even, like nearbyintf in the default mode */
-            q = fminf(fmaxf(q, -7.0f), 7.0f);
-            nib[i] = (uint32_t)((int)q) & 0xFu;
+                    for (int i = 0; i < 4; ++i)
+                        if (!isfinite(e[i])) atomicMin(&status->bad_element, (unsigned long long)(base + i) + 1ull);
+                }
+                continue;
+            }
+            const uint16_t scale_bits = top == 0u ? (uint16_t)0x3F80u : bf16_rne_bits(__fdiv_rn(__uint_as_float(top), 7.0f));
+            const float scale = bf16_bits_to_f32(scale_bits);
+            if (CHECK && lane == 0 && (!(scale > 0.0f) || !isfinite(scale))) atomicMin(&status->bad_group, (unsigned long long)grp + 1ull);
+            if (CHECK && !packed) continue;
+            if (lane == 0) scales[grp] = scale_bits;
+            /* The code is rint(e / scale), nearest even, of the correctly rounded quotient.  The product with the
+             * reciprocal is within 2e-6 of it (|quotient| < 7.1, three roundings), so the two agree unless the product
+             * lies that close to a half; those, and groups whose scale is too small for the bound, divide.
+             * Adding 1.5 * 2^23 leaves the rounded integer in the low bits, in two's complement. */
+            uint32_t nib[4];
+            const float recip = __frcp_rn(scale);
+            float off = 0.0f;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const float t = e[i] * recip, m = t + 12582912.0f;
+                off = fmaxf(off, fabsf(t - (m - 12582912.0f)));
+                nib[i] = __float_as_uint(m) & 0xFu;
+            }
+            if (!(off < 0.49999f) || scale < 7.8886091e-31f /* 2^-100 */) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const float q = fminf(fmaxf(rintf(__fdiv_rn(e[i], scale)), -7.0f), 7.0f);
+                    nib[i] = (uint32_t)((int)q) & 0xFu;
+                }
+            }
+            const uint16_t two = (uint16_t)(nib[0] | (nib[1] << 4) | (nib[2] << 8) | (nib[3] << 12));
+            *(uint16_t *)(packed + base / 2) = two;
         }
-        const uint16_t two = (uint16_t)(nib[0] | (nib[1] << 4) | (nib[2] << 8) | (nib[3] << 12));
-        *(uint16_t *)(packed + base / 2) = two;
     }
+}
+
+/* The quantized bytes from scratch to the caller, unless something was refused.  Both counts are in units of
+ * T: 16 bytes where the caller's pointers allow it, else 2. */
+template <typename T>
+__global__ void __launch_bounds__(kQuantThreads) quantize_deliver_kernel(T *__restrict__ packed, const T *__restrict__ from_packed, long long np,
+                                                                        T *__restrict__ scales, const T *__restrict__ from_scales, long long ns,
+                                                                        const QuantStatus *status) {
+    if (status->bad_element != ~0ull || status->bad_group != ~0ull) return;
+    const long long step = (long long)gridDim.x * kQuantThreads, at = (long long)blockIdx.x * kQuantThreads + threadIdx.x;
+    for (long long i = at; i < np; i += step) packed[i] = from_packed[i];
+    for (long long i = at; i < ns; i += step) scales[i] = from_scales[i];
 }
 
 }  // namespace ffn
@@ -90,17 +134,33 @@ extern "C" int ffn_quantize_int4(const void *weights, void *packed, void *scales
     if (((uintptr_t)weights & 15) || ((uintptr_t)packed & 1) || ((uintptr_t)scales & 1))
         return fail(FFN_ERR_CONFIG, "ffn_quantize_int4: weights must be 16-byte aligned, outputs 2-byte aligned");
     const long long groups = n * (k / FFN_INT4_GROUP);
-    QuantStatus *status = nullptr;
-    if (cudaMalloc(&status, sizeof(QuantStatus)) != cudaSuccess) { (void)cudaGetLastError(); return fail(FFN_ERR_ALLOC, "ffn_quantize_int4: cannot allocate the status words"); }
+    const long long packed_bytes = n * k / 2, scale_bytes = groups * 2;
+    const bool keep = (size_t)(packed_bytes + scale_bytes) <= kScratchMost;
+    const size_t scales_at = 256 + ((size_t)packed_bytes + 255) / 256 * 256;
+    uint8_t *scratch = nullptr;
+    if (scratch_alloc((void **)&scratch, keep ? scales_at + (size_t)scale_bytes : 256, stream) != FFN_OK)
+        return fail(FFN_ERR_ALLOC, "ffn_quantize_int4: cannot allocate the status words");
+    QuantStatus *status = (QuantStatus *)scratch;
     int rc = FFN_OK;
     QuantStatus host;
-    const unsigned grid = (unsigned)((groups + 7) / 8 < 148ll * 16 ? (groups + 7) / 8 : 148ll * 16);
+    const long long turns = (groups + kGroupsInFlight * 8 - 1) / (kGroupsInFlight * 8);
+    const unsigned grid = (unsigned)(turns < 148ll * 16 ? turns : 148ll * 16);
     do {
         if (cudaMemsetAsync(status, 0xFF, sizeof(QuantStatus), stream) != cudaSuccess) { rc = fail(FFN_ERR_CUDA, "ffn_quantize_int4: memset failed"); break; }
-        quantize_int4_kernel<false><<<grid, 256, 0, stream>>>((const float *)weights, nullptr, nullptr, groups, status);
-        if (cudaMemcpyAsync(&host, status, sizeof(host), cudaMemcpyDeviceToHost, stream) != cudaSuccess ||
+        quantize_int4_kernel<true><<<grid, kQuantThreads, 0, stream>>>((const float *)weights, keep ? scratch + 256 : nullptr,
+                                                                       keep ? (uint16_t *)(scratch + scales_at) : nullptr, groups, status);
+        if (!keep) {
+            quantize_int4_kernel<false><<<grid, kQuantThreads, 0, stream>>>((const float *)weights, (uint8_t *)packed, (uint16_t *)scales, groups, status);
+        } else if (!(((uintptr_t)packed | (uintptr_t)scales | (uintptr_t)scale_bytes) & 15)) {
+            quantize_deliver_kernel<uint4><<<148 * 8, kQuantThreads, 0, stream>>>((uint4 *)packed, (const uint4 *)(scratch + 256), packed_bytes / 16, (uint4 *)scales,
+                                                                                  (const uint4 *)(scratch + scales_at), scale_bytes / 16, status);
+        } else {
+            quantize_deliver_kernel<uint16_t><<<148 * 8, kQuantThreads, 0, stream>>>((uint16_t *)packed, (const uint16_t *)(scratch + 256), packed_bytes / 2,
+                                                                                     (uint16_t *)scales, (const uint16_t *)(scratch + scales_at), scale_bytes / 2, status);
+        }
+        if (cudaGetLastError() != cudaSuccess || cudaMemcpyAsync(&host, status, sizeof(host), cudaMemcpyDeviceToHost, stream) != cudaSuccess ||
             cudaStreamSynchronize(stream) != cudaSuccess) {
-            rc = fail(FFN_ERR_CUDA, "ffn_quantize_int4: checking pass failed: %s", cudaGetErrorString(cudaGetLastError()));
+            rc = fail(FFN_ERR_CUDA, "ffn_quantize_int4: quantizing failed: %s", cudaGetErrorString(cudaGetLastError()));
             break;
         }
         if (host.bad_element != ~0ull) {
@@ -114,10 +174,7 @@ extern "C" int ffn_quantize_int4(const void *weights, void *packed, void *scales
                       "the format cannot represent it", g / per_row, g % per_row);
             break;
         }
-        quantize_int4_kernel<true><<<grid, 256, 0, stream>>>((const float *)weights, (uint8_t *)packed, (uint16_t *)scales, groups, status);
-        if (cudaGetLastError() != cudaSuccess || cudaStreamSynchronize(stream) != cudaSuccess)
-            rc = fail(FFN_ERR_CUDA, "ffn_quantize_int4: writing pass failed");
     } while (0);
-    cudaFree(status);
+    (void)cudaFreeAsync(scratch, stream);
     return rc;
 }
