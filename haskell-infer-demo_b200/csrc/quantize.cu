@@ -14,12 +14,12 @@
  * HBM bound: the FP32 input is read once.  The checking pass quantizes into scratch as it goes, and a second
  * launch moves the bytes to the caller once nothing was refused - it looks at the verdict itself, so the host
  * waits once, at the end.  5120 x 17408: 221 us with a checking and a writing pass over the input, a wait
- * between them and cudaMalloc / cudaFree around them; MEASURED now.  Where the bytes exceed the scratch that
+ * between them and cudaMalloc / cudaFree around them; 118 now.  Where the bytes exceed the scratch that
  * the library keeps (kScratchMost) the second launch quantizes again instead.
  *
- * One warp per group, four groups in flight: a lane loads four consecutive elements of each (16-byte loads,
- * 512 contiguous bytes per warp), the maximum is a five-step shuffle, and each lane stores its two packed
- * bytes.
+ * Eight lanes per group: a lane holds sixteen elements in four 16-byte loads (128 contiguous bytes of a group
+ * each), so the group's division, reciprocal and reduction are paid once per sixteen elements: instructions, not
+ * bytes, are what is left (142 us with a warp per group and four elements a lane).
  */
 #include "common.cuh"
 #include "kernels.h"
@@ -50,61 +50,62 @@ __global__ void __launch_bounds__(kQuantThreads) quantize_int4_kernel(const floa
                                                                      uint16_t *__restrict__ scales, long long groups_total,
                                                                      QuantStatus *status) {
     if (!CHECK && (status->bad_element != ~0ull || status->bad_group != ~0ull)) return;
-    const int lane = threadIdx.x & 31;
+    const int lane = threadIdx.x & 31, sub = lane & 7;
     const long long warp = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     const long long nwarps = (long long)gridDim.x * (blockDim.x >> 5);
     for (long long first = warp * kGroupsInFlight; first < groups_total; first += nwarps * kGroupsInFlight) {
-        float4 v[kGroupsInFlight];
+        const long long grp = first + (lane >> 3);
+        const bool live = grp < groups_total; /* the lanes of a group agree */
+        const long long base = grp * FFN_INT4_GROUP + sub * 4;
+        float e[16]; /* elements base + 32 * j + i */
 #pragma unroll
-        for (int j = 0; j < kGroupsInFlight; ++j)
-            v[j] = first + j < groups_total ? __ldcs((const float4 *)(w + (first + j) * FFN_INT4_GROUP) + lane) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-#pragma unroll
-        for (int j = 0; j < kGroupsInFlight; ++j) {
-            const long long grp = first + j;
-            if (grp >= groups_total) break;
-            const long long base = grp * FFN_INT4_GROUP + lane * 4;
-            const float e[4] = {v[j].x, v[j].y, v[j].z, v[j].w};
-            /* magnitudes compare like their bits, with Inf and NaN above every finite one */
-            unsigned top = 0;
-#pragma unroll
-            for (int i = 0; i < 4; ++i) top = max(top, __float_as_uint(e[i]) & 0x7FFFFFFFu);
-            top = __reduce_max_sync(0xFFFFFFFFu, top);
-            if (top >= 0x7F800000u) { /* a group with an Inf or a NaN */
-                if (CHECK) {
-#pragma unroll
-                    for (int i = 0; i < 4; ++i)
-                        if (!isfinite(e[i])) atomicMin(&status->bad_element, (unsigned long long)(base + i) + 1ull);
-                }
-                continue;
-            }
-            const uint16_t scale_bits = top == 0u ? (uint16_t)0x3F80u : bf16_rne_bits(__fdiv_rn(__uint_as_float(top), 7.0f));
-            const float scale = bf16_bits_to_f32(scale_bits);
-            if (CHECK && lane == 0 && (!(scale > 0.0f) || !isfinite(scale))) atomicMin(&status->bad_group, (unsigned long long)grp + 1ull);
-            if (CHECK && !packed) continue;
-            if (lane == 0) scales[grp] = scale_bits;
-            /* The code is rint(e / scale), nearest even, of the correctly rounded quotient.  The product with the
-             * reciprocal is within 2e-6 of it (|quotient| < 7.1, three roundings), so the two agree unless the product
-             * lies that close to a half; those, and groups whose scale is too small for the bound, divide.
-             * Adding 1.5 * 2^23 leaves the rounded integer in the low bits, in two's complement. */
-            uint32_t nib[4];
-            const float recip = __frcp_rn(scale);
-            float off = 0.0f;
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const float t = e[i] * recip, m = t + 12582912.0f;
-                off = fmaxf(off, fabsf(t - (m - 12582912.0f)));
-                nib[i] = __float_as_uint(m) & 0xFu;
-            }
-            if (!(off < 0.49999f) || scale < 7.8886091e-31f /* 2^-100 */) {
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const float q = fminf(fmaxf(rintf(__fdiv_rn(e[i], scale)), -7.0f), 7.0f);
-                    nib[i] = (uint32_t)((int)q) & 0xFu;
-                }
-            }
-            const uint16_t two = (uint16_t)(nib[0] | (nib[1] << 4) | (nib[2] << 8) | (nib[3] << 12));
-            *(uint16_t *)(packed + base / 2) = two;
+        for (int j = 0; j < 4; ++j) {
+            const float4 v = live ? __ldcs((const float4 *)(w + base + 32 * j)) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            e[4 * j] = v.x; e[4 * j + 1] = v.y; e[4 * j + 2] = v.z; e[4 * j + 3] = v.w;
         }
+        /* magnitudes compare like their bits, with Inf and NaN above every finite one */
+        unsigned top = 0;
+#pragma unroll
+        for (int i = 0; i < 16; ++i) top = max(top, __float_as_uint(e[i]) & 0x7FFFFFFFu);
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) top = max(top, __shfl_xor_sync(0xFFFFFFFFu, top, o));
+        if (top >= 0x7F800000u) { /* a group with an Inf or a NaN */
+            if (CHECK) {
+#pragma unroll
+                for (int i = 0; i < 16; ++i)
+                    if (!isfinite(e[i])) atomicMin(&status->bad_element, (unsigned long long)(base + 32 * (i >> 2) + (i & 3)) + 1ull);
+            }
+            continue;
+        }
+        if (!live) continue;
+        const uint16_t scale_bits = top == 0u ? (uint16_t)0x3F80u : bf16_rne_bits(__fdiv_rn(__uint_as_float(top), 7.0f));
+        const float scale = bf16_bits_to_f32(scale_bits);
+        if (CHECK && sub == 0 && (!(scale > 0.0f) || !isfinite(scale))) atomicMin(&status->bad_group, (unsigned long long)grp + 1ull);
+        if (CHECK && !packed) continue;
+        if (sub == 0) scales[grp] = scale_bits;
+        /* The code is rint(e / scale), nearest even, of the correctly rounded quotient.  The product with the
+         * reciprocal is within 2e-6 of it (|quotient| < 7.1, three roundings), so the two agree unless the product
+         * lies that close to a half; those, and groups whose scale is too small for the bound, divide.
+         * Adding 1.5 * 2^23 leaves the rounded integer in the low bits, in two's complement. */
+        uint32_t nib[16];
+        const float recip = __frcp_rn(scale);
+        float off = 0.0f;
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+            const float t = e[i] * recip, m = t + 12582912.0f;
+            off = fmaxf(off, fabsf(t - (m - 12582912.0f)));
+            nib[i] = __float_as_uint(m) & 0xFu;
+        }
+        if (!(off < 0.49999f) || scale < 7.8886091e-31f /* 2^-100 */) {
+#pragma unroll
+            for (int i = 0; i < 16; ++i) {
+                const float q = fminf(fmaxf(rintf(__fdiv_rn(e[i], scale)), -7.0f), 7.0f);
+                nib[i] = (uint32_t)((int)q) & 0xFu;
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            *(uint16_t *)(packed + base / 2 + 16 * j) = (uint16_t)(nib[4 * j] | (nib[4 * j + 1] << 4) | (nib[4 * j + 2] << 8) | (nib[4 * j + 3] << 12));
     }
 }
 
