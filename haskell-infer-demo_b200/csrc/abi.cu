@@ -55,7 +55,7 @@ static int mlp_common(cudaStream_t stream, const void *normed, void *ws, void *l
     uint16_t *act = packed_act + (size_t)2 * tokens * I;         /* [T, I] */
     int st = g_fused_enabled ? fused_ffn_try(stream, normed, act, layer_out, w, tokens, H, I) : FFN_NOT_ADMITTED;
     if (st != FFN_NOT_ADMITTED) return st;
-    if (g_fused_enabled) { /* 3..64 tokens per pass on the tensor cores; longer batches in blocks of 64 */
+    if (g_fused_enabled) { /* the streaming tensor-core kernel; where it does not take the call, the pairs in passes of 64 tokens */
         unsigned *status = nullptr;
         if ((st = fused_status_word(&status))) return st;
         if ((st = stream_tc_ffn_launch(stream, normed, act, layer_out, w, tokens, H, I, nullptr, nullptr, nullptr, status)) != FFN_NOT_ADMITTED) return st;
@@ -150,6 +150,11 @@ int ffn_int4_describe_plan(int tokens, int hidden, int intermediate, int sm_coun
             const size_t used = strlen(out);
             snprintf(out + used, out_bytes - used, " passes=%d", (tokens + 63) / 64);
         }
+        char one[160]; /* without tensor parallelism the streaming kernel comes first */
+        if (stream_tc_describe(tokens, hidden, smem_optin, one, sizeof(one))) {
+            const size_t used = strlen(out);
+            snprintf(out + used, out_bytes - used, " one_rank_kernel=%s", one);
+        }
         return FFN_OK;
     }
     snprintf(out, out_bytes, "kernel=generic launches=3 (gate/up GEMM, SiLU*up, down GEMM)");
@@ -207,7 +212,9 @@ int ffn_int4_describe_gemm_plan(int m, int n, int k, int sm_count, int smem_opti
     if (m < 1 || n <= 0 || k <= 0 || k % FFN_INT4_GROUP || sm_count < 1 || smem_optin < 1)
         return fail(FFN_ERR_CONFIG, "ffn_int4_describe_gemm_plan: invalid shape or device description");
     if (m <= 2 && gemv_describe_plan(m, n, k, sm_count, smem_optin, out, out_bytes)) return FFN_OK;
-    snprintf(out, out_bytes, "kernel=generic launches=1");
+    char stream[160];
+    if (stream_tc_describe(m, k, smem_optin, stream, sizeof(stream))) snprintf(out, out_bytes, "kernel=%s", stream);
+    else snprintf(out, out_bytes, "kernel=generic launches=1");
     return FFN_OK;
 }
 

@@ -37,6 +37,9 @@
  * caller.  Every wait is bounded; a wait that runs out records where, and every thread still reaches the
  * end of the kernel, where tensor memory is released.
  */
+#include <stdio.h>
+
+#include <atomic>
 #include <mutex>
 
 #include "kernels.h"
@@ -617,6 +620,14 @@ static int st_device(int *dev, int *sm_count) {
     return smem >= kStSmem ? FFN_OK : FFN_NOT_ADMITTED;
 }
 
+bool stream_tc_describe(int tokens, int K, int smem_optin, char *out, size_t out_bytes) {
+    if (tokens < 3 || tc_get_mode() != 2 || smem_optin < kStSmem) return false;
+    const StTokens t = st_tokens(tokens < kStSlab ? tokens : kStSlab);
+    snprintf(out, out_bytes, "stream_tc columns=%d token_blocks=%d launches_of_%d_tokens=%d units_per_block=%d", t.np, t.blocks, kStSlab,
+             (tokens + kStSlab - 1) / kStSlab, (K / FFN_INT4_GROUP + 1) / 2);
+    return true;
+}
+
 /* Scratch of the FFN pair per device, sized for a whole slab of tokens and grown for larger layers (calls
  * on one device are serialised by the caller). */
 struct StScratch {
@@ -707,6 +718,16 @@ int scratch_alloc(void **out, size_t bytes, cudaStream_t stream) {
 int stream_tc_gemm(const void *a, const void *packed, const void *scales, void *out, int M, int N, int K, cudaStream_t stream) {
     int dev = 0, sm_count = 0, st = st_device(&dev, &sm_count);
     if (st) return st;
+    /* The device's first call creates the status word and the pool, which a stream that is being captured must
+     * not do: such a call takes the shape-generic kernel, as every call of three rows and more once did. */
+    static std::atomic<bool> ready[64];
+    if (!ready[dev].load()) {
+        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(stream, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone) {
+            (void)cudaGetLastError();
+            return FFN_NOT_ADMITTED;
+        }
+    }
     unsigned *status = nullptr;
     if ((st = fused_status_word(&status))) return st;
     const StTokens most = st_tokens(M < kStSlab ? M : kStSlab);
@@ -716,6 +737,7 @@ int stream_tc_gemm(const void *a, const void *packed, const void *scales, void *
     if ((st = weight_tile_map(&P.wmap, packed, N, K, kTcRows))) return st;
     uint8_t *base = nullptr;
     if ((st = scratch_alloc((void **)&base, counters + partial + tiles, stream))) return st;
+    ready[dev].store(true);
     for (int m0 = 0; m0 < M && st == FFN_OK; m0 += kStSlab) {
         const int m = M - m0 < kStSlab ? M - m0 : kStSlab;
         const StTokens t = st_tokens(m);

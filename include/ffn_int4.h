@@ -12,8 +12,9 @@
  *
  * Concurrency: the FFN entry points of one device (ffn_forward_mlp*, ffn_forward_mlp_tp,
  * ffn_decode_stack, ffn_gemm_int4_bf16 with one or two rows, ffn_tp_allreduce_sum) share that
- * device's synchronisation words, kernel status word and, for 3..64 tokens, one scratch region
- * (permuted activations, split-K partial sums, arrival counters).  Calls on one device must
+ * device's synchronisation words, kernel status word and, from three tokens on, one scratch region
+ * (activations in the kernels' order, split-K partial sums, arrival counters; sized for 512 tokens of
+ * the largest layer seen: 42 MB for 5120 x 17408).  Calls on one device must
  * therefore be serialised: issue them on one stream, or order the streams with events.  Calls on
  * different devices are independent.  The first call on a device, and the first call of the batched
  * path there, allocate these words with cudaMalloc: make them before capturing a CUDA graph.
@@ -80,7 +81,9 @@ const char *ffn_int4_numerical_policy(void);
 /* Which kernel a call of this shape takes and its launch geometry (grid, shared memory, pipeline
  * stages, tile sizes, K splits), as one line of key=value text, for a device with `sm_count` SMs and
  * `smem_optin` bytes of opt-in shared memory per block.  Pure host arithmetic: needs no GPU, so the
- * planning can be checked for any shape anywhere.  `intermediate` is the rank-local size.  No
+ * planning can be checked for any shape anywhere.  `intermediate` is the rank-local size.  From three
+ * tokens on, kernel= names the pair that serves the shape under tensor parallelism and what follows is
+ * its geometry; one_rank_kernel= names the kernel that a single rank runs, where that is another.  No
  * counterpart in the reference (its launch shapes are fixed constants, csrc/kernels/gemm_quant.cu:20-31). */
 int ffn_int4_describe_plan(int tokens, int hidden, int intermediate, int sm_count, int smem_optin, char *out,
                            size_t out_bytes);
@@ -112,8 +115,12 @@ int ffn_int4_set_fused(int enabled);
  * csrc/linear_weight.cpp:63-68).  M == 0 or N == 0 is a successful no-op.  Asynchronous on
  * `stream`.  One or two rows (the decode case: the FFN's matrices on their own, attention / GDN
  * projections, the LM head) stream through the persistent bulk-copy kernel when N % 8 == 0, K <=
- * 34816 (17408 for two rows) and the three operands are 16-byte aligned; everything else takes the
- * shape-generic kernel.  A non-finite activation makes the outputs it reaches non-finite in both. */
+ * 34816 (17408 for two rows) and the three operands are 16-byte aligned; three rows and more take the
+ * streaming tensor-core kernel (tcgen05, 128 rows a block, 512 a launch), whose scratch comes from a
+ * stream-ordered pool of the library's (at most 64 MiB kept between calls), so calls on different
+ * streams and threads are independent; everything else, and a device's first such call when its
+ * stream is being captured, takes the shape-generic kernel.  A non-finite activation makes the outputs
+ * it reaches non-finite in all of them. */
 int ffn_gemm_int4_bf16(const void *a, const void *packed, const void *scales, void *out, int M,
                        int N, int K, int group, void *stream);
 
@@ -259,10 +266,13 @@ int ffn_int4_describe_kmajor_plan(int tokens, int hidden, int intermediate, int 
  * opt-in and kept for A/B measurement.  Returns the previous setting. */
 int ffn_int4_set_decode_kernel(int which);
 
-/* Which pair of kernels serves 3..64 tokens per pass: 1 the mma.sync pair; 0 the tcgen05 pair
+/* Which kernels serve three tokens and more.  2 (default): on one rank the streaming tcgen05 kernel
+ * (csrc/ffn_stream_tc.cu: 50 us at 8 tokens, 55 at 27, 104 at 128 on the 5120 x 17408 layer); under tensor
+ * parallelism, whose exchange only the pairs have, one of the two pairs below by the rule given there.  0 and 1
+ * force a pair, in passes of up to 64 tokens, on one rank too: 1 the mma.sync pair; 0 the tcgen05 pair
  * (tcgen05.mma with FP32 accumulators and the converted BF16 operand in tensor memory, packed INT4 rows
  * brought in by tiled TMA loads), falling back to the mma.sync pair for shapes it does not take (hidden
- * size not a multiple of 128, intermediate size not a multiple of 64); 2 (default) the tcgen05 pair
+ * size not a multiple of 128, intermediate size not a multiple of 64); and the default's rule among the pairs: the tcgen05 pair
  * where it measured faster on B200 - more than 16 tokens and enough gate/up units (intermediate size / 64)
  * for half the SMs: 123 vs 186 us at 64 tokens, 93 vs 96 at 32 on the 5120 x 17408 layer, 114 vs 132 at
  * 64 tokens on its TP=2 slice - and the mma.sync pair elsewhere (73 vs 82 us at 16 tokens).  Same arithmetic in both: exact codes times BF16
