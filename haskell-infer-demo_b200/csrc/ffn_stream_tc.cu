@@ -208,7 +208,8 @@ __device__ __forceinline__ void st_finish(const StreamTcParams &P, const float (
     }
 }
 
-template <int NP, bool PAIRS>
+/* WIDE: the scales come in pieces of four (st_launch) */
+template <int NP, bool PAIRS, bool WIDE>
 __global__ void __launch_bounds__(StPlan<NP>::kThreads, 1) stream_tc_kernel(const __grid_constant__ StreamTcParams P) {
     using L = StPlan<NP>;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -387,9 +388,10 @@ __global__ void __launch_bounds__(StPlan<NP>::kThreads, 1) stream_tc_kernel(cons
             if (PAIRS) return (lane < 16 ? 0 : P.up_offset) + min(rb * 64 + quadrant * 16 + (lane & 15), P.N - 1);
             return min(rb * kTcRows + quadrant * 32 + lane, P.N - 1);
         };
-        /* a unit's two scales, fetched two units ahead (the weights' scales never change) */
+        /* the scales, which never change, are fetched two units ahead */
         uint16_t sc[2][2] = {{0, 0}, {0, 0}};
-        int s_block = block, s_unit = unit, s_left = count;
+        uint2 piece = make_uint2(0u, 0u), piece_ahead = make_uint2(0u, 0u);
+        int s_block = block, s_unit = WIDE ? unit & ~1 : unit, s_left = WIDE ? count + (unit & 1) : count;
         const uint16_t *s_from = P.s + (size_t)scale_row(block) * G;
         auto fetch = [&](uint16_t (&to)[2]) {
             if (s_left <= 0) return;
@@ -397,6 +399,13 @@ __global__ void __launch_bounds__(StPlan<NP>::kThreads, 1) stream_tc_kernel(cons
             to[0] = ld_scale(s_from + 2 * s_unit);
             to[1] = ld_scale(s_from + min(2 * s_unit + 1, G - 1));
             if (++s_unit == U) { s_unit = 0; if (s_left > 0) s_from = P.s + (size_t)scale_row(++s_block) * G; }
+        };
+        auto fetch_piece = [&](uint2 &to) {
+            if (s_left <= 0) return;
+            s_left -= 2;
+            asm volatile("ld.global.nc.v2.u32 {%0, %1}, [%2];" : "=r"(to.x), "=r"(to.y) : "l"(s_from + 2 * s_unit));
+            s_unit += 2;
+            if (s_unit >= U) { s_unit = 0; if (s_left > 0) s_from = P.s + (size_t)scale_row(++s_block) * G; }
         };
         /* a row's scales lie far apart from the next row's, so each new 32 bytes come from HBM: ask for a block's
          * ahead of time, this one's now and the next one's when it is begun */
@@ -406,8 +415,8 @@ __global__ void __launch_bounds__(StPlan<NP>::kThreads, 1) stream_tc_kernel(cons
             for (int g = 0; g < G; g += 16) prefetch_l2(row + g);
         };
         if (c0 == 0) { ahead(block); ahead(block + 1); }
-        fetch(sc[0]);
-        fetch(sc[1]);
+        if (WIDE) { fetch_piece(piece); fetch_piece(piece_ahead); }
+        else { fetch(sc[0]); fetch(sc[1]); }
         griddep_wait(); /* before the first write: earlier launches may still read what this one overwrites */
         float acc[COLS];
 #pragma unroll
@@ -419,8 +428,15 @@ __global__ void __launch_bounds__(StPlan<NP>::kThreads, 1) stream_tc_kernel(cons
             for (int par = 0; par < 2; ++par) {
                 const int i = i0 + par;
                 if (i >= count || !ok) break;
-                const float scale[2] = {bf16_bits_to_f32(sc[par][0]), bf16_bits_to_f32(sc[par][1])};
-                fetch(sc[par]);
+                float scale[2];
+                if (WIDE) {
+                    const uint32_t two = unit & 1 ? piece.y : piece.x;
+                    scale[0] = bf16_lo(two); scale[1] = bf16_hi(two);
+                    if (unit & 1) { piece = piece_ahead; fetch_piece(piece_ahead); }
+                } else {
+                    scale[0] = bf16_bits_to_f32(sc[par][0]); scale[1] = bf16_bits_to_f32(sc[par][1]);
+                    fetch(sc[par]);
+                }
 #pragma unroll
                 for (int k = 0; k < 2; ++k) {
                     if (k % L::kGroups == 0) {
@@ -573,18 +589,27 @@ static size_t st_counter_bytes(int sm_count) { return st_round((size_t)sm_count 
 static size_t st_partial_bytes(int sm_count, int np) { return (size_t)sm_count * 2 * np * kTcRows * sizeof(float); }
 static size_t st_tile_bytes(const StTokens &t, int K) { return st_round((size_t)t.blocks * t.np * K * 2); }
 
-template <int NP, bool PAIRS>
-static int st_launch(const StreamTcParams &P, int ctas, cudaStream_t stream) {
+template <int NP, bool PAIRS, bool WIDE>
+static int st_launch_kernel(const StreamTcParams &P, int ctas, cudaStream_t stream) {
     using L = StPlan<NP>;
-    FFN_CUDA_TRY(cudaFuncSetAttribute(stream_tc_kernel<NP, PAIRS>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kSmem), "streaming tcgen05: shared-memory opt-in");
+    FFN_CUDA_TRY(cudaFuncSetAttribute(stream_tc_kernel<NP, PAIRS, WIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kSmem), "streaming tcgen05: shared-memory opt-in");
     cudaLaunchAttribute attr = {};
     attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr.val.programmaticStreamSerializationAllowed = 1;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)ctas); cfg.blockDim = dim3(L::kThreads); cfg.dynamicSmemBytes = L::kSmem; cfg.stream = stream;
     cfg.attrs = &attr; cfg.numAttrs = fused_launch_overlap() ? 1 : 0;
-    FFN_CUDA_TRY(cudaLaunchKernelEx(&cfg, stream_tc_kernel<NP, PAIRS>, P), "streaming tcgen05 launch");
+    FFN_CUDA_TRY(cudaLaunchKernelEx(&cfg, stream_tc_kernel<NP, PAIRS, WIDE>, P), "streaming tcgen05 launch");
     return FFN_OK;
+}
+/* A warp's 32 rows are 32 sectors to a load of scales, and shared memory leaves no L1 to keep them in.  Above
+ * 64 tokens, where 16 epilogue warps load them, pieces of two units (rows of whole pieces, K a multiple of 512,
+ * on 8 bytes) are worth it: 5120 x 17408, 128 tokens 103.5 -> 99 us.  Below they are not: the LM head, 5 rows
+ * 132 -> 136. */
+template <int NP, bool PAIRS>
+static int st_launch(const StreamTcParams &P, int ctas, cudaStream_t stream) {
+    if (NP > 64 && P.K % (4 * FFN_INT4_GROUP) == 0 && !((uintptr_t)P.s & 7)) return st_launch_kernel<NP, PAIRS, (NP > 64)>(P, ctas, stream);
+    return st_launch_kernel<NP, PAIRS, false>(P, ctas, stream);
 }
 template <bool PAIRS>
 static int st_launch_np(const StreamTcParams &P, int np, int ctas, cudaStream_t stream) {

@@ -58,6 +58,18 @@ def test_more_tokens_than_one_launch_takes(cuda):
     L.device_status()
 
 
+def test_scales_off_their_alignment(cuda):
+    """Scales at a 2-byte offset are read one by one, with the same result."""
+    packed, scales = ops.quantize_int4(torch.randn((1048, 2048), device=cuda) * 0.02)
+    store = torch.empty(scales.numel() + 1, dtype=torch.bfloat16, device=cuda)
+    off = store[1:].view(scales.shape)
+    off.copy_(scales)
+    for rows in (9, 100):
+        a = torch.randn((rows, 2048), device=cuda).to(torch.bfloat16)
+        assert torch.equal(ops.gemm_int4_bf16(a, packed, off), ops.gemm_int4_bf16(a, packed, scales))
+    L.device_status()
+
+
 def test_a_row_with_nan_stays_alone(cuda):
     packed, scales = ops.quantize_int4(torch.randn((520, 640), device=cuda) * 0.02)
     a = torch.randn((21, 640), device=cuda).to(torch.bfloat16)
