@@ -390,7 +390,8 @@ def run_ours(args):
         peak, peak_kind = measured_peak_gbs()
         gbs = nl * per_rank_bytes / us_step / 1e3
         kmajor = m <= 2 and args.kmajor   # layers with k-major copies: the persistent decode kernel
-        per_layer = 1 if (m <= 2 or kmajor) else (4 if stack else 3)
+        one_rank = world == 1 and L.load().ffn_int4_set_batched_kernel(-1) == 2    # the norm is then part of the input pre-pass
+        per_layer = 1 if (m <= 2 or kmajor) else (4 if stack and not one_rank else 3)
         launches = nl * per_layer
         if stack and kmajor:
             launches = -(-nl // 64)          # the whole stack in one persistent launch per 64 layers
@@ -417,6 +418,8 @@ def run_ours(args):
             "gpu_launches": args.steps * launches,
             "kernel": ("persistent decode kernel over k-major down projections (dp4a)" if kmajor else
                        "row-major single-launch kernel (dp4a)" if m <= 2 else
+                       "streaming tcgen05 kernel (TMA-tiled weights, accumulators and converted operand in tensor memory)"
+                       if world == 1 and L.load().ffn_int4_set_batched_kernel(-1) == 2 else
                        "batched pair (tcgen05, accumulators and converted operand in tensor memory)"
                        if L.load().ffn_int4_set_batched_kernel(-1) == 0 or (L.load().ffn_int4_set_batched_kernel(-1) == 2 and m > 16 and 2 * ((i // tp) // 64) >= 148)
                        else "batched pair (mma.sync bf16)"),
@@ -617,7 +620,7 @@ def run_gemv(args):
                                                      "plan": plan.value.decode()},
                       "roofline": {"bound": "hbm", "achieved": round(bytes_per / us / 1e3, 1), "peak": peak, "unit": "GB/s",
                                    "frac": round(bytes_per / us / 1e3 / peak, 4), "peak_source": peak_kind},
-                      "gpu_launches": args.steps}), flush=True)
+                      "gpu_launches": args.steps * (1 if m <= 2 else 2 * -(-m // 512))}), flush=True)
 
 
 def main():
