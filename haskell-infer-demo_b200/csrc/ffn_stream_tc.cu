@@ -380,6 +380,7 @@ __global__ void __launch_bounds__(StPlan<NP>::kThreads, 1) stream_tc_kernel(cons
     } else {
         /* ---------------- epilogue ---------------- */
         constexpr int COLS = L::kCols;
+        constexpr bool kTight = PAIRS && NP > 64; /* no registers to spare: 72 a thread */
         const int quadrant = warp & 3, c0 = (warp >> 2) * COLS;
         const uint32_t d_lane = tmem + ((uint32_t)(quadrant * 32) << 16) + (uint32_t)c0;
         /* this lane's row of block b; rows past a ragged end read the last row's scales */
@@ -466,30 +467,76 @@ __global__ void __launch_bounds__(StPlan<NP>::kThreads, 1) stream_tc_kernel(cons
                 if (!ok) break;
                 if (++unit == U || i + 1 == count) {
                     /* the end of a block, or of this CTA's piece of the line */
-                    const long long first = (long long)block * U, last = first + U;
                     const int rb = block / P.token_blocks, tb = block % P.token_blocks;
                     bool finish = true;
-                    if (first < it0 || last > it1) {
-                        /* slot 0: the block began in an earlier CTA; 1: it begins here */
-                        const size_t per_slot = (size_t)NP * kTcRows, mine = (size_t)c0 * kTcRows + quadrant * 32 + lane;
-                        float *to = P.partial + ((size_t)blockIdx.x * 2 + (it0 > first ? 0 : 1)) * per_slot + mine;
+                    if constexpr (kTight) {
+                        /* As below without the shortcut.  Any change to this path has cost more in spills, in the loop
+                         * above, than the hand-over takes: 5120 x 17408, 128 tokens 98 us so, 101 to 104 with it. */
+                        const long long first = (long long)block * U, last = first + U;
+                        if (first < it0 || last > it1) {
+                            /* slot 0: the block began in an earlier CTA; 1: it begins here */
+                            const size_t per_slot = (size_t)NP * kTcRows, mine = (size_t)c0 * kTcRows + quadrant * 32 + lane;
+                            float *to = P.partial + ((size_t)blockIdx.x * 2 + (it0 > first ? 0 : 1)) * per_slot + mine;
 #pragma unroll
-                        for (int c = 0; c < COLS; ++c) __stcg(to + c * kTcRows, acc[c]);
-                        __threadfence();
-                        __syncwarp();
-                        /* CTA q holds unit u when q = floor(((u + 1) * CTAs - 1) / total) */
-                        const int q0 = (int)(((first + 1) * gridDim.x - 1) / total), q1 = (int)((last * gridDim.x - 1) / total);
-                        unsigned before = 0;
-                        if (lane == 0) before = atomicAdd(P.arrivals + (size_t)q0 * kStMaxEpiWarps + warp, 1u);
-                        finish = __shfl_sync(~0u, before, 0) == (unsigned)(q1 - q0);
-                        if (finish) {
+                            for (int c = 0; c < COLS; ++c) __stcg(to + c * kTcRows, acc[c]);
                             __threadfence();
+                            __syncwarp();
+                            /* CTA q holds unit u when q = floor(((u + 1) * CTAs - 1) / total) */
+                            const int q0 = (int)(((first + 1) * gridDim.x - 1) / total), q1 = (int)((last * gridDim.x - 1) / total);
+                            unsigned before = 0;
+                            if (lane == 0) before = atomicAdd(P.arrivals + (size_t)q0 * kStMaxEpiWarps + warp, 1u);
+                            finish = __shfl_sync(~0u, before, 0) == (unsigned)(q1 - q0);
+                            if (finish) {
+                                __threadfence();
 #pragma unroll
-                            for (int c = 0; c < COLS; ++c) acc[c] = 0.0f;
-                            for (int q = q0; q <= q1; ++q) {
-                                const float *from = P.partial + ((size_t)q * 2 + (total * q / gridDim.x > first ? 0 : 1)) * per_slot + mine;
+                                for (int c = 0; c < COLS; ++c) acc[c] = 0.0f;
+                                for (int q = q0; q <= q1; ++q) {
+                                    const float *from = P.partial + ((size_t)q * 2 + (total * q / gridDim.x > first ? 0 : 1)) * per_slot + mine;
 #pragma unroll
-                                for (int c = 0; c < COLS; ++c) acc[c] += __ldcg(from + c * kTcRows);
+                                    for (int c = 0; c < COLS; ++c) acc[c] += __ldcg(from + c * kTcRows);
+                                }
+                            }
+                        }
+                    } else {
+                        const bool begins_here = i + 1 >= unit;
+                        const bool ends_here = unit == U;
+                        if (!begins_here || !ends_here) {
+                            const long long line = (long long)P.blocks * U, first = (long long)block * U;
+                            /* slot 0: the block began in an earlier CTA; 1: it begins here */
+                            const size_t per_slot = (size_t)NP * kTcRows, mine = (size_t)c0 * kTcRows + quadrant * 32 + lane;
+                            /* CTA q holds unit u when q = floor(((u + 1) * CTAs - 1) / line) */
+                            const int q0 = (int)(((first + 1) * gridDim.x - 1) / line), q1 = (int)(((first + U) * gridDim.x - 1) / line);
+                            unsigned *arrive = P.arrivals + (size_t)q0 * kStMaxEpiWarps + warp;
+                            /* The others take their piece of a block first in their lines, the CTA in which it begins takes
+                             * its own last, at the end of the launch: it usually finds them all there, and then neither
+                             * hands over its sums nor waits for them (5120 x 17408, 8 tokens 49.5 -> 46.7 us; LM head, 5 rows
+                             * 132 -> 128). */
+                            bool all_there = false;
+                            if (begins_here) {
+                                unsigned seen = 0;
+                                if (lane == 0) seen = ld_acquire_gpu(arrive);
+                                all_there = __shfl_sync(~0u, seen, 0) == (unsigned)(q1 - q0);
+                            }
+                            if (!all_there) {
+                                float *to = P.partial + ((size_t)blockIdx.x * 2 + (begins_here ? 1 : 0)) * per_slot + mine;
+#pragma unroll
+                                for (int c = 0; c < COLS; ++c) __stcg(to + c * kTcRows, acc[c]);
+                                __threadfence();
+                                __syncwarp();
+                                unsigned before = 0;
+                                if (lane == 0) before = atomicAdd(arrive, 1u);
+                                finish = __shfl_sync(~0u, before, 0) == (unsigned)(q1 - q0);
+                            }
+                            if (finish) {
+                                /* in CTA order, from zero; sums still in registers are the first CTA's */
+                                __threadfence();
+#pragma unroll
+                                for (int c = 0; c < COLS; ++c) acc[c] = all_there ? 0.0f + acc[c] : 0.0f;
+                                for (int q = all_there ? q0 + 1 : q0; q <= q1; ++q) {
+                                    const float *from = P.partial + ((size_t)q * 2 + (line * q / gridDim.x > first ? 0 : 1)) * per_slot + mine;
+#pragma unroll
+                                    for (int c = 0; c < COLS; ++c) acc[c] += __ldcg(from + c * kTcRows);
+                                }
                             }
                         }
                     }
