@@ -1,5 +1,5 @@
 """The GPU quantizer's rounding where the quotient is a half or next to one, at scales from the smallest to the
-largest that the format holds, and both ways of delivering the bytes: byte for byte against the CPU checker."""
+largest that the format holds, and both ways of delivering the bytes: byte for byte against the CPU oracle."""
 import numpy as np
 import pytest
 import torch
