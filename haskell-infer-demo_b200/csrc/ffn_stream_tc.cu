@@ -487,6 +487,7 @@ __global__ void __launch_bounds__(StPlan<NP>::kThreads, 1) stream_tc_kernel(cons
                             if (lane == 0) before = atomicAdd(P.arrivals + (size_t)q0 * kStMaxEpiWarps + warp, 1u);
                             finish = __shfl_sync(~0u, before, 0) == (unsigned)(q1 - q0);
                             if (finish) {
+                                __syncwarp(); /* lane 0's count before the other lanes' loads: a shuffle orders no memory */
                                 __threadfence();
 #pragma unroll
                                 for (int c = 0; c < COLS; ++c) acc[c] = 0.0f;
@@ -529,6 +530,7 @@ __global__ void __launch_bounds__(StPlan<NP>::kThreads, 1) stream_tc_kernel(cons
                             }
                             if (finish) {
                                 /* in CTA order, from zero; sums still in registers are the first CTA's */
+                                __syncwarp(); /* as above */
                                 __threadfence();
 #pragma unroll
                                 for (int c = 0; c < COLS; ++c) acc[c] = all_there ? 0.0f + acc[c] : 0.0f;
