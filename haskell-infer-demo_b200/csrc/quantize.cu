@@ -15,7 +15,7 @@
  * launch moves the bytes to the caller once nothing was refused - it looks at the verdict itself, so the host
  * waits once, at the end.  5120 x 17408: 221 us with a checking and a writing pass over the input, a wait
  * between them and cudaMalloc / cudaFree around them; 118 now.  Where the bytes exceed the scratch that
- * the library keeps (kScratchMost) the second launch quantizes again instead.
+ * the library keeps (kScratchMost), or there is no memory for them, the second launch quantizes again instead.
  *
  * Eight lanes per group: a lane holds sixteen elements in four 16-byte loads (128 contiguous bytes of a group
  * each), so the group's division, reciprocal and reduction are paid once per sixteen elements: instructions, not
@@ -136,11 +136,15 @@ extern "C" int ffn_quantize_int4(const void *weights, void *packed, void *scales
         return fail(FFN_ERR_CONFIG, "ffn_quantize_int4: weights must be 16-byte aligned, outputs 2-byte aligned");
     const long long groups = n * (k / FFN_INT4_GROUP);
     const long long packed_bytes = n * k / 2, scale_bytes = groups * 2;
-    const bool keep = (size_t)(packed_bytes + scale_bytes) <= kScratchMost;
+    bool keep = (size_t)(packed_bytes + scale_bytes) <= kScratchMost;
     const size_t scales_at = 256 + ((size_t)packed_bytes + 255) / 256 * 256;
     uint8_t *scratch = nullptr;
-    if (scratch_alloc((void **)&scratch, keep ? scales_at + (size_t)scale_bytes : 256, stream) != FFN_OK)
-        return fail(FFN_ERR_ALLOC, "ffn_quantize_int4: cannot allocate the status words");
+    const bool pooled = scratch_alloc((void **)&scratch, keep ? scales_at + (size_t)scale_bytes : 256, stream) == FFN_OK;
+    if (!pooled) {
+        /* no room for the bytes (the call is made while weights fill the device): two passes and the status words */
+        keep = false;
+        if (cudaMalloc(&scratch, sizeof(QuantStatus)) != cudaSuccess) { (void)cudaGetLastError(); return fail(FFN_ERR_ALLOC, "ffn_quantize_int4: cannot allocate the status words"); }
+    }
     QuantStatus *status = (QuantStatus *)scratch;
     int rc = FFN_OK;
     QuantStatus host;
@@ -152,7 +156,7 @@ extern "C" int ffn_quantize_int4(const void *weights, void *packed, void *scales
                                                                        keep ? (uint16_t *)(scratch + scales_at) : nullptr, groups, status);
         if (!keep) {
             quantize_int4_kernel<false><<<grid, kQuantThreads, 0, stream>>>((const float *)weights, (uint8_t *)packed, (uint16_t *)scales, groups, status);
-        } else if (!(((uintptr_t)packed | (uintptr_t)scales | (uintptr_t)scale_bytes) & 15)) {
+        } else if (!(((uintptr_t)packed | (uintptr_t)scales) & 15)) { /* both counts are multiples of 16: n % 8 == 0, k % 128 == 0 */
             quantize_deliver_kernel<uint4><<<148 * 8, kQuantThreads, 0, stream>>>((uint4 *)packed, (const uint4 *)(scratch + 256), packed_bytes / 16, (uint4 *)scales,
                                                                                   (const uint4 *)(scratch + scales_at), scale_bytes / 16, status);
         } else {
@@ -176,6 +180,7 @@ extern "C" int ffn_quantize_int4(const void *weights, void *packed, void *scales
             break;
         }
     } while (0);
-    (void)cudaFreeAsync(scratch, stream);
+    if (pooled) (void)cudaFreeAsync(scratch, stream);
+    else cudaFree(scratch);
     return rc;
 }
