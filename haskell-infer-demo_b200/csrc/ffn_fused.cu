@@ -551,7 +551,13 @@ static int device_state(DeviceState **out) {
         FFN_CUDA_TRY(cudaDeviceGetAttribute(&d.cooperative, cudaDevAttrCooperativeLaunch, dev), "cooperative launch");
         if (cudaMalloc(&d.sync, 4 * sizeof(unsigned)) != cudaSuccess)
             return fail(FFN_ERR_ALLOC, "cannot allocate the kernel's synchronisation words");
-        FFN_CUDA_TRY(cudaMemset(d.sync, 0, 4 * sizeof(unsigned)), "clear synchronisation words");
+        /* not on the legacy stream: that one may not be used while another thread captures a blocking stream */
+        if (cudaMemsetAsync(d.sync, 0, 4 * sizeof(unsigned), cudaStreamPerThread) != cudaSuccess || cudaStreamSynchronize(cudaStreamPerThread) != cudaSuccess) {
+            const cudaError_t e = cudaGetLastError();
+            cudaFree(d.sync);
+            d.sync = nullptr;
+            return fail(FFN_ERR_CUDA, "clear synchronisation words: %s", cudaGetErrorString(e));
+        }
         d.ready = true;
     }
     *out = &d;

@@ -39,7 +39,6 @@
  */
 #include <stdio.h>
 
-#include <atomic>
 #include <mutex>
 
 #include "kernels.h"
@@ -789,21 +788,32 @@ int scratch_alloc(void **out, size_t bytes, cudaStream_t stream) {
     return FFN_NOT_ADMITTED;
 }
 
+/* The calling thread may allocate although another thread captures a stream in global mode: what the scope
+ * allocates belongs to no capture. */
+struct OutsideOtherCaptures {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    OutsideOtherCaptures() { (void)cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~OutsideOtherCaptures() { (void)cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
 int stream_tc_gemm(const void *a, const void *packed, const void *scales, void *out, int M, int N, int K, cudaStream_t stream) {
     int dev = 0, sm_count = 0, st = st_device(&dev, &sm_count);
     if (st) return st;
-    /* The device's first call creates the status word and the pool, which a stream that is being captured must
-     * not do: such a call takes the shape-generic kernel, as every call of three rows and more once did. */
-    static std::atomic<bool> ready[64];
-    if (!ready[dev].load()) {
-        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-        if (cudaStreamIsCapturing(stream, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone) {
-            (void)cudaGetLastError();
-            return FFN_NOT_ADMITTED;
-        }
+    /* Scratch from the pool would put allocation and free nodes into a graph, which then can be neither
+     * instantiated twice nor cloned nor used as a child, and scratch of the graph's own could be shared by two of its
+     * instances at once.  A captured call takes the shape-generic kernel, which needs none. */
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(stream, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone) {
+        (void)cudaGetLastError();
+        return FFN_NOT_ADMITTED;
     }
+    const OutsideOtherCaptures scope;
     unsigned *status = nullptr;
-    if ((st = fused_status_word(&status))) return st;
+    if ((st = fused_status_word(&status))) { /* no memory for it: the shape-generic kernel needs none */
+        (void)cudaGetLastError();
+        clear_error();
+        return FFN_NOT_ADMITTED;
+    }
     const StTokens most = st_tokens(M < kStSlab ? M : kStSlab);
     const size_t counters = st_counter_bytes(sm_count), partial = st_partial_bytes(sm_count, M <= kStSlab ? most.np : kStMaxTokens);
     const size_t tiles = M <= kStSlab ? st_tile_bytes(most, K) : st_round((size_t)kStSlab * K * 2);
@@ -811,7 +821,6 @@ int stream_tc_gemm(const void *a, const void *packed, const void *scales, void *
     if ((st = weight_tile_map(&P.wmap, packed, N, K, kTcRows))) return st;
     uint8_t *base = nullptr;
     if ((st = scratch_alloc((void **)&base, counters + partial + tiles, stream))) return st;
-    ready[dev].store(true);
     for (int m0 = 0; m0 < M && st == FFN_OK; m0 += kStSlab) {
         const int m = M - m0 < kStSlab ? M - m0 : kStSlab;
         const StTokens t = st_tokens(m);
