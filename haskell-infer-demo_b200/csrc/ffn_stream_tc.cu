@@ -701,14 +701,50 @@ bool stream_tc_describe(int tokens, int K, int smem_optin, char *out, size_t out
     return true;
 }
 
-/* Scratch of the FFN pair per device, sized for a whole slab of tokens and grown for larger layers (calls
- * on one device are serialised by the caller). */
+/* Scratch of the FFN pair, per device one for calls of up to 64 tokens and one for longer ones (42 MB for a
+ * launch of 512 tokens of a 5120 x 17408 layer, 13 MB for 64: what the pairs take).  Each is allocated by the
+ * first call of its class and grown for larger layers (calls on one device are serialised by the caller). */
+constexpr int kStSmallSlab = 64;
 struct StScratch {
     uint8_t *base = nullptr;
     size_t bytes = 0;
 };
-static StScratch g_st_scratch[64];
+static StScratch g_st_scratch[64][2];
 static std::mutex g_st_mutex;
+
+struct StLayout { /* [arrivals of both launches | partial sums | input | act] for launches of up to `slab` tokens */
+    int slab;
+    size_t counters, partial, input, bytes;
+};
+static StLayout st_layout(int slab, int H, int I, int sm_count) {
+    const StTokens most = st_tokens(slab); /* both slabs are whole blocks: no smaller number of tokens takes more */
+    StLayout l;
+    l.slab = slab;
+    l.counters = st_counter_bytes(sm_count);
+    l.partial = st_partial_bytes(sm_count, most.np);
+    l.input = st_tile_bytes(most, H);
+    l.bytes = 2 * l.counters + l.partial + l.input + st_tile_bytes(most, I);
+    return l;
+}
+/* The scratch that holds `bytes`, or none: there is no memory for it, or it would have to be allocated while the
+ * stream is being captured.  What is there stays until the larger one is had. */
+static int st_reserve(StScratch &sc, size_t bytes, cudaStream_t stream) {
+    if (sc.bytes >= bytes) return FFN_OK;
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(stream, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone) {
+        (void)cudaGetLastError();
+        return FFN_NOT_ADMITTED;
+    }
+    uint8_t *base = nullptr;
+    if (cudaMalloc(&base, bytes) != cudaSuccess) { (void)cudaGetLastError(); return FFN_NOT_ADMITTED; }
+    if (sc.base) {
+        const cudaError_t e = cudaDeviceSynchronize();
+        if (e != cudaSuccess) { cudaFree(base); return fail(FFN_ERR_CUDA, "streaming tcgen05: scratch regrow: %s", cudaGetErrorString(e)); }
+        cudaFree(sc.base);
+    }
+    sc.base = base; sc.bytes = bytes;
+    return FFN_OK;
+}
 
 int stream_tc_ffn_launch(cudaStream_t stream, const void *x, void *act, void *layer_out, const FfnMlpWeights *w, int tokens, int H,
                          int I, void *residual, const FusedNorm *norm, void *normed, unsigned *status) {
@@ -716,37 +752,36 @@ int stream_tc_ffn_launch(cudaStream_t stream, const void *x, void *act, void *la
     if (((uintptr_t)w->gate_up_i4 & 15) || ((uintptr_t)w->down_i4 & 15) || ((uintptr_t)x & 15) || ((uintptr_t)normed & 15)) return FFN_NOT_ADMITTED;
     int dev = 0, sm_count = 0, st = st_device(&dev, &sm_count);
     if (st) return st;
-    /* layout: [arrivals of both launches | partial sums | input | act] */
-    const StTokens most = {kStSlab / kStMaxTokens, kStMaxTokens, kStMaxTokens};
-    const size_t counters = st_counter_bytes(sm_count), partial = st_partial_bytes(sm_count, kStMaxTokens);
-    const size_t want = 2 * counters + partial + st_tile_bytes(most, H) + st_tile_bytes(most, I);
     std::lock_guard<std::mutex> lock(g_st_mutex);
-    StScratch &sc = g_st_scratch[dev];
-    if (sc.bytes < want) {
-        if (sc.base) { FFN_CUDA_TRY(cudaDeviceSynchronize(), "streaming tcgen05: scratch regrow"); cudaFree(sc.base); }
-        sc.base = nullptr; sc.bytes = 0;
-        if (cudaMalloc(&sc.base, want) != cudaSuccess) { (void)cudaGetLastError(); return fail(FFN_ERR_ALLOC, "streaming tcgen05: cannot allocate %zu bytes of scratch", want); }
-        sc.bytes = want;
+    /* a long call makes do with launches of 64 tokens, and the pairs serve where there is no room for that either */
+    bool large = tokens > kStSmallSlab;
+    StLayout l = st_layout(large ? kStSlab : kStSmallSlab, H, I, sm_count);
+    st = st_reserve(g_st_scratch[dev][large], l.bytes, stream);
+    if (st == FFN_NOT_ADMITTED && large) {
+        large = false;
+        l = st_layout(kStSmallSlab, H, I, sm_count);
+        st = st_reserve(g_st_scratch[dev][large], l.bytes, stream);
     }
+    if (st) return st;
+    uint8_t *base = g_st_scratch[dev][large].base, *partial = base + 2 * l.counters, *xt = partial + l.partial, *act_t = xt + l.input;
     StreamTcParams A = {}, B = {};
     if ((st = weight_tile_map(&A.wmap, w->gate_up_i4, 2 * I, H, 64))) return st;
     if ((st = weight_tile_map(&B.wmap, w->down_i4, H, I, kTcRows))) return st;
-    for (int m0 = 0; m0 < tokens; m0 += kStSlab) {
-        const int m = tokens - m0 < kStSlab ? tokens - m0 : kStSlab;
+    for (int m0 = 0; m0 < tokens; m0 += l.slab) {
+        const int m = tokens - m0 < l.slab ? tokens - m0 : l.slab;
         const StTokens t = st_tokens(m);
-        uint8_t *xt = sc.base + 2 * counters + partial, *act_t = xt + st_tile_bytes(most, H);
-        if ((st = st_tile_input(xt, (const uint16_t *)x + (size_t)m0 * H, norm, normed ? (uint16_t *)normed + (size_t)m0 * H : nullptr, m, t, H, (unsigned *)sc.base, 2 * counters, stream))) return st;
+        if ((st = st_tile_input(xt, (const uint16_t *)x + (size_t)m0 * H, norm, normed ? (uint16_t *)normed + (size_t)m0 * H : nullptr, m, t, H, (unsigned *)base, 2 * l.counters, stream))) return st;
         A.s = (const uint16_t *)w->gate_up_i4_scales; A.xt = xt;
         A.M = m; A.per_block = t.per_block; A.token_blocks = t.blocks;
         A.N = I; A.K = H; A.up_offset = I; A.blocks = (I / 64) * t.blocks;
         A.out = (uint16_t *)act + (size_t)m0 * I; A.act_t = act_t;
-        A.partial = (float *)(sc.base + 2 * counters); A.arrivals = (unsigned *)sc.base; A.status = status;
+        A.partial = (float *)partial; A.arrivals = (unsigned *)base; A.status = status;
         if ((st = st_launch_np<true>(A, t.np, st_ctas(A.blocks, H / FFN_INT4_GROUP, sm_count), stream))) return st;
         B.s = (const uint16_t *)w->down_i4_scales; B.xt = act_t;
         B.M = m; B.per_block = t.per_block; B.token_blocks = t.blocks;
         B.N = H; B.K = I; B.blocks = (H / kTcRows) * t.blocks;
         B.out = (uint16_t *)layer_out + (size_t)m0 * H; B.residual = residual ? (uint16_t *)residual + (size_t)m0 * H : nullptr;
-        B.partial = A.partial; B.arrivals = (unsigned *)(sc.base + counters); B.status = status;
+        B.partial = A.partial; B.arrivals = (unsigned *)(base + l.counters); B.status = status;
         if ((st = st_launch_np<false>(B, t.np, st_ctas(B.blocks, I / FFN_INT4_GROUP, sm_count), stream))) return st;
     }
     return FFN_OK;

@@ -12,12 +12,16 @@
  *
  * Concurrency: the FFN entry points of one device (ffn_forward_mlp*, ffn_forward_mlp_tp,
  * ffn_decode_stack, ffn_gemm_int4_bf16 with one or two rows, ffn_tp_allreduce_sum) share that
- * device's synchronisation words, kernel status word and, from three tokens on, one scratch region
- * (activations in the kernels' order, split-K partial sums, arrival counters; sized for 512 tokens of
- * the largest layer seen: 42 MB for 5120 x 17408).  Calls on one device must
+ * device's synchronisation words, kernel status word and, from three tokens on, a scratch region for
+ * calls of up to 64 tokens and one for longer ones (activations in the kernels' order, split-K partial
+ * sums, arrival counters; sized for 64 and for 512 tokens of the largest layer seen: 13 and 42 MB for
+ * 5120 x 17408).  Calls on one device must
  * therefore be serialised: issue them on one stream, or order the streams with events.  Calls on
  * different devices are independent.  The first call on a device, and the first call of the batched
- * path there, allocate these words with cudaMalloc: make them before capturing a CUDA graph.
+ * path there, allocate these words with cudaMalloc: make them before capturing a CUDA graph, the batched
+ * one with the largest layer (a larger layer replaces a region that a graph of a smaller one would still use).
+ * Where a longer call's region is missing - there is no memory for it, or no such call came before the
+ * capture - the call runs in launches of 64 tokens.
  *
  * Data layouts (identical to the reference's, csrc/include/linear_weight.h:12-13, 46-54):
  *   packed [N][K/2]   u8, row-major; byte j of a row = code(k=2j) | code(k=2j+1) << 4; codes are

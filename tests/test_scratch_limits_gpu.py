@@ -66,6 +66,34 @@ assert torch.equal(packed, want_p) and torch.equal(scales, want_s.view(torch.int
 print('quantized')
 """
 
+_FFN = _PREAMBLE + r"""
+h, i = 5120, 17408
+gen = torch.Generator(device='cuda').manual_seed(3)
+# any bytes are weights; made without the quantizer, whose pool would hold memory that the driver can take back
+weights = [(torch.randint(0, 256, (n, k // 2), dtype=torch.uint8, device='cuda', generator=gen),
+            (0.002 + 0.002 * torch.rand((n, k // 128), device='cuda', generator=gen)).to(torch.bfloat16)) for n, k in ((2 * i, h), (h, i))]
+torch.cuda.synchronize()
+torch.cuda.empty_cache()
+mlp = ops.DenseMlp(*weights[0], *weights[1])
+state = {}
+for m in (3, 128):
+    x = torch.randn((m, h), device='cuda', generator=gen).to(torch.bfloat16)
+    state[m] = x, mlp.workspace(m), torch.empty_like(x)
+mlp.forward_mlp_prepared(state[3][0][:1].contiguous())             # the status word
+torch.cuda.synchronize()
+with Full(20 << 20):                                               # the pairs need 14 MB, 512 tokens' scratch 42
+    got = {m: (mlp.forward_mlp_prepared(*state[m]), L.device_status())[0].clone() for m in state}
+for m in state:
+    want = mlp.forward_mlp_prepared(*state[m])
+    L.device_status()
+    # another split of the tokens and of K over CTAs: FP32 order, then BF16 roundings of act and y
+    err = ((got[m].float() - want.float()).norm() / want.float().norm()).item()
+    print(m, 'tokens, relative difference', err)
+    assert err <= 2.0 ** -8
+print('computed')
+"""
+
+
 def child(code):
     proc = subprocess.run([sys.executable, "-c", code, ROOT], capture_output=True, text=True, timeout=600,
                           env=dict(os.environ, CUDA_MODULE_LOADING="EAGER"))
@@ -75,3 +103,7 @@ def child(code):
 
 def test_quantizer_needs_a_few_bytes_only(cuda):
     assert "quantized" in child(_QUANTIZER)
+
+
+def test_batched_ffn_makes_do_with_what_the_pairs_needed(cuda):
+    assert "computed" in child(_FFN)
