@@ -354,7 +354,8 @@ int ffn_forward_mlp(void *cublas, void *stream, const void *residual, void *ws, 
     const void *normed = residual;
     if (w->post_norm_w) {
         if (!(dims->rms_eps > 0.0f)) return fail(FFN_ERR_CONFIG, "ffn_forward_mlp: invalid shape or epsilon");
-        if (g_fused_enabled && tokens > 2) { /* the norm in the input stage of the FFN's own kernels */
+        /* the norm in the input stage of the FFN's own kernels; a prepared layer's opt-in kernel comes first (mlp_common) */
+        if (g_fused_enabled && tokens > 2 && !(tokens <= 4 && ffn_decode_layer_is_prepared(w))) {
             const FusedNorm norm = {w->post_norm_w, dims->rms_eps, dims->norm_style == 0};
             uint16_t *act = (uint16_t *)ws + (size_t)tokens * dims->hidden_size + (size_t)2 * tokens * dims->intermediate_size;
             unsigned *status = nullptr;
