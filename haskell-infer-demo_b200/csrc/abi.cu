@@ -151,7 +151,7 @@ int ffn_int4_describe_plan(int tokens, int hidden, int intermediate, int sm_coun
             snprintf(out + used, out_bytes - used, " passes=%d", (tokens + 63) / 64);
         }
         char one[160]; /* without tensor parallelism the streaming kernel comes first */
-        if (stream_tc_describe(tokens, hidden, smem_optin, one, sizeof(one))) {
+        if (tc_get_mode() == 2 && stream_tc_describe(tokens, hidden, smem_optin, one, sizeof(one))) {
             const size_t used = strlen(out);
             snprintf(out + used, out_bytes - used, " one_rank_kernel=%s", one);
         }

@@ -694,7 +694,7 @@ static int st_device(int *dev, int *sm_count) {
 }
 
 bool stream_tc_describe(int tokens, int K, int smem_optin, char *out, size_t out_bytes) {
-    if (tokens < 3 || tc_get_mode() != 2 || smem_optin < kStSmem) return false;
+    if (tokens < 3 || smem_optin < kStSmem) return false;
     const StTokens t = st_tokens(tokens < kStSlab ? tokens : kStSlab);
     snprintf(out, out_bytes, "stream_tc columns=%d token_blocks=%d launches_of_%d_tokens=%d units_per_block=%d", t.np, t.blocks, kStSlab,
              (tokens + kStSlab - 1) / kStSlab, (K / FFN_INT4_GROUP + 1) / 2);

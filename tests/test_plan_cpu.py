@@ -85,6 +85,22 @@ def test_batched_plan(tokens, hidden, inter, tp):
     assert 1 <= p["down_k_splits"] <= 8 and p["down_k_splits"] * 2 <= max(local // 128, 2)
 
 
+@pytest.mark.parametrize("switch", [0, 1, 2])
+def test_the_batched_switch_concerns_the_ffn_alone(switch):
+    def gemm(m, smem=SMEM):
+        buf = ctypes.create_string_buffer(1024)
+        assert L.load().ffn_int4_describe_gemm_plan(m, 12288, 5120, SMS, smem, buf, len(buf)) == 0
+        return buf.value.decode()
+    old = L.load().ffn_int4_set_batched_kernel(switch)
+    try:
+        for m in (3, 16, 64, 128, 700):
+            assert gemm(m).startswith("kernel=stream_tc ")
+            assert gemm(m, 100 * 1024).startswith("kernel=generic ")
+            assert ("one_rank_kernel" in plan(m, 5120, 17408)) == (switch == 2)
+    finally:
+        L.load().ffn_int4_set_batched_kernel(old)
+
+
 def test_long_batches_run_in_blocks_of_64_and_small_devices_fall_back():
     assert plan(100, 5120, 17408)["passes"] == 2
     assert plan(4, 5120, 17408, smem=40 * 1024)["kernel"] == "generic"   # no room for the pair's pipeline
