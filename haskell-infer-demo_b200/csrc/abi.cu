@@ -150,8 +150,8 @@ int ffn_int4_describe_plan(int tokens, int hidden, int intermediate, int sm_coun
             const size_t used = strlen(out);
             snprintf(out + used, out_bytes - used, " passes=%d", (tokens + 63) / 64);
         }
-        char one[160]; /* without tensor parallelism the streaming kernel comes first */
-        if (tc_get_mode() == 2 && stream_tc_describe(tokens, hidden, smem_optin, one, sizeof(one))) {
+        char one[200]; /* without tensor parallelism the streaming kernel comes first (its gate/up launch) */
+        if (tc_get_mode() == 2 && stream_tc_describe(tokens, 2 * intermediate, hidden, sm_count, smem_optin, one, sizeof(one))) {
             const size_t used = strlen(out);
             snprintf(out + used, out_bytes - used, " one_rank_kernel=%s", one);
         }
@@ -212,8 +212,8 @@ int ffn_int4_describe_gemm_plan(int m, int n, int k, int sm_count, int smem_opti
     if (m < 1 || n <= 0 || k <= 0 || k % FFN_INT4_GROUP || sm_count < 1 || smem_optin < 1)
         return fail(FFN_ERR_CONFIG, "ffn_int4_describe_gemm_plan: invalid shape or device description");
     if (m <= 2 && gemv_describe_plan(m, n, k, sm_count, smem_optin, out, out_bytes)) return FFN_OK;
-    char stream[160];
-    if (stream_tc_describe(m, k, smem_optin, stream, sizeof(stream))) snprintf(out, out_bytes, "kernel=%s", stream);
+    char stream[200];
+    if (stream_tc_describe(m, n, k, sm_count, smem_optin, stream, sizeof(stream))) snprintf(out, out_bytes, "kernel=%s", stream);
     else snprintf(out, out_bytes, "kernel=generic launches=1");
     return FFN_OK;
 }

@@ -534,7 +534,7 @@ __global__ void __launch_bounds__(StPlan<NP>::kThreads, 1) stream_tc_kernel(cons
 #pragma unroll
                                 for (int c = 0; c < COLS; ++c) acc[c] = all_there ? 0.0f + acc[c] : 0.0f;
                                 for (int q = all_there ? q0 + 1 : q0; q <= q1; ++q) {
-                                    const float *from = P.partial + ((size_t)q * 2 + (line * q / gridDim.x > first ? 0 : 1)) * per_slot + mine;
+                                    const float *from = P.partial + ((size_t)q * 2 + (q == q0 ? 1 : 0)) * per_slot + mine; /* it begins in q0 */
 #pragma unroll
                                     for (int c = 0; c < COLS; ++c) acc[c] += __ldcg(from + c * kTcRows);
                                 }
@@ -628,9 +628,15 @@ static StTokens st_tokens(int tokens) {
     t.np = (t.per_block + 15) / 16 * 16;
     return t;
 }
-/* One CTA per SM, and none without a unit. */
+/* One CTA per SM, and none without a unit; where that would split a block among many, fewer.  With p of its U units
+ * to a CTA the launch takes p steps and then, one after the other, the sums of U / p contributors, a trip to L2
+ * each, which costs about a step: p = sqrt(U).  us per FFN at 3 tokens, one unit a CTA -> so: 1024 x 3072 20.4 ->
+ * 13.6, 512 x 8192 28.1 -> 16.9, 2560 x 9728 24.9 -> 22.8; 5120 x 17408 has more blocks than it concerns (44.1). */
 static int st_ctas(int blocks, int G, int sm_count) {
-    const long long n = (long long)blocks * ((G + 1) / 2);
+    const int U = (G + 1) / 2;
+    int share = 1;
+    while (share * share < U) ++share;
+    const long long n = (long long)blocks * share;
     return n < sm_count ? (int)n : sm_count;
 }
 static size_t st_counter_bytes(int sm_count) { return st_round((size_t)sm_count * kStMaxEpiWarps * sizeof(unsigned)); }
@@ -693,11 +699,12 @@ static int st_device(int *dev, int *sm_count) {
     return smem >= kStSmem ? FFN_OK : FFN_NOT_ADMITTED;
 }
 
-bool stream_tc_describe(int tokens, int K, int smem_optin, char *out, size_t out_bytes) {
+bool stream_tc_describe(int tokens, int N, int K, int sm_count, int smem_optin, char *out, size_t out_bytes) {
     if (tokens < 3 || smem_optin < kStSmem) return false;
     const StTokens t = st_tokens(tokens < kStSlab ? tokens : kStSlab);
-    snprintf(out, out_bytes, "stream_tc columns=%d token_blocks=%d launches_of_%d_tokens=%d units_per_block=%d", t.np, t.blocks, kStSlab,
-             (tokens + kStSlab - 1) / kStSlab, (K / FFN_INT4_GROUP + 1) / 2);
+    const int row_blocks = (N + kTcRows - 1) / kTcRows;
+    snprintf(out, out_bytes, "stream_tc columns=%d token_blocks=%d launches_of_%d_tokens=%d units_per_block=%d row_blocks=%d ctas=%d", t.np, t.blocks, kStSlab,
+             (tokens + kStSlab - 1) / kStSlab, (K / FFN_INT4_GROUP + 1) / 2, row_blocks, st_ctas(row_blocks * t.blocks, K / FFN_INT4_GROUP, sm_count));
     return true;
 }
 

@@ -171,7 +171,7 @@ int stream_tc_ffn_launch(cudaStream_t stream, const void *x, void *act, void *la
                          int I, void *residual, const FusedNorm *norm, void *normed, unsigned *status);
 /* How that kernel would take the call, as text after "kernel="; false when it does not.  The batched switch, which
  * concerns the FFN alone, is the caller's to ask. */
-bool stream_tc_describe(int tokens, int K, int smem_optin, char *out, size_t out_bytes);
+bool stream_tc_describe(int tokens, int N, int K, int sm_count, int smem_optin, char *out, size_t out_bytes);
 int scratch_alloc(void **out, size_t bytes, cudaStream_t stream); /* stream-ordered; FFN_NOT_ADMITTED when there is none */
 int stream_tc_gemm(const void *a, const void *packed, const void *scales, void *out, int M, int N, int K, cudaStream_t stream);
 /* Device address of the status word shared by the kernels of this library (allocating it on first use). */

@@ -101,6 +101,18 @@ def test_the_batched_switch_concerns_the_ffn_alone(switch):
         L.load().ffn_int4_set_batched_kernel(old)
 
 
+@pytest.mark.parametrize("m,n,k", [(16, 128, 17408), (9, 1024, 3072), (32, 512, 24576), (27, 5120, 17408), (12, 264, 128), (16, 130, 256), (512, 12288, 5120)])
+def test_a_block_is_split_among_the_square_root_of_its_units(m, n, k):
+    buf = ctypes.create_string_buffer(1024)
+    assert L.load().ffn_int4_describe_gemm_plan(m, n, k, SMS, SMEM, buf, len(buf)) == 0
+    p = {f: int(v) for f, v in (t.split("=") for t in buf.value.decode().split()[1:])}
+    blocks, units = p["row_blocks"] * p["token_blocks"], p["units_per_block"]
+    assert p["row_blocks"] == -(-n // 128) and units == -(-k // 256)
+    share = next(s for s in range(1, units + 1) if s * s >= units)
+    assert p["ctas"] == min(SMS, blocks * share)
+    assert p["ctas"] <= blocks * units                       # no CTA without a unit
+
+
 def test_long_batches_run_in_blocks_of_64_and_small_devices_fall_back():
     assert plan(100, 5120, 17408)["passes"] == 2
     assert plan(4, 5120, 17408, smem=40 * 1024)["kernel"] == "generic"   # no room for the pair's pipeline

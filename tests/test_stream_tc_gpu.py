@@ -12,7 +12,7 @@ from oracle import ffn_oracle as o
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("n,k", [(8, 128), (264, 256), (4104, 1280), (37896, 512), (512, 17408)])
+@pytest.mark.parametrize("n,k", [(8, 128), (264, 256), (4104, 1280), (37896, 512), (512, 17408), (128, 640)])
 @pytest.mark.parametrize("rows", [3, 16, 17, 33, 48, 64, 65, 81, 112, 128, 129, 300, 513])
 def test_gemm_against_fp64(cuda, rows, n, k):
     gen = torch.Generator(device="cuda").manual_seed(rows * 100003 + n)
