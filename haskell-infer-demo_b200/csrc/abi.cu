@@ -213,7 +213,7 @@ int ffn_int4_describe_gemm_plan(int m, int n, int k, int sm_count, int smem_opti
         return fail(FFN_ERR_CONFIG, "ffn_int4_describe_gemm_plan: invalid shape or device description");
     if (m <= 2 && gemv_describe_plan(m, n, k, sm_count, smem_optin, out, out_bytes)) return FFN_OK;
     char stream[200];
-    if (stream_tc_describe(m, n, k, sm_count, smem_optin, stream, sizeof(stream))) snprintf(out, out_bytes, "kernel=%s", stream);
+    if (!gemm_int4_generic_wins(m, n, k) && stream_tc_describe(m, n, k, sm_count, smem_optin, stream, sizeof(stream))) snprintf(out, out_bytes, "kernel=%s", stream);
     else snprintf(out, out_bytes, "kernel=generic launches=1");
     return FFN_OK;
 }

@@ -123,6 +123,20 @@ static int launch_rows(const uint16_t *a, const uint8_t *packed, const uint16_t 
     return FFN_OK;
 }
 
+/* Where three to eight rows are better off here than in the streaming tensor-core kernel, whose input pre-pass and
+ * scratch cost the host some 4 us more than one launch does: a small matrix, neither long nor wide, and few launches
+ * (8, 4, 2 and 1 rows each).  B200, us a call alone, this kernel / that one, on either side of the line:
+ *   4 rows  4096 x 2560 27 / 31   512 x 5120 31 / 32    16384 x 512 31 / 32 | 8192 x 2560 34 / 33  20480 x 512 34 / 31
+ *   8 rows  2048 x 2048 28 / 31   2048 x 2560 31 / 31                       | 4096 x 2560 32 / 31  512 x 4096 36 / 31
+ *   3 rows  2048 x 2048 29 / 31   2048 x 2560 32 / 32                       | 4096 x 2560 33 / 31  2048 x 3328 36 / 34
+ *   6 rows  1024 x 1024 28 / 30   4096 x 1024 28 / 30                       | 2048 x 2048 31 / 31 */
+bool gemm_int4_generic_wins(int M, int N, int K) {
+    if (M < 3 || M > 8 || M == 7) return false; /* seven rows are three launches */
+    const int launches = M == 4 || M == 8 ? 1 : 2;
+    return (long long)M * K <= (launches == 1 ? 20480 : 8192) && (long long)M * N * launches <= 65536 &&
+           (long long)M * N * K * launches <= 48ll << 20;
+}
+
 int gemm_int4_generic(const void *a, const void *packed, const void *scales, void *out_bf16,
                       float *out_f32, int M, int N, int K, cudaStream_t stream) {
     const uint16_t *ap = (const uint16_t *)a;

@@ -947,7 +947,7 @@ int gemm_int4_dispatch(const void *a, const void *packed, const void *scales, vo
     if (M <= 2) {
         const int st = gemv_int4_stream(a, packed, scales, out, M, N, K, stream);
         if (st != FFN_NOT_ADMITTED) return st;
-    } else {
+    } else if (!gemm_int4_generic_wins(M, N, K)) {
         const int st = stream_tc_gemm(a, packed, scales, out, M, N, K, stream);
         if (st != FFN_NOT_ADMITTED) return st;
     }

@@ -10,6 +10,7 @@ struct CUtensorMap_st;
 namespace ffn {
 
 /* basic_kernels.cu */
+bool gemm_int4_generic_wins(int M, int N, int K);
 int gemm_int4_generic(const void *a, const void *packed, const void *scales, void *out_bf16,
                       float *out_f32, int M, int N, int K, cudaStream_t stream);
 int silu_mul_packed(void *out, const void *packed, int tokens, int inter, cudaStream_t stream);

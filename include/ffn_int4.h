@@ -122,9 +122,9 @@ int ffn_int4_set_fused(int enabled);
  * 34816 (17408 for two rows) and the three operands are 16-byte aligned; three rows and more take the
  * streaming tensor-core kernel (tcgen05, 128 rows a block, 512 a launch), whose scratch comes from a
  * stream-ordered pool of the library's (at most 64 MiB kept between calls), so calls on different
- * streams and threads are independent; everything else, and a call of three rows and more whose stream
- * is being captured or whose scratch cannot be had, takes the shape-generic kernel, so that a captured
- * graph holds kernels only (no allocation nodes).  A non-finite activation makes the outputs
+ * streams and threads are independent; everything else - up to eight rows of a small matrix among it -
+ * and a call of three rows and more whose stream is being captured or whose scratch cannot be had,
+ * takes the shape-generic kernel, so that a captured graph holds kernels only (no allocation nodes).  A non-finite activation makes the outputs
  * it reaches non-finite in all of them. */
 int ffn_gemm_int4_bf16(const void *a, const void *packed, const void *scales, void *out, int M,
                        int N, int K, int group, void *stream);

@@ -42,6 +42,22 @@ def upload_layer(layer, device, tp=1, rank=0, with_norm=False, prepare=False):
     return mlp.prepare() if prepare else mlp
 
 
+KERNEL_KINDS = ("stream_tc_kernel", "ffn_imma_kernel", "ffn_kmajor_kernel", "ffn_fused_kernel", "gate_up_mma_kernel", "ffn_tc_kernel",
+                "gemm_int4_rows_kernel")
+
+
+def kernels(call):
+    """Which of the library's matrix kernels a second call of ``call`` launches, by the names that a profiler sees."""
+    from torch.profiler import ProfilerActivity, profile
+    call()
+    torch.cuda.synchronize()
+    with profile(activities=[ProfilerActivity.CUDA]) as prof:
+        call()
+        torch.cuda.synchronize()
+    names = [e.name for e in prof.events()]
+    return {kind for kind in KERNEL_KINDS if any(kind in name for name in names)}
+
+
 def bf16_ulp(values):
     """One BF16 unit in the last place at |values| (FP32 array)."""
     a = np.abs(values.astype(np.float32))

@@ -113,6 +113,18 @@ def test_a_block_is_split_among_the_square_root_of_its_units(m, n, k):
     assert p["ctas"] <= blocks * units                       # no CTA without a unit
 
 
+@pytest.mark.parametrize("m,n,k,generic", [(4, 4096, 3072, True), (4, 4104, 3072, False), (4, 8, 5120, True), (4, 8, 5248, False),
+                                           (4, 16384, 512, True), (4, 16392, 512, False),
+                                           (8, 2456, 2560, True), (8, 2464, 2560, False), (8, 8, 2688, False), (8, 8192, 128, True),
+                                           (8, 8200, 128, False), (3, 3272, 2560, True), (3, 3280, 2560, False), (3, 8, 2688, True),
+                                           (3, 8, 2816, False), (5, 2560, 1536, True), (5, 8, 1664, False), (6, 2560, 1280, True),
+                                           (6, 8, 1408, False), (7, 8, 128, False), (9, 8, 128, False), (3, 2147483640, 2560, False)])
+def test_few_rows_of_a_small_matrix_take_the_generic_kernel(m, n, k, generic):
+    buf = ctypes.create_string_buffer(1024)
+    assert L.load().ffn_int4_describe_gemm_plan(m, n, k, SMS, SMEM, buf, len(buf)) == 0
+    assert buf.value.decode().startswith("kernel=generic " if generic else "kernel=stream_tc ")
+
+
 def test_long_batches_run_in_blocks_of_64_and_small_devices_fall_back():
     assert plan(100, 5120, 17408)["passes"] == 2
     assert plan(4, 5120, 17408, smem=40 * 1024)["kernel"] == "generic"   # no room for the pair's pipeline

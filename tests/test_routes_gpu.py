@@ -2,24 +2,12 @@
 kernels that stand behind the intended one, too."""
 import pytest
 import torch
-from torch.profiler import ProfilerActivity, profile
 
+from gpu_util import kernels
 from haskell_infer_demo_b200 import lib as L
 from haskell_infer_demo_b200 import ops
 
 pytestmark = pytest.mark.gpu
-KINDS = ("stream_tc_kernel", "ffn_imma_kernel", "ffn_kmajor_kernel", "ffn_fused_kernel", "gate_up_mma_kernel", "ffn_tc_kernel",
-         "gemm_int4_rows_kernel")
-
-
-def kernels(call):
-    call()
-    torch.cuda.synchronize()
-    with profile(activities=[ProfilerActivity.CUDA]) as prof:
-        call()
-        torch.cuda.synchronize()
-    names = [e.name for e in prof.events()]
-    return {kind for kind in KINDS if any(kind in name for name in names)}
 
 
 def layer(cuda, hidden, inter):
@@ -50,8 +38,19 @@ def test_batched_ffn_on_one_rank(cuda, tokens):
     assert kernels(lambda: mlp.forward_mlp(x)) == {"stream_tc_kernel"}
 
 
-@pytest.mark.parametrize("rows,n,k", [(3, 12288, 5120), (8, 12288, 5120), (9, 264, 256), (128, 4104, 1280), (513, 520, 512)])
+@pytest.mark.parametrize("rows,n,k", [(3, 12288, 5120), (3, 8, 2816), (8, 12288, 5120), (8, 2464, 2560), (7, 8, 128), (9, 264, 256),
+                                      (128, 4104, 1280), (513, 520, 512)])
 def test_gemm(cuda, rows, n, k):
     packed, scales = ops.quantize_int4(torch.empty((n, k), device=cuda).normal_(0.0, 0.02))
     a = torch.randn((rows, k), device=cuda).to(torch.bfloat16)
     assert kernels(lambda: ops.gemm_int4_bf16(a, packed, scales)) == {"stream_tc_kernel"}
+
+
+@pytest.mark.parametrize("rows,n,k", [(3, 2048, 2560), (4, 4096, 2560), (5, 8, 128), (6, 264, 256), (8, 2456, 2560)])
+def test_gemm_of_a_few_rows_and_a_small_matrix(cuda, rows, n, k):
+    packed, scales = ops.quantize_int4(torch.empty((n, k), device=cuda).normal_(0.0, 0.02))
+    a = torch.randn((rows, k), device=cuda).to(torch.bfloat16)
+    assert kernels(lambda: ops.gemm_int4_bf16(a, packed, scales)) == {"gemm_int4_rows_kernel"}
+    want = a.double() @ ops.dequantize_int4(packed, scales)[0].double().T
+    # half a BF16 ulp, and sums in FP32 of a few hundred terms each: far below that ulp
+    assert (ops.gemm_int4_bf16(a, packed, scales).double() - want).norm() / want.norm() <= 2.0 ** -8
