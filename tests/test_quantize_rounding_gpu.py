@@ -1,5 +1,6 @@
 """The GPU quantizer's rounding where the quotient is a half or next to one, at scales from the smallest to the
-largest that the format holds, and both ways of delivering the bytes: byte for byte against the CPU oracle."""
+largest that the format holds, byte for byte against the CPU oracle; and the ways of delivering the bytes: through
+scratch in 16-byte or in 2-byte pieces, and by a second pass."""
 import numpy as np
 import pytest
 import torch

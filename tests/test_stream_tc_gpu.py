@@ -4,7 +4,7 @@ import numpy as np
 import pytest
 import torch
 
-from gpu_util import assert_ffn_close, dev_bf16, host_f32, upload_layer
+from gpu_util import assert_ffn_close, dev_bf16, host_f32, kernels, upload_layer
 from haskell_infer_demo_b200 import lib as L
 from haskell_infer_demo_b200 import ops
 from oracle import ffn_oracle as o
@@ -18,12 +18,19 @@ def test_gemm_against_fp64(cuda, rows, n, k):
     gen = torch.Generator(device="cuda").manual_seed(rows * 100003 + n)
     packed, scales = ops.quantize_int4(torch.randn((n, k), generator=gen, device=cuda) * 0.02)
     a = torch.randn((rows, k), generator=gen, device=cuda).to(torch.bfloat16)
+    # three rows of a small matrix are the shape-generic kernel's: as sharp a check of that one, then
+    small = rows == 3 and k <= 2730 and rows * n * 2 <= 65536 and rows * n * k * 2 <= 48 << 20
+    assert kernels(lambda: ops.gemm_int4_bf16(a, packed, scales)) == {"gemm_int4_rows_kernel" if small else "stream_tc_kernel"}
     got = ops.gemm_int4_bf16(a, packed, scales).double()
     w = ops.dequantize_int4(packed, scales)[0].double()
     want = a.double() @ w.T
-    # half a BF16 ulp of the result, and FP32 sums of k products: k * 2^-24 of the sum of magnitudes at most
-    bound = want.abs() * 2.0 ** -8 + (a.double().abs() @ w.abs().T) * (k * 2.0 ** -24)
-    assert (got - want).abs().le(bound).all()
+    # FP32 sums: 128 products of a group (the tensor core may truncate: 2^-23 each), the groups one after the other,
+    # the pieces of a block (at most the square root of its units); the generic kernel's are no deeper.  Then
+    # half a BF16 ulp: 2^-8 of a value at most; over many values its root mean square, ulp / sqrt(12), is 1.7e-3 of theirs.
+    groups = k // 128
+    off = (a.double().abs() @ w.abs().T) * ((128 + groups + groups ** 0.5 + 1) * 2.0 ** -23)
+    assert (got - want).abs().le((want.abs() + off) * 2.0 ** -8 + off).all()
+    assert want.numel() < 1000 or (got - want).norm() <= want.norm() * 2.0 ** -9
     assert torch.equal(ops.gemm_int4_bf16(a, packed, scales).double(), got)     # a fixed order of summation
     L.device_status()
 
@@ -36,7 +43,9 @@ def test_ffn_with_norm_against_oracle(cuda, tokens, hidden, inter):
     want, _, act = o.ffn(layer, o.gemma_rmsnorm(x, layer.w_norm), intermediates=True)
     mlp = upload_layer(layer, cuda, with_norm=True)
     ws = mlp.workspace(tokens)
-    got = mlp.forward_mlp(dev_bf16(x, cuda), ws=ws)
+    xd = dev_bf16(x, cuda)
+    assert kernels(lambda: mlp.forward_mlp(xd, ws=ws)) == {"stream_tc_kernel"}
+    got = mlp.forward_mlp(xd, ws=ws)
     L.device_status()
     assert_ffn_close(host_f32(got), want, f"{hidden}x{inter} M={tokens}")
     left = host_f32(ws[tokens * (hidden + 2 * inter):tokens * (hidden + 3 * inter)].view(tokens, inter))
