@@ -379,7 +379,6 @@ __global__ void __launch_bounds__(StPlan<NP>::kThreads, 1) stream_tc_kernel(cons
     } else {
         /* ---------------- epilogue ---------------- */
         constexpr int COLS = L::kCols;
-        constexpr bool kTight = PAIRS && NP > 64; /* no registers to spare: 72 a thread */
         const int quadrant = warp & 3, c0 = (warp >> 2) * COLS;
         const uint32_t d_lane = tmem + ((uint32_t)(quadrant * 32) << 16) + (uint32_t)c0;
         /* this lane's row of block b; rows past a ragged end read the last row's scales */
@@ -468,76 +467,45 @@ __global__ void __launch_bounds__(StPlan<NP>::kThreads, 1) stream_tc_kernel(cons
                     /* the end of a block, or of this CTA's piece of the line */
                     const int rb = block / P.token_blocks, tb = block % P.token_blocks;
                     bool finish = true;
-                    if constexpr (kTight) {
-                        /* As below without the shortcut.  Any change to this path has cost more in spills, in the loop
-                         * above, than the hand-over takes: 5120 x 17408, 128 tokens 98 us so, 101 to 104 with it. */
-                        const long long first = (long long)block * U, last = first + U;
-                        if (first < it0 || last > it1) {
-                            /* slot 0: the block began in an earlier CTA; 1: it begins here */
-                            const size_t per_slot = (size_t)NP * kTcRows, mine = (size_t)c0 * kTcRows + quadrant * 32 + lane;
-                            float *to = P.partial + ((size_t)blockIdx.x * 2 + (it0 > first ? 0 : 1)) * per_slot + mine;
+                    const bool begins_here = i + 1 >= unit;
+                    const bool ends_here = unit == U;
+                    if (!begins_here || !ends_here) {
+                        const long long line = (long long)P.blocks * U, first = (long long)block * U;
+                        /* slot 0: the block began in an earlier CTA; 1: it begins here */
+                        const size_t per_slot = (size_t)NP * kTcRows, mine = (size_t)c0 * kTcRows + quadrant * 32 + lane;
+                        /* CTA q holds unit u when q = floor(((u + 1) * CTAs - 1) / line) */
+                        const int q0 = (int)(((first + 1) * gridDim.x - 1) / line), q1 = (int)(((first + U) * gridDim.x - 1) / line);
+                        unsigned *arrive = P.arrivals + (size_t)q0 * kStMaxEpiWarps + warp;
+                        /* The others take their piece of a block first in their lines, the CTA in which it begins takes
+                         * its own last, at the end of the launch: it usually finds them all there, and then neither
+                         * hands over its sums nor waits for them (5120 x 17408, 8 tokens 45.7 -> 44.6 us, 128 tokens 105.4 ->
+                         * 101.9; LM head, 5 rows 156.4 -> 155.0). */
+                        bool all_there = false;
+                        if (begins_here) {
+                            unsigned seen = 0;
+                            if (lane == 0) seen = ld_acquire_gpu(arrive);
+                            all_there = __shfl_sync(~0u, seen, 0) == (unsigned)(q1 - q0);
+                        }
+                        if (!all_there) {
+                            float *to = P.partial + ((size_t)blockIdx.x * 2 + (begins_here ? 1 : 0)) * per_slot + mine;
 #pragma unroll
                             for (int c = 0; c < COLS; ++c) __stcg(to + c * kTcRows, acc[c]);
                             __threadfence();
                             __syncwarp();
-                            /* CTA q holds unit u when q = floor(((u + 1) * CTAs - 1) / total) */
-                            const int q0 = (int)(((first + 1) * gridDim.x - 1) / total), q1 = (int)((last * gridDim.x - 1) / total);
                             unsigned before = 0;
-                            if (lane == 0) before = atomicAdd(P.arrivals + (size_t)q0 * kStMaxEpiWarps + warp, 1u);
+                            if (lane == 0) before = atomicAdd(arrive, 1u);
                             finish = __shfl_sync(~0u, before, 0) == (unsigned)(q1 - q0);
-                            if (finish) {
-                                __syncwarp(); /* lane 0's count before the other lanes' loads: a shuffle orders no memory */
-                                __threadfence();
-#pragma unroll
-                                for (int c = 0; c < COLS; ++c) acc[c] = 0.0f;
-                                for (int q = q0; q <= q1; ++q) {
-                                    const float *from = P.partial + ((size_t)q * 2 + (total * q / gridDim.x > first ? 0 : 1)) * per_slot + mine;
-#pragma unroll
-                                    for (int c = 0; c < COLS; ++c) acc[c] += __ldcg(from + c * kTcRows);
-                                }
-                            }
                         }
-                    } else {
-                        const bool begins_here = i + 1 >= unit;
-                        const bool ends_here = unit == U;
-                        if (!begins_here || !ends_here) {
-                            const long long line = (long long)P.blocks * U, first = (long long)block * U;
-                            /* slot 0: the block began in an earlier CTA; 1: it begins here */
-                            const size_t per_slot = (size_t)NP * kTcRows, mine = (size_t)c0 * kTcRows + quadrant * 32 + lane;
-                            /* CTA q holds unit u when q = floor(((u + 1) * CTAs - 1) / line) */
-                            const int q0 = (int)(((first + 1) * gridDim.x - 1) / line), q1 = (int)(((first + U) * gridDim.x - 1) / line);
-                            unsigned *arrive = P.arrivals + (size_t)q0 * kStMaxEpiWarps + warp;
-                            /* The others take their piece of a block first in their lines, the CTA in which it begins takes
-                             * its own last, at the end of the launch: it usually finds them all there, and then neither
-                             * hands over its sums nor waits for them (5120 x 17408, 8 tokens 49.5 -> 46.7 us; LM head, 5 rows
-                             * 132 -> 128). */
-                            bool all_there = false;
-                            if (begins_here) {
-                                unsigned seen = 0;
-                                if (lane == 0) seen = ld_acquire_gpu(arrive);
-                                all_there = __shfl_sync(~0u, seen, 0) == (unsigned)(q1 - q0);
-                            }
-                            if (!all_there) {
-                                float *to = P.partial + ((size_t)blockIdx.x * 2 + (begins_here ? 1 : 0)) * per_slot + mine;
+                        if (finish) {
+                            /* in CTA order, from zero; sums still in registers are the first CTA's */
+                            __syncwarp(); /* lane 0's count before the other lanes' loads: a shuffle orders no memory */
+                            __threadfence();
 #pragma unroll
-                                for (int c = 0; c < COLS; ++c) __stcg(to + c * kTcRows, acc[c]);
-                                __threadfence();
-                                __syncwarp();
-                                unsigned before = 0;
-                                if (lane == 0) before = atomicAdd(arrive, 1u);
-                                finish = __shfl_sync(~0u, before, 0) == (unsigned)(q1 - q0);
-                            }
-                            if (finish) {
-                                /* in CTA order, from zero; sums still in registers are the first CTA's */
-                                __syncwarp(); /* as above */
-                                __threadfence();
+                            for (int c = 0; c < COLS; ++c) acc[c] = all_there ? 0.0f + acc[c] : 0.0f;
+                            for (int q = all_there ? q0 + 1 : q0; q <= q1; ++q) {
+                                const float *from = P.partial + ((size_t)q * 2 + (q == q0 ? 1 : 0)) * per_slot + mine; /* it begins in q0 */
 #pragma unroll
-                                for (int c = 0; c < COLS; ++c) acc[c] = all_there ? 0.0f + acc[c] : 0.0f;
-                                for (int q = all_there ? q0 + 1 : q0; q <= q1; ++q) {
-                                    const float *from = P.partial + ((size_t)q * 2 + (q == q0 ? 1 : 0)) * per_slot + mine; /* it begins in q0 */
-#pragma unroll
-                                    for (int c = 0; c < COLS; ++c) acc[c] += __ldcg(from + c * kTcRows);
-                                }
+                                for (int c = 0; c < COLS; ++c) acc[c] += __ldcg(from + c * kTcRows);
                             }
                         }
                     }
@@ -755,7 +723,11 @@ static int st_reserve(StScratch &sc, size_t bytes, cudaStream_t stream) {
 
 int stream_tc_ffn_launch(cudaStream_t stream, const void *x, void *act, void *layer_out, const FfnMlpWeights *w, int tokens, int H,
                          int I, void *residual, const FusedNorm *norm, void *normed, unsigned *status) {
-    if (tokens <= 2 || tc_get_mode() != 2) return FFN_NOT_ADMITTED; /* 3..16 tokens: the mma.sync pair, 63 against 81 us at 8 on the 5120 x 17408 layer */
+    /* One and two tokens are the single-launch kernel's.  At two, without a norm, us on the device, that kernel / this:
+     * 1024 x 3072 11.0 / 13.1, 2560 x 9728 20.7 / 22.6, 5120 x 4352 17.7 / 21.7, 5120 x 8704 27.3 / 27.6, 4096 x 14336
+     * 33.1 / 32.9, 5120 x 17408 46.7 / 43.5; with the norm as a launch of its own before it 13.0 / 13.2, 22.7 / 22.5,
+     * 19.6 / 22.1, 29.3 / 28.0, 35.2 / 32.9, 48.4 / 44.5. */
+    if (tokens <= 2 || tc_get_mode() != 2) return FFN_NOT_ADMITTED;
     if (((uintptr_t)w->gate_up_i4 & 15) || ((uintptr_t)w->down_i4 & 15) || ((uintptr_t)x & 15) || ((uintptr_t)normed & 15)) return FFN_NOT_ADMITTED;
     int dev = 0, sm_count = 0, st = st_device(&dev, &sm_count);
     if (st) return st;
