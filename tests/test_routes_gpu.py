@@ -3,11 +3,18 @@ kernels that stand behind the intended one, too."""
 import pytest
 import torch
 
-from gpu_util import kernels
+import gpu_util
 from haskell_infer_demo_b200 import lib as L
 from haskell_infer_demo_b200 import ops
 
 pytestmark = pytest.mark.gpu
+
+
+def kernels(call):
+    seen = gpu_util.kernels(call)
+    if seen is None:
+        pytest.skip("the profiler reports no kernels here")
+    return seen
 
 
 def layer(cuda, hidden, inter):
