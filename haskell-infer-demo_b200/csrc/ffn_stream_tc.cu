@@ -49,7 +49,7 @@ namespace ffn {
 constexpr int kStMaxTokens = 128;            /* tokens of a block = MMA columns */
 constexpr int kStSlab = 512;                 /* tokens of a launch */
 constexpr int kStMaxEpiWarps = 16;
-constexpr int kStMaxRing = 8, kStMaxA = 4, kStMaxD = 2; /* a ring of ten units of weights is no faster (5120 x 17408, 8 tokens: 50.3 us, 49.5 with eight) */
+constexpr int kStMaxRing = 8, kStMaxA = 4, kStMaxD = 2; /* a ring of ten units of weights is slower (5120 x 17408, 8 tokens: 45.6 us, 44.7 with eight) */
 constexpr int kStUnitBytes = kTcRows * 128;  /* packed bytes of a unit */
 constexpr int kStHeader = 1024;
 constexpr int kStSmem = 232448;
@@ -156,7 +156,8 @@ __device__ __forceinline__ void st_give_up(StSmem *sm, unsigned *status, int whe
     atomicCAS(status, 0u, (unsigned)where | ((unsigned)blockIdx.x << 8));
 }
 /* Bounded wait.  try_wait suspends the thread in hardware, so there is no sleep between polls: a role's
- * turn is a chain of such waits, and a sleeping thread would answer late. */
+ * turn is a chain of such waits, and a sleeping thread would answer late.  The limit is a number of polls, each 0.07
+ * (32 warps polling) to 1.4 us (one): a wait gives up after 0.3 to 6 seconds. */
 __device__ __forceinline__ bool st_wait(uint64_t *bar, uint32_t parity, volatile int *abort_flag) {
     for (uint32_t i = 0; i < kSpinLimit; ++i) {
         if (mbar_try_wait(bar, parity)) return true;
@@ -626,8 +627,9 @@ static int st_launch_kernel(const StreamTcParams &P, int ctas, cudaStream_t stre
 }
 /* A warp's 32 rows are 32 sectors to a load of scales, and shared memory leaves no L1 to keep them in.  Above
  * 64 tokens, where 16 epilogue warps load them, pieces of two units (rows of whole pieces, K a multiple of 512,
- * on 8 bytes) are worth it: 5120 x 17408, 128 tokens 103.5 -> 99 us.  Below they are not: the LM head, 5 rows
- * 132 -> 136. */
+ * on 8 bytes) are worth it: 5120 x 17408, 128 tokens 104.0 -> 101.9 us; 2560 x 9728, 500 tokens 110.9 -> 108.2; the
+ * 12288 x 5120 matrix, 100 rows 25.8 either way.  Up to 64 they give a hundredth (LM head, 5 rows 155.2 -> 153.3;
+ * 5120 x 17408, 8 tokens 44.6 -> 44.3, 27 tokens 52.8 -> 52.3), and eight more kernels are not built for it. */
 template <int NP, bool PAIRS>
 static int st_launch(const StreamTcParams &P, int ctas, cudaStream_t stream) {
     if (NP > 64 && P.K % (4 * FFN_INT4_GROUP) == 0 && !((uintptr_t)P.s & 7)) return st_launch_kernel<NP, PAIRS, (NP > 64)>(P, ctas, stream);

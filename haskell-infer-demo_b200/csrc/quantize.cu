@@ -14,7 +14,7 @@
  * HBM bound: the FP32 input is read once.  The checking pass quantizes into scratch as it goes, and a second
  * launch moves the bytes to the caller once nothing was refused - it looks at the verdict itself, so the host
  * waits once, at the end.  5120 x 17408: 221 us with a checking and a writing pass over the input, a wait
- * between them and cudaMalloc / cudaFree around them; 118 now.  Where the bytes exceed the scratch that
+ * between them and cudaMalloc / cudaFree around them; 111 now.  Where the bytes exceed the scratch that
  * the library keeps (kScratchMost), or there is no memory for them, the second launch quantizes again instead.
  *
  * Eight lanes per group: a lane holds sixteen elements in four 16-byte loads (128 contiguous bytes of a group

@@ -272,7 +272,7 @@ int ffn_int4_describe_kmajor_plan(int tokens, int hidden, int intermediate, int 
 int ffn_int4_set_decode_kernel(int which);
 
 /* Which kernels serve three tokens and more.  2 (default): on one rank the streaming tcgen05 kernel
- * (csrc/ffn_stream_tc.cu: 45 us at 8 tokens, 53 at 27, 98 at 128 on the 5120 x 17408 layer); under tensor
+ * (csrc/ffn_stream_tc.cu: 45 us at 8 tokens, 52 at 27, 102 at 128, norm included, on the 5120 x 17408 layer); under tensor
  * parallelism, whose exchange only the pairs have, one of the two pairs below by the rule given there.  0 and 1
  * force a pair, in passes of up to 64 tokens, on one rank too: 1 the mma.sync pair; 0 the tcgen05 pair
  * (tcgen05.mma with FP32 accumulators and the converted BF16 operand in tensor memory, packed INT4 rows
