@@ -214,7 +214,7 @@ int ffn_int4_describe_gemm_plan(int m, int n, int k, int sm_count, int smem_opti
     if (m <= 2 && gemv_describe_plan(m, n, k, sm_count, smem_optin, out, out_bytes)) return FFN_OK;
     char stream[200];
     if (!gemm_int4_generic_wins(m, n, k) && stream_tc_describe(m, n, k, sm_count, smem_optin, stream, sizeof(stream))) snprintf(out, out_bytes, "kernel=%s", stream);
-    else snprintf(out, out_bytes, "kernel=generic launches=1");
+    else snprintf(out, out_bytes, "kernel=generic launches=%d", m / 8 + (m >> 2 & 1) + (m >> 1 & 1) + (m & 1)); /* 8, 4, 2, 1 rows */
     return FFN_OK;
 }
 

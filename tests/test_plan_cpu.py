@@ -123,6 +123,8 @@ def test_few_rows_of_a_small_matrix_take_the_generic_kernel(m, n, k, generic):
     buf = ctypes.create_string_buffer(1024)
     assert L.load().ffn_int4_describe_gemm_plan(m, n, k, SMS, SMEM, buf, len(buf)) == 0
     assert buf.value.decode().startswith("kernel=generic " if generic else "kernel=stream_tc ")
+    if generic:
+        assert buf.value.decode().endswith(f" launches={m // 8 + bin(m % 8).count('1')}")
 
 
 def test_long_batches_run_in_blocks_of_64_and_small_devices_fall_back():
