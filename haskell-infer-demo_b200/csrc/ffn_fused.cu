@@ -84,6 +84,19 @@ struct FusedParams {
 #define FFN_DEBUG_BIT(P, b) 0
 #endif
 
+/* A stack of layers in one launch (ffn_stack_kernel): the launch's parameters (weights excepted) and each layer's operands. */
+constexpr int kStackMaxLayers = 64;
+struct StackLayer {
+    const uint8_t *gate_up, *down;
+    const uint16_t *gate_up_s, *down_s, *norm_w;
+};
+struct StackParams {
+    FusedParams f;
+    int layers;
+    StackLayer layer[kStackMaxLayers];
+};
+static_assert(sizeof(StackParams) <= 4096, "kernel parameters");
+
 struct Smem;
 __host__ __device__ constexpr size_t fused_smem_header(int tokens); /* bytes before the activation copy */
 struct Smem {
@@ -91,7 +104,7 @@ struct Smem {
     uint64_t empty[kMaxStages];
     uint64_t part_full[kPartSlots];
     uint64_t part_empty[kPartSlots];
-    uint64_t x_full[2];
+    uint64_t norm_full, x_full; /* a stack: every warp's part of the sum of squares is there; the hand-over's copy is */
     int abort_flag;
     int pad[11];
     float norm_red[2][kConsumerWarps + 3];
@@ -121,9 +134,11 @@ __device__ __forceinline__ void stamp(const FusedParams &P, int slot) {
 }
 
 /* ---- consumer side of one phase ------------------------------------------------------------ */
-template <int CIT, int MT, bool PAIRS>
+/* `hand` numbers the hand-over between CTAs that brings the phase's input (act of the launch's first layer 0,
+ * then the residual stream and act in turn), -1: it is there when the kernel starts. */
+template <int CIT, int MT, bool PAIRS, bool STACK>
 __device__ __forceinline__ void consume_phase(const FusedParams &P, const PhasePlan &pl, Smem *sm,
-                                              const uint16_t *xs, uint8_t *ring, int tile0) {
+                                              const uint16_t *xs, uint8_t *ring, int tile0, int hand, const uint16_t *norm_w) {
     constexpr int NVROW = (PAIRS ? 2 : 1) * MT;
     constexpr int VALS = 4 * MT;   /* values a thread carries through a tile: one transposed reduction per four */
     constexpr int JTM = VALS / NVROW; /* row steps per thread per tile: 2 of pairs, 4 of single rows */
@@ -142,9 +157,16 @@ __device__ __forceinline__ void consume_phase(const FusedParams &P, const PhaseP
      * global memory: it is there when the kernel starts, so the loads are in flight while the
      * producer is still setting up.  Phase 2 waits for the copy of act the producer brings into
      * shared memory once the grid barrier has opened. */
-    const bool direct = PAIRS || P.gemv; /* single-matrix mode: the activation is an input too */
-    if (!direct && !mbar_wait<64>(&sm->x_full[1], 0u, &sm->abort_flag)) {
-        give_up(sm, P.sync, ST_X_FULL);
+    const bool direct = STACK ? hand < 0 : PAIRS || P.gemv; /* single-matrix mode: the activation is an input too */
+    uint4 nw[STACK && PAIRS ? CIT : 1][4]; /* a stack's norm weights are fetched while the layer before is finished elsewhere */
+    if (STACK && PAIRS) {
+#pragma unroll
+        for (int c = 0; c < CIT; ++c)
+#pragma unroll
+            for (int q = 0; q < 4; ++q) nw[c][q] = __ldg((const uint4 *)(norm_w + (size_t)min(ct + c * pl.CT, pl.cpr - 1) * 32 + q * 8));
+    }
+    if (!direct && !mbar_wait<64>(&sm->x_full, (uint32_t)hand & 1u, &sm->abort_flag)) {
+        give_up(sm, P.sync, STACK && PAIRS ? ST_NEXT_X : ST_X_FULL);
         return;
     }
     const uint16_t *src = direct ? P.x : xs;
@@ -161,7 +183,7 @@ __device__ __forceinline__ void consume_phase(const FusedParams &P, const PhaseP
     float inv_rms[MT];
 #pragma unroll
     for (int m = 0; m < MT; ++m) inv_rms[m] = 1.0f;
-    const bool normalize = PAIRS && P.norm_w != nullptr;
+    const bool normalize = PAIRS && (STACK || norm_w != nullptr);
     if (normalize) { /* every CTA needs the whole normalized vector, so every CTA takes the (cheap) norm */
 #pragma unroll
         for (int m = 0; m < MT; ++m) {
@@ -179,7 +201,15 @@ __device__ __forceinline__ void consume_phase(const FusedParams &P, const PhaseP
             ss = warp_sum(ss);
             if (lane == 0) sm->norm_red[m][ti >> 5] = ss;
         }
-        asm volatile("bar.sync 1, %0;" ::"n"(kConsumerThreads) : "memory");
+        if (STACK) { /* a wait with a limit: a warp that gave up in an earlier phase does not come */
+            if (lane == 0) mbar_arrive(&sm->norm_full);
+            if (!mbar_wait<20>(&sm->norm_full, (uint32_t)((hand + 1) >> 1) & 1u, &sm->abort_flag)) {
+                give_up(sm, P.sync, ST_NEXT_X);
+                return;
+            }
+        } else {
+            asm volatile("bar.sync 1, %0;" ::"n"(kConsumerThreads) : "memory");
+        }
 #pragma unroll
         for (int m = 0; m < MT; ++m) {
             float total = 0.0f;
@@ -195,9 +225,13 @@ __device__ __forceinline__ void consume_phase(const FusedParams &P, const PhaseP
         for (int m = 0; m < MT; ++m) {
             const int col = ct + c * pl.CT;
             const bool on = active && col < pl.cpr;
-            prepare_chunk(xc[c][m], xv[c][m], on,
-                          normalize ? P.norm_w + (size_t)min(col, pl.cpr - 1) * 32 : nullptr, inv_rms[m],
-                          P.norm_gemma ? 1.0f : 0.0f);
+            const float gemma = P.norm_gemma ? 1.0f : 0.0f;
+            if (STACK && PAIRS) {
+                if (on) norm_chunk(xv[c][m], nw[STACK && PAIRS ? c : 0], inv_rms[m], gemma);
+                prepare_chunk(xc[c][m], xv[c][m], on);
+            } else {
+                prepare_chunk(xc[c][m], xv[c][m], on, normalize ? norm_w + (size_t)min(col, pl.cpr - 1) * 32 : nullptr, inv_rms[m], gemma);
+            }
         }
     if (threadIdx.x == 32) stamp(P, PAIRS ? 2 : 7);
 
@@ -295,8 +329,9 @@ __device__ __forceinline__ void consume_phase(const FusedParams &P, const PhaseP
 }
 
 /* ---- epilogue side of one phase ------------------------------------------------------------ */
-template <int MT, bool PAIRS>
-__device__ __forceinline__ bool epilogue_phase(const FusedParams &P, const PhasePlan &pl, Smem *sm, int tile0, unsigned seq) {
+/* STACK: one rank; the output is stored for the last layer only, the residual stream is there and read early */
+template <int MT, bool PAIRS, bool STACK>
+__device__ __forceinline__ bool epilogue_phase(const FusedParams &P, const PhasePlan &pl, Smem *sm, int tile0, unsigned seq, bool store_out) {
     constexpr int NVROW = (PAIRS ? 2 : 1) * MT;
     const int lane = threadIdx.x & 31;
     const int row_begin = cta_begin(pl.rows_total, blockIdx.x, gridDim.x);
@@ -306,6 +341,9 @@ __device__ __forceinline__ bool epilogue_phase(const FusedParams &P, const Phase
         const int tile = tile0 + lt;
         const int pslot = tile % kPartSlots;
         const int rows = min(pl.TR, row_end - (row_begin + lt * pl.TR));
+        float res = 0.0f;
+        if (STACK && !PAIRS && lane < rows * MT) /* this thread's own store of the layer before */
+            res = bf16_bits_to_f32(P.residual[(size_t)(lane % MT) * P.H + row_begin + lt * pl.TR + lane / MT]);
         if (!mbar_wait<100>(&sm->part_full[pslot], (uint32_t)(tile / kPartSlots) & 1u, &sm->abort_flag)) {
             give_up(sm, P.sync, ST_PART_FULL);
             return false;
@@ -324,6 +362,12 @@ __device__ __forceinline__ bool epilogue_phase(const FusedParams &P, const Phase
                 for (int h = 0; h < pl.nhw; ++h) b += pb[h];
                 const float g = round_bf16(a), u = round_bf16(b);
                 P.act[(size_t)m * P.I + row] = f32_to_bf16_bits(silu_mul(g, u));
+            } else if (STACK) {
+                const size_t o = (size_t)m * P.H + row;
+                const float y = round_bf16(a);
+                if (i != lane) res = bf16_bits_to_f32(P.residual[o]);
+                P.residual[o] = f32_to_bf16_bits(res + y);
+                if (store_out) P.out[o] = f32_to_bf16_bits(y);
             } else if (P.tp == 1) {
                 const float y = round_bf16(a);
                 P.out[(size_t)m * P.H + row] = f32_to_bf16_bits(y);
@@ -341,6 +385,58 @@ __device__ __forceinline__ bool epilogue_phase(const FusedParams &P, const Phase
     return true;
 }
 
+/* ---- producer: the copies of one tile ---------------------------------------------------------- */
+/* gate/up pairs from r0 on.  Scale runs are widened to 16-byte boundaries (the array's end is one: row counts
+ * are multiples of 8, so N*G*2 is a multiple of 16). */
+__device__ __forceinline__ void copy_pairs(const FusedParams &P, const uint8_t *w, const uint16_t *s, int r0, int end, uint8_t *dst, uint64_t *full) {
+    const int rows = min(P.p1.TR, end - r0);
+    const uint32_t bytes = (uint32_t)rows * P.p1.rb;
+    const size_t g0 = (size_t)r0 * P.p1.G * 2, g1 = (size_t)(r0 + P.p1.up_offset) * P.p1.G * 2;
+    const size_t len = (size_t)rows * P.p1.G * 2;
+    const size_t a0 = g0 & ~(size_t)15, a1 = g1 & ~(size_t)15;
+    const uint32_t n0 = (uint32_t)(((g0 + len + 15) & ~(size_t)15) - a0);
+    const uint32_t n1 = (uint32_t)(((g1 + len + 15) & ~(size_t)15) - a1);
+    mbar_expect_tx(full, 2 * bytes + n0 + n1);
+    bulk_g2s(dst, w + (size_t)r0 * P.p1.rb, bytes, full);
+    bulk_g2s(dst + bytes, w + (size_t)(r0 + P.p1.up_offset) * P.p1.rb, bytes, full);
+    bulk_g2s(dst + P.stage_w_bytes, (const uint8_t *)s + a0, n0, full);
+    bulk_g2s(dst + P.stage_w_bytes + P.sc_half_bytes, (const uint8_t *)s + a1, n1, full);
+}
+/* rows of the down projection */
+__device__ __forceinline__ void copy_rows(const FusedParams &P, const uint8_t *w, const uint16_t *s, int r0, int end, uint8_t *dst, uint64_t *full) {
+    const int rows = min(P.p2.TR, end - r0);
+    const uint32_t bytes = (uint32_t)rows * P.p2.rb;
+    const size_t g0 = (size_t)r0 * P.p2.G * 2, len = (size_t)rows * P.p2.G * 2;
+    const size_t a0 = g0 & ~(size_t)15;
+    const uint32_t n0 = (uint32_t)(((g0 + len + 15) & ~(size_t)15) - a0);
+    mbar_expect_tx(full, bytes + n0);
+    bulk_g2s(dst, w + (size_t)r0 * P.p2.rb, bytes, full);
+    bulk_g2s(dst + P.stage_w_bytes, (const uint8_t *)s + a0, n0, full);
+}
+__device__ __forceinline__ void init_barriers(Smem *sm, int lane, int ns) {
+    if (lane < ns) { mbar_init(&sm->full[lane], 1); mbar_init(&sm->empty[lane], kConsumerWarps); }
+    if (lane >= 8 && lane < 8 + kPartSlots) { mbar_init(&sm->part_full[lane - 8], kConsumerWarps); mbar_init(&sm->part_empty[lane - 8], 1); }
+    if (lane == 16) mbar_init(&sm->norm_full, kConsumerWarps);
+    if (lane == 17) mbar_init(&sm->x_full, 1);
+    if (lane == 31) sm->abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+}
+/* bounded wait until the arrivals at the grid barrier have reached `target` */
+__device__ __forceinline__ bool grid_barrier_open(const unsigned *arrivals, unsigned target, volatile int *abort_flag) {
+    for (uint32_t i = 0; i < kSpinLimit; ++i) {
+        if ((int)(ld_acquire_gpu(arrivals) - target) >= 0) return true;
+        if ((i & 63) == 63 && *abort_flag) return false;
+        __nanosleep(32);
+    }
+    return false;
+}
+/* never leave with a copy of ours in flight: bounded wait for the barrier's phase */
+__device__ __forceinline__ void drain(uint64_t *bar, uint32_t parity, unsigned *sync) {
+    bool done = false;
+    for (uint32_t i = 0; i < kSpinLimit && !done; ++i) done = mbar_try_wait(bar, parity);
+    if (!done) atomicCAS(sync + 3, 0u, (unsigned)ST_DRAIN | ((unsigned)blockIdx.x << 8));
+}
+
 /* ---- the kernel ----------------------------------------------------------------------------- */
 template <int CIT1, int CIT2, int MT>
 __global__ void __launch_bounds__(kThreads, 1) ffn_fused_kernel(const FusedParams P) {
@@ -354,11 +450,7 @@ __global__ void __launch_bounds__(kThreads, 1) ffn_fused_kernel(const FusedParam
     if (threadIdx.x == 0) griddep_launch(); /* the next launch may take this CTA's SM the moment it is free */
     if (warp == 0) {
         if (lane == 0) stamp(P, 0);
-        if (lane < ns) { mbar_init(&sm->full[lane], 1); mbar_init(&sm->empty[lane], kConsumerWarps); }
-        if (lane >= 8 && lane < 8 + kPartSlots) { mbar_init(&sm->part_full[lane - 8], kConsumerWarps); mbar_init(&sm->part_empty[lane - 8], 1); }
-        if (lane >= 16 && lane < 18) mbar_init(&sm->x_full[lane - 16], 1);
-        if (lane == 31) sm->abort_flag = 0;
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        init_barriers(sm, lane, ns);
     }
     __syncthreads();
 
@@ -374,33 +466,9 @@ __global__ void __launch_bounds__(kThreads, 1) ffn_fused_kernel(const FusedParam
             int t = 0;
             auto issue_tile = [&](int t) {
                 const int s = t % ns;
-                uint8_t *dst = ring + (size_t)s * P.stage_bytes;
                 if (FFN_DEBUG_BIT(P, 2)) { mbar_arrive(&sm->full[s]); return; }
-                if (t < nt1) {
-                    const int r0 = b1 + t * P.p1.TR, rows = min(P.p1.TR, e1 - r0);
-                    const uint32_t bytes = (uint32_t)rows * P.p1.rb;
-                    /* scale runs widened to 16-byte boundaries (the array's end is one: row counts
-                     * are multiples of 8, so N*G*2 is a multiple of 16) */
-                    const size_t g0 = (size_t)r0 * P.p1.G * 2, g1 = (size_t)(r0 + P.p1.up_offset) * P.p1.G * 2;
-                    const size_t len = (size_t)rows * P.p1.G * 2;
-                    const size_t a0 = g0 & ~(size_t)15, a1 = g1 & ~(size_t)15;
-                    const uint32_t n0 = (uint32_t)(((g0 + len + 15) & ~(size_t)15) - a0);
-                    const uint32_t n1 = (uint32_t)(((g1 + len + 15) & ~(size_t)15) - a1);
-                    mbar_expect_tx(&sm->full[s], 2 * bytes + n0 + n1);
-                    bulk_g2s(dst, P.p1.w + (size_t)r0 * P.p1.rb, bytes, &sm->full[s]);
-                    bulk_g2s(dst + bytes, P.p1.w + (size_t)(r0 + P.p1.up_offset) * P.p1.rb, bytes, &sm->full[s]);
-                    bulk_g2s(dst + P.stage_w_bytes, (const uint8_t *)P.p1.s + a0, n0, &sm->full[s]);
-                    bulk_g2s(dst + P.stage_w_bytes + P.sc_half_bytes, (const uint8_t *)P.p1.s + a1, n1, &sm->full[s]);
-                } else {
-                    const int r0 = b2 + (t - nt1) * P.p2.TR, rows = min(P.p2.TR, e2 - r0);
-                    const uint32_t bytes = (uint32_t)rows * P.p2.rb;
-                    const size_t g0 = (size_t)r0 * P.p2.G * 2, len = (size_t)rows * P.p2.G * 2;
-                    const size_t a0 = g0 & ~(size_t)15;
-                    const uint32_t n0 = (uint32_t)(((g0 + len + 15) & ~(size_t)15) - a0);
-                    mbar_expect_tx(&sm->full[s], bytes + n0);
-                    bulk_g2s(dst, P.p2.w + (size_t)r0 * P.p2.rb, bytes, &sm->full[s]);
-                    bulk_g2s(dst + P.stage_w_bytes, (const uint8_t *)P.p2.s + a0, n0, &sm->full[s]);
-                }
+                if (t < nt1) copy_pairs(P, P.p1.w, P.p1.s, b1 + t * P.p1.TR, e1, ring + (size_t)s * P.stage_bytes, &sm->full[s]);
+                else copy_rows(P, P.p2.w, P.p2.s, b2 + (t - nt1) * P.p2.TR, e2, ring + (size_t)s * P.stage_bytes, &sm->full[s]);
             };
             /* The weights never change, so the first fill of every stage need not wait for the launch
              * before this one in the stream: with programmatic dependent launch this CTA starts as soon
@@ -417,18 +485,10 @@ __global__ void __launch_bounds__(kThreads, 1) ffn_fused_kernel(const FusedParam
             /* Phase 2's activation vector is fetched once the grid barrier has opened (every CTA has
              * stored its rows of act). */
             auto fetch_act = [&]() {
-                bool open = false;
-                for (uint32_t i = 0; i < kSpinLimit && !open; ++i) {
-                    open = (int)(ld_acquire_gpu(P.sync + 0) - bar_target) >= 0;
-                    if (!open) {
-                        if ((i & 63) == 63 && sm->abort_flag) break;
-                        __nanosleep(32);
-                    }
-                }
-                if (!open) { give_up(sm, P.sync, ST_GRID_BARRIER); failed = true; return; }
+                if (!grid_barrier_open(P.sync + 0, bar_target, &sm->abort_flag)) { give_up(sm, P.sync, ST_GRID_BARRIER); failed = true; return; }
                 stamp(P, 6);
-                mbar_expect_tx(&sm->x_full[1], (uint32_t)(P.M * P.I * 2));
-                bulk_g2s(xs, P.act, (uint32_t)(P.M * P.I * 2), &sm->x_full[1]);
+                mbar_expect_tx(&sm->x_full, (uint32_t)(P.M * P.I * 2));
+                bulk_g2s(xs, P.act, (uint32_t)(P.M * P.I * 2), &sm->x_full);
                 act_issued = true;
             };
             for (; t < total && !failed; ++t) {
@@ -447,22 +507,14 @@ __global__ void __launch_bounds__(kThreads, 1) ffn_fused_kernel(const FusedParam
             if (!act_issued && !failed && !P.gemv) fetch_act();
             /* Never leave with a copy of ours still in flight: wait (bounded) for the most recent
              * fill of every stage and for the activation copies. */
-            for (int u = max(0, t - ns); u < t; ++u) {
-                bool done = false;
-                for (uint32_t i = 0; i < kSpinLimit && !done; ++i) done = mbar_try_wait(&sm->full[u % ns], (uint32_t)(u / ns) & 1u);
-                if (!done) atomicCAS(P.sync + 3, 0u, (unsigned)ST_DRAIN | ((unsigned)blockIdx.x << 8));
-            }
-            if (act_issued) {
-                bool done = false;
-                for (uint32_t i = 0; i < kSpinLimit && !done; ++i) done = mbar_try_wait(&sm->x_full[1], 0u);
-                if (!done) atomicCAS(P.sync + 3, 0u, (unsigned)ST_DRAIN | ((unsigned)blockIdx.x << 8));
-            }
+            for (int u = max(0, t - ns); u < t; ++u) drain(&sm->full[u % ns], (uint32_t)(u / ns) & 1u, P.sync);
+            if (act_issued) drain(&sm->x_full, 0u, P.sync);
         }
     } else if (warp <= kConsumerWarps) {
         /* ---------------- consumers ---------------- */
         griddep_wait(); /* the input may be the previous kernel's output */
-        if (!P.gemv) consume_phase<CIT1, MT, true>(P, P.p1, sm, xs, ring, 0);
-        if (!sm->abort_flag) consume_phase<CIT2, MT, false>(P, P.p2, sm, xs, ring, nt1);
+        if (!P.gemv) consume_phase<CIT1, MT, true, false>(P, P.p1, sm, xs, ring, 0, -1, P.norm_w);
+        if (!sm->abort_flag) consume_phase<CIT2, MT, false, false>(P, P.p2, sm, xs, ring, nt1, 0, nullptr);
     } else {
         /* ---------------- epilogue ---------------- */
         griddep_wait(); /* act, out, the residual and the exchange slots may still be in use by the previous launch */
@@ -470,7 +522,7 @@ __global__ void __launch_bounds__(kThreads, 1) ffn_fused_kernel(const FusedParam
         const unsigned seq = P.tp > 1 ? ld_acquire_gpu(P.tp_seq) : 0u;
         bool ok = true;
         if (!P.gemv) {
-            ok = epilogue_phase<MT, true>(P, P.p1, sm, 0, seq);
+            ok = epilogue_phase<MT, true, false>(P, P.p1, sm, 0, seq, true);
             /* arrive at the grid barrier: the act rows of this CTA are stored */
             /* The lanes' act stores are ordered before lane 0's release by the warp barrier (release is
              * cumulative over it), so no lane needs a fence of its own. */
@@ -480,7 +532,7 @@ __global__ void __launch_bounds__(kThreads, 1) ffn_fused_kernel(const FusedParam
                 stamp(P, 5);
             }
         }
-        if (ok) ok = epilogue_phase<MT, false>(P, P.p2, sm, nt1, seq);
+        if (ok) ok = epilogue_phase<MT, false, false>(P, P.p2, sm, nt1, seq, true);
         if (lane == 0) stamp(P, 10);
         if (P.tp > 1) {
             /* every rank's partial sums of this CTA's rows arrive in this rank's own buffer as
@@ -512,6 +564,118 @@ __global__ void __launch_bounds__(kThreads, 1) ffn_fused_kernel(const FusedParam
     }
 }
 
+/* ---- a stack of layers: h <- bf16(h + FFN_l(RMSNorm_l(h))) for every layer in one launch ------- */
+/* HBM bound as the single layer, but its weights stream on through the hand-overs, and what a layer takes is the chain
+ * of one: residual stream in (grid barrier, copy, norm and conversion), gate/up, act (the same), down.  Every CTA has rows
+ * in both phases (the host sees to it), so an arrival at the barrier says that all the CTA's warps have read the input
+ * before, and one copy in shared memory and the barriers' one-bit phases do.  The ring is cut into stages that hold the most
+ * (plan_stack).  36 layers of 2560 x 9728, one token: 741 us as 36 launches, 633 so. */
+template <int CIT1, int CIT2, int MT>
+__global__ void __launch_bounds__(kThreads, 1) ffn_stack_kernel(const __grid_constant__ StackParams S) {
+    const FusedParams &P = S.f;
+    extern __shared__ __align__(128) uint8_t smem_raw[];
+    Smem *sm = (Smem *)smem_raw;
+    uint16_t *xs = (uint16_t *)(smem_raw + fused_smem_header(MT));
+    uint8_t *ring = (uint8_t *)xs + P.xs_bytes;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int ns = P.nstages, hands = 2 * S.layers - 1;
+
+    if (threadIdx.x == 0) griddep_launch();
+    if (warp == 0) {
+        if (lane == 0) stamp(P, 0);
+        init_barriers(sm, lane, ns);
+    }
+    __syncthreads();
+
+    const int b1 = cta_begin(P.p1.rows_total, blockIdx.x, gridDim.x), e1 = cta_begin(P.p1.rows_total, blockIdx.x + 1, gridDim.x);
+    const int b2 = cta_begin(P.p2.rows_total, blockIdx.x, gridDim.x), e2 = cta_begin(P.p2.rows_total, blockIdx.x + 1, gridDim.x);
+    const int nt1 = (e1 - b1 + P.p1.TR - 1) / P.p1.TR, nt2 = (e2 - b2 + P.p2.TR - 1) / P.p2.TR, nt = nt1 + nt2;
+
+    if (warp == 0) {
+        /* ---------------- producer ---------------- */
+        if (lane == 0) {
+            const int total = S.layers * nt;
+            int t = 0, l = 0, i = 0; /* tile t is tile i of layer l */
+            auto issue_next = [&]() {
+                const int s = t % ns;
+                const StackLayer &ly = S.layer[l];
+                if (i < nt1) copy_pairs(P, ly.gate_up, ly.gate_up_s, b1 + i * P.p1.TR, e1, ring + (size_t)s * P.stage_bytes, &sm->full[s]);
+                else copy_rows(P, ly.down, ly.down_s, b2 + (i - nt1) * P.p2.TR, e2, ring + (size_t)s * P.stage_bytes, &sm->full[s]);
+                ++t;
+                if (++i == nt) { i = 0; ++l; }
+            };
+            if (P.early_weights)
+                while (t < min(ns, total)) issue_next();
+            griddep_wait();
+            const unsigned base = P.sync[1];
+            stamp(P, 1);
+            bool failed = false;
+            int fetched = 0;
+            /* hand-over k: act of layer k / 2 (k even), the residual stream behind layer k / 2 (k odd) */
+            auto fetch = [&]() {
+                if (!grid_barrier_open(P.sync + 0, base + (unsigned)(fetched + 1) * gridDim.x, &sm->abort_flag)) {
+                    give_up(sm, P.sync, ST_GRID_BARRIER);
+                    failed = true;
+                    return;
+                }
+                const bool of_act = !(fetched & 1);
+                const uint32_t bytes = (uint32_t)(P.M * (of_act ? P.I : P.H) * 2);
+                stamp(P, of_act ? 6 : 13);
+                asm volatile("fence.proxy.async;" ::: "memory"); /* the other CTAs' stores before this thread's copy */
+                mbar_expect_tx(&sm->x_full, bytes);
+                bulk_g2s(xs, of_act ? P.act : P.residual, bytes, &sm->x_full);
+                ++fetched;
+            };
+            /* The stage to be filled is released once its last tile has been multiplied, so that tile's input has
+             * to be fetched first: hand-over 2l - 1 for a tile of gate/up, 2l for one of the down projection. */
+            int freed_l = 0, freed_i = 0;
+            while (t < total && !failed) {
+                if (t >= ns) {
+                    const int need = 2 * freed_l - (freed_i < nt1 ? 1 : 0);
+                    while (fetched <= need && !failed) fetch();
+                    if (failed) break;
+                    if (++freed_i == nt) { freed_i = 0; ++freed_l; }
+                    if (!mbar_wait<20>(&sm->empty[t % ns], (uint32_t)(t / ns - 1) & 1u, &sm->abort_flag)) {
+                        give_up(sm, P.sync, ST_PRODUCER_EMPTY);
+                        failed = true;
+                        break;
+                    }
+                }
+                issue_next();
+            }
+            while (fetched < hands && !failed) fetch();
+            for (int u = max(0, t - ns); u < t; ++u) drain(&sm->full[u % ns], (uint32_t)(u / ns) & 1u, P.sync);
+            if (fetched > 0) drain(&sm->x_full, (uint32_t)(fetched - 1) & 1u, P.sync);
+        }
+    } else if (warp <= kConsumerWarps) {
+        /* ---------------- consumers ---------------- */
+        griddep_wait();
+        for (int l = 0; l < S.layers && !*(volatile int *)&sm->abort_flag; ++l) {
+            consume_phase<CIT1, MT, true, true>(P, P.p1, sm, xs, ring, l * nt, 2 * l - 1, S.layer[l].norm_w);
+            if (*(volatile int *)&sm->abort_flag) break;
+            consume_phase<CIT2, MT, false, true>(P, P.p2, sm, xs, ring, l * nt + nt1, 2 * l, nullptr);
+        }
+    } else {
+        /* ---------------- epilogue ---------------- */
+        griddep_wait();
+        for (int l = 0; l < S.layers; ++l) {
+            if (!epilogue_phase<MT, true, true>(P, P.p1, sm, l * nt, 0, false)) break;
+            __syncwarp();
+            if (lane == 0) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(P.sync + 0) : "memory");
+            if (lane == 0) stamp(P, 5);
+            if (!epilogue_phase<MT, false, true>(P, P.p2, sm, l * nt + nt1, 0, l + 1 == S.layers)) break;
+            __syncwarp();
+            if (l + 1 < S.layers && lane == 0) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(P.sync + 0) : "memory");
+            if (lane == 0) stamp(P, 10);
+        }
+    }
+    __syncthreads();
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        P.sync[1] += (unsigned)hands * gridDim.x;
+        stamp(P, 12);
+    }
+}
+
 /* ============================================================================================= */
 /* Host side: per-device state, the tiling plan, the launch                                      */
 /* ============================================================================================= */
@@ -522,7 +686,7 @@ struct DeviceState {
     int smem_optin = 0;
     int cooperative = 0;
     unsigned *sync = nullptr; /* 4 words: count, generation, sequence, status */
-    bool attr_set[2][2][2] = {};
+    bool attr_set[2][2][2][2] = {};
     int overlap_ok = 0; /* dependent launch next to a cooperative one: 0 not tried yet, 1 taken, -1 refused */
 };
 static DeviceState g_dev[64];
@@ -564,6 +728,19 @@ static int device_state(DeviceState **out) {
     return FFN_OK;
 }
 
+/* The stages of a launch whose tiles and input copy are known. */
+static bool plan_ring(FusedParams &P, int tokens, int smem_optin, size_t &smem) {
+    P.stage_w_bytes = round_up(max(2 * P.p1.TR * P.p1.rb, P.p2.TR * P.p2.rb), 128);
+    P.sc_half_bytes = round_up(max(P.p1.TR * P.p1.G * 2, P.p2.TR * P.p2.G * 2) + 32, 16);
+    P.stage_bytes = round_up(P.stage_w_bytes + 2 * P.sc_half_bytes, 128);
+    const size_t fixed = fused_smem_header(tokens) + (size_t)P.xs_bytes;
+    if (fixed + 2 * (size_t)P.stage_bytes > (size_t)smem_optin) return false;
+    P.nstages = (int)min((size_t)kMaxStages, ((size_t)smem_optin - fixed) / (size_t)P.stage_bytes);
+    if (P.nstages < 2) return false;
+    smem = fixed + (size_t)P.nstages * P.stage_bytes;
+    return true;
+}
+
 /* The whole geometry of a launch from the shape alone (no device needed): the two phases' thread
  * layouts and tiles, the stage size, how many stages the shared memory holds.  Pointers are left to
  * the caller.  Returns false when the kernel does not take the shape. */
@@ -579,30 +756,20 @@ static bool plan_fused(FusedParams &P, int tokens, int H, int I, int smem_optin,
     P.p2.rows_total = H; P.p2.up_offset = 0;
     const int part_floats = tokens == 1 ? kPartFloats1 : kPartFloats2;
     if (P.p1.TR * 2 * tokens * P.p1.nhw > part_floats || P.p2.TR * tokens * P.p2.nhw > part_floats) return false;
-    P.stage_w_bytes = round_up(max(2 * P.p1.TR * P.p1.rb, P.p2.TR * P.p2.rb), 128);
-    P.sc_half_bytes = round_up(max(P.p1.TR * P.p1.G * 2, P.p2.TR * P.p2.G * 2) + 32, 16);
-    P.stage_bytes = round_up(P.stage_w_bytes + 2 * P.sc_half_bytes, 128);
     P.xs_bytes = round_up(tokens * I * 2, 128); /* act only: x is read from global memory */
-    const size_t fixed = fused_smem_header(tokens) + (size_t)P.xs_bytes;
-    if (fixed + 2 * (size_t)P.stage_bytes > (size_t)smem_optin) return false;
-    P.nstages = (int)min((size_t)kMaxStages, ((size_t)smem_optin - fixed) / (size_t)P.stage_bytes);
-    if (P.nstages < 2) return false;
-    smem = fixed + (size_t)P.nstages * P.stage_bytes;
-    return true;
+    return plan_ring(P, tokens, smem_optin, smem);
 }
 
-template <int C1, int C2, int MT>
-static int launch_fused(DeviceState &d, const FusedParams &P_in, int grid, size_t smem, cudaStream_t stream) {
+/* `kernel` with its parameters `params`, whose FusedParams part is P */
+template <typename Params>
+static int launch_cooperative(DeviceState &d, bool &attr_set, void (*kernel)(const Params), Params &params, FusedParams &P, int grid, size_t smem, cudaStream_t stream) {
     {
         std::lock_guard<std::mutex> lock(g_dev_mutex);
-        bool &set = d.attr_set[C1 - 1][C2 - 1][MT - 1];
-        if (!set) {
-            FFN_CUDA_TRY(cudaFuncSetAttribute(ffn_fused_kernel<C1, C2, MT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                              d.smem_optin), "fused FFN: shared-memory opt-in");
-            set = true;
+        if (!attr_set) {
+            FFN_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, d.smem_optin), "fused FFN: shared-memory opt-in");
+            attr_set = true;
         }
     }
-    FusedParams P = P_in;
     /* Programmatic dependent launch: consecutive launches in one stream overlap this launch's start
      * (CTA scheduling, barrier set-up, the first weight copies) with the tail of the one before.
      * Whether the driver takes the attribute next to a cooperative launch is found out once per
@@ -631,7 +798,7 @@ static int launch_fused(DeviceState &d, const FusedParams &P_in, int grid, size_
         attrs[1].val.cooperative = 1;
         cfg.attrs = attrs;
         cfg.numAttrs = 2;
-        const cudaError_t err = cudaLaunchKernelEx(&cfg, ffn_fused_kernel<C1, C2, MT>, P);
+        const cudaError_t err = cudaLaunchKernelEx(&cfg, kernel, params);
         if (err == cudaSuccess) {
             if (overlap == 2) d.overlap_ok = 1;
             return FFN_OK;
@@ -641,10 +808,18 @@ static int launch_fused(DeviceState &d, const FusedParams &P_in, int grid, size_
         d.overlap_ok = -1;
         P.early_weights = 0;
     }
-    void *args[] = {(void *)&P};
-    FFN_CUDA_TRY(cudaLaunchCooperativeKernel((const void *)ffn_fused_kernel<C1, C2, MT>, dim3(grid), dim3(kThreads),
-                                             args, smem, stream), "fused FFN launch");
+    void *args[] = {(void *)&params};
+    FFN_CUDA_TRY(cudaLaunchCooperativeKernel((const void *)kernel, dim3(grid), dim3(kThreads), args, smem, stream), "fused FFN launch");
     return FFN_OK;
+}
+template <int C1, int C2, int MT>
+static int launch_fused(DeviceState &d, const FusedParams &P_in, int grid, size_t smem, cudaStream_t stream) {
+    FusedParams P = P_in;
+    return launch_cooperative(d, d.attr_set[0][C1 - 1][C2 - 1][MT - 1], ffn_fused_kernel<C1, C2, MT>, P, P, grid, smem, stream);
+}
+template <int C1, int C2, int MT>
+static int launch_stack(DeviceState &d, StackParams &S, int grid, size_t smem, cudaStream_t stream) {
+    return launch_cooperative(d, d.attr_set[1][C1 - 1][C2 - 1][MT - 1], ffn_stack_kernel<C1, C2, MT>, S, S.f, grid, smem, stream);
 }
 
 int fused_ffn_launch(cudaStream_t stream, const void *normed, void *act, void *layer_out,
@@ -713,6 +888,73 @@ int fused_ffn_launch(cudaStream_t stream, const void *normed, void *act, void *l
     }
     FFN_LAUNCH(1, 1, 2);
 #undef FFN_LAUNCH
+}
+
+/* Bytes of the smaller phase's tiles that the ring holds: what is on its way from HBM at the worst time. */
+static size_t ring_bytes(const FusedParams &P) { return (size_t)P.nstages * min(2 * P.p1.TR * P.p1.rb, P.p2.TR * P.p2.rb); }
+/* The plan of a stack: the threads' columns and rows of a single layer's (the same sums in the same order), with
+ * the row steps of both phases' tiles chosen so that the ring holds the most. */
+static bool plan_stack(FusedParams &P, int tokens, int H, int I, int smem_optin, int &c1, int &c2, size_t &smem) {
+    if (!plan_fused(P, tokens, H, I, smem_optin, kDefaultStageTarget, c1, c2, smem)) return false;
+    FusedParams best = P;
+    const int most1 = P.p1.JT, most2 = P.p2.JT, xs_bytes = round_up(tokens * max(H, I) * 2, 128); /* act or the residual stream */
+    for (int j1 = most1; j1 >= 1; --j1)
+        for (int j2 = most2; j2 >= 1; --j2) {
+            FusedParams T = P;
+            T.p1.JT = j1; T.p1.TR = j1 * T.p1.RG;
+            T.p2.JT = j2; T.p2.TR = j2 * T.p2.RG;
+            T.xs_bytes = xs_bytes;
+            size_t bytes = 0;
+            if (plan_ring(T, tokens, smem_optin, bytes) && (best.xs_bytes != xs_bytes || ring_bytes(T) > ring_bytes(best))) {
+                best = T;
+                smem = bytes;
+            }
+        }
+    P = best;
+    return P.xs_bytes == xs_bytes;
+}
+
+int fused_stack_launch(cudaStream_t stream, void *h, void *act, void *layer_out, const FfnMlpWeights *layers, int num_layers,
+                       int tokens, int H, int I, float eps, int gemma) {
+    if (tokens < 1 || tokens > 2 || num_layers < 2) return FFN_NOT_ADMITTED;
+    DeviceState *dp = nullptr;
+    const int st = device_state(&dp);
+    if (st) return st;
+    DeviceState &d = *dp;
+    const int grid = d.sm_count;
+    if (!d.cooperative || H < grid || I < grid) return FFN_NOT_ADMITTED; /* every CTA has rows in both phases */
+    uintptr_t any = (uintptr_t)h | (uintptr_t)act;
+    for (int l = 0; l < num_layers; ++l) {
+        const FfnMlpWeights &w = layers[l];
+        if (!w.gate_up_i4 || !w.gate_up_i4_scales || !w.down_i4 || !w.down_i4_scales || w.i4_group != FFN_INT4_GROUP || !w.post_norm_w) return FFN_NOT_ADMITTED;
+        if (ffn_decode_layer_is_prepared(&w)) return FFN_NOT_ADMITTED; /* its own kernel */
+        any |= (uintptr_t)w.gate_up_i4 | (uintptr_t)w.gate_up_i4_scales | (uintptr_t)w.down_i4 | (uintptr_t)w.down_i4_scales | (uintptr_t)w.post_norm_w;
+    }
+    if (any & 15) return FFN_NOT_ADMITTED;
+    StackParams S = {};
+    FusedParams &P = S.f;
+    int c1 = 0, c2 = 0;
+    size_t smem = 0;
+    if (!plan_stack(P, tokens, H, I, d.smem_optin, c1, c2, smem)) return FFN_NOT_ADMITTED;
+    P.x = (const uint16_t *)h; P.residual = (uint16_t *)h;
+    P.act = (uint16_t *)act; P.out = (uint16_t *)layer_out;
+    P.sync = d.sync;
+    P.tp = 1;
+    P.norm_eps = eps; P.norm_gemma = gemma;
+    P.trace = g_trace;
+    for (int l0 = 0; l0 < num_layers; l0 += kStackMaxLayers) {
+        S.layers = min(kStackMaxLayers, num_layers - l0);
+        for (int l = 0; l < S.layers; ++l) {
+            const FfnMlpWeights &w = layers[l0 + l];
+            S.layer[l] = {w.gate_up_i4, w.down_i4, (const uint16_t *)w.gate_up_i4_scales, (const uint16_t *)w.down_i4_scales, (const uint16_t *)w.post_norm_w};
+        }
+        int rc;
+        if (tokens == 2) rc = launch_stack<1, 1, 2>(d, S, grid, smem, stream);
+        else if (c1 == 1) rc = c2 == 1 ? launch_stack<1, 1, 1>(d, S, grid, smem, stream) : launch_stack<1, 2, 1>(d, S, grid, smem, stream);
+        else rc = c2 == 1 ? launch_stack<2, 1, 1>(d, S, grid, smem, stream) : launch_stack<2, 2, 1>(d, S, grid, smem, stream);
+        if (rc) return rc;
+    }
+    return FFN_OK;
 }
 
 int fused_ffn_try(cudaStream_t stream, const void *normed, void *act, void *layer_out,

@@ -158,21 +158,28 @@ __device__ __forceinline__ void load_chunk(uint32_t (&v)[16], const uint16_t *sr
     }
 }
 
+/* RMSNorm of a slice: the reference's expression and its BF16 rounding */
+__device__ __forceinline__ void norm_chunk(uint32_t (&v)[16], const uint4 (&w)[4], float inv_rms, float gemma) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const uint32_t ww[4] = {w[q].x, w[q].y, w[q].z, w[q].w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const float lo = bf16_lo(v[4 * q + i]) * inv_rms * (bf16_lo(ww[i]) + gemma);
+            const float hi = bf16_hi(v[4 * q + i]) * inv_rms * (bf16_hi(ww[i]) + gemma);
+            v[4 * q + i] = (uint32_t)f32_to_bf16_bits(lo) | ((uint32_t)f32_to_bf16_bits(hi) << 16);
+        }
+    }
+}
+
 __device__ __forceinline__ void prepare_chunk(XChunk &xc, uint32_t (&v)[16], bool on,
                                               const uint16_t *norm_w = nullptr /* global, this chunk's 32 weights */,
                                               float inv_rms = 1.0f, float gemma = 0.0f) {
-    if (norm_w != nullptr && on) { /* fused RMSNorm: the reference's expression and its BF16 rounding */
+    if (norm_w != nullptr && on) {
+        uint4 w[4];
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const uint4 wq = __ldg((const uint4 *)(norm_w + q * 8));
-            const uint32_t ww[4] = {wq.x, wq.y, wq.z, wq.w};
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const float lo = bf16_lo(v[4 * q + i]) * inv_rms * (bf16_lo(ww[i]) + gemma);
-                const float hi = bf16_hi(v[4 * q + i]) * inv_rms * (bf16_hi(ww[i]) + gemma);
-                v[4 * q + i] = (uint32_t)f32_to_bf16_bits(lo) | ((uint32_t)f32_to_bf16_bits(hi) << 16);
-            }
-        }
+        for (int q = 0; q < 4; ++q) w[q] = __ldg((const uint4 *)(norm_w + q * 8));
+        norm_chunk(v, w, inv_rms, gemma);
     }
     uint32_t mx = 0; /* per-halfword maximum of the magnitude bits */
 #pragma unroll

@@ -44,7 +44,7 @@ def upload_layer(layer, device, tp=1, rank=0, with_norm=False, prepare=False):
     return mlp.prepare() if prepare else mlp
 
 
-KERNEL_KINDS = ("stream_tc_kernel", "ffn_imma_kernel", "ffn_kmajor_kernel", "ffn_fused_kernel", "gate_up_mma_kernel", "ffn_tc_kernel",
+KERNEL_KINDS = ("stream_tc_kernel", "ffn_imma_kernel", "ffn_kmajor_kernel", "ffn_fused_kernel", "ffn_stack_kernel", "gate_up_mma_kernel", "ffn_tc_kernel",
                 "gemm_int4_rows_kernel")
 
 
