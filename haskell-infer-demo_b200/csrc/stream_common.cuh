@@ -19,10 +19,10 @@ constexpr int kPartSlots = 4;
 constexpr int kPartFloats1 = 160;                      /* floats per partial slot, one token: JT*NVROW*RG*CT/16 <= 4*544/16 = 136 */
 constexpr int kPartFloats2 = 288;                      /* two tokens: <= 8*544/16 = 272 */
 constexpr int kMaxJT = 4;                              /* row steps per thread per tile */
-/* Bounded waits, in polls.  Of a word in global memory: 32..100 ns and more each, i.e. 0.15 .. 0.5 s.  A try_wait that
+/* Bounded waits, in polls.  Of a word in global memory: 32..100 ns and more each, i.e. 1.2 .. 4 s.  A try_wait that
  * finds the barrier closed has suspended its thread for 0.07 us (32 warps of a CTA polling) to 1.4 us (a single one)
- * on B200, to which mbar_wait adds its sleep: 0.3 .. 6 s. */
-constexpr uint32_t kSpinLimit = 1u << 22;
+ * on B200, to which mbar_wait adds its sleep: 2.4 .. 48 s.  Long enough for a launch some of whose CTAs wait for an SM. */
+constexpr uint32_t kSpinLimit = 1u << 25;
 
 /* status word values (where a wait gave up) */
 enum { ST_OK = 0, ST_PRODUCER_EMPTY = 1, ST_CONSUMER_FULL = 2, ST_PART_EMPTY = 3, ST_PART_FULL = 4,

@@ -301,7 +301,7 @@ long long ffn_int4_tile_order_offset(int token, int k, int padded_tokens);
  * output or the exchange slots.  The weight copies issued before that wait read the INT4 operands and
  * their scales, which therefore must not be written by the kernel that directly precedes the call in
  * the stream (the reference loads them once at start-up: csrc/safetensors_loader.cu); every other
- * operand may be.  0 turns the attribute off (plain cooperative launches, as CUDA orders them); any
+ * operand may be.  0 turns the attribute off (cooperative launches, as CUDA orders them); any
  * other value queries.  Returns the previous setting.  The reference has no counterpart: its launches
  * are ordered by the stream alone (csrc/kernels/layers.cu:164, forward_mlp_prepared). */
 int ffn_int4_set_launch_overlap(int on);
