@@ -52,9 +52,11 @@ struct FusedParams {
     uint16_t *out;        /* [M][H] bf16 */
     PhasePlan p1, p2;
     int M, H, I;
-    int stage_bytes, nstages, xs_bytes;
+    int stage_bytes, nstages;
+    int xs_bytes;         /* copied input; a stack's byte planes take its place and the slices' factors follow at fac_offset */
+    int fac_offset;
     int stage_w_bytes;    /* weights part of a stage; the tile's scales follow it */
-    int sc_half_bytes;    /* room for one contiguous run of scales (gate or up) incl. 16 bytes of slack */
+    int sc_half_bytes;    /* room for the gate rows' run of scales with its slack to 16-byte boundaries; the up rows' run follows */
     unsigned *sync;       /* [0] arrivals (monotonic), [1] arrivals at the end of the previous launch,
                              [2] unused, [3] status */
     /* tensor parallelism (tp == 1: unused) */
@@ -104,9 +106,9 @@ struct Smem {
     uint64_t empty[kMaxStages];
     uint64_t part_full[kPartSlots];
     uint64_t part_empty[kPartSlots];
-    uint64_t norm_full, x_full; /* a stack: every warp's part of the sum of squares is there; the hand-over's copy is */
+    uint64_t norm_full, x_full, prep_full; /* every warp's part of the sum of squares is there; the hand-over's copy; every warp's part of the prepared input */
     int abort_flag;
-    int pad[11];
+    int pad[9];
     float norm_red[2][kConsumerWarps + 3];
     float part[1]; /* kPartSlots slots of kPartFloats1 or kPartFloats2 floats follow (sized by the token count) */
 };
@@ -133,12 +135,136 @@ __device__ __forceinline__ void stamp(const FusedParams &P, int slot) {
     }
 }
 
+/* ---- a stack's input of one phase: block fixed point, once per CTA ------------------------------- */
+/* A consumer thread multiplies every row of its row group by the same 32 or 64 activations, and a CTA has up to 34 row
+ * groups: converting them in every thread, as the single layer does, is up to 4.4 us of instructions a phase (a norm and
+ * 1024 values, 34 row groups).  Here four lanes share a slice of 32 values, 8 each, and leave its byte planes in `xs` - where
+ * the BF16 values lay if a copy brought them - and its factor behind them: piece p (he, ho, le, lo) of slice c at 16-byte
+ * slot (p + c / 2) % 4 of the slice's 64 bytes, so that neither the lanes' words here nor the threads' 16-byte loads later
+ * share banks.  us per stack, 1 token: 24 layers of 1024 x 3072 320 -> 239, 36 of 2560 x 9728 607 -> 587, 32 of 5120 x 17408
+ * 1052 -> 1013 (the latter two with tiles of their full size, plan_stack).  The single layer has no use for it: 5120 x 17408
+ * 30.7 -> 31.8 us.  `hand` as below. */
+constexpr int kStageRounds = 4; /* pieces of 8 values a thread holds at a time: 17408 values in one go */
+__device__ __forceinline__ int plane_slot(int chunk, int piece) { return chunk * 64 + (((piece + (chunk >> 1)) & 3) << 4); }
+
+template <int CIT, int MT, bool PAIRS>
+__device__ __forceinline__ bool stage_input(const FusedParams &P, const PhasePlan &pl, Smem *sm, uint16_t *xs, int hand, const uint16_t *norm_w) {
+    const int ti = threadIdx.x - 32, lane = threadIdx.x & 31;
+    const bool direct = hand < 0;
+    const int per_row = pl.K / 8, total = MT * per_row, batch = kStageRounds * kConsumerThreads;
+    float *fac = (float *)((uint8_t *)xs + P.fac_offset);
+    uint4 v[kStageRounds], nw[PAIRS ? kStageRounds : 1];
+    auto load_norm = [&](int b) {
+#pragma unroll
+        for (int r = 0; r < kStageRounds; ++r) {
+            const int q = b + r * kConsumerThreads + ti;
+            nw[PAIRS ? r : 0] = make_uint4(0, 0, 0, 0);
+            if (q < total) nw[PAIRS ? r : 0] = __ldg((const uint4 *)norm_w + (MT == 2 && q >= per_row ? q - per_row : q));
+        }
+    };
+    auto load = [&](int b) {
+#pragma unroll
+        for (int r = 0; r < kStageRounds; ++r) {
+            const int q = b + r * kConsumerThreads + ti;
+            v[r] = make_uint4(0, 0, 0, 0);
+            if (q < total) v[r] = direct ? __ldg((const uint4 *)P.x + q) : lds16(xs + q * 8);
+        }
+    };
+    if (PAIRS) load_norm(0); /* a stack: while the layer before is finished elsewhere */
+    if (!direct && !mbar_wait<64>(&sm->x_full, (uint32_t)hand & 1u, &sm->abort_flag)) {
+        give_up(sm, P.sync, PAIRS ? ST_NEXT_X : ST_X_FULL);
+        return false;
+    }
+    if (threadIdx.x == 32) stamp(P, PAIRS ? 15 : 14);
+    load(0);
+    float inv_rms[MT];
+#pragma unroll
+    for (int m = 0; m < MT; ++m) inv_rms[m] = 1.0f;
+    if (PAIRS) { /* every CTA needs the whole normalized vector, so every CTA takes the (cheap) norm */
+        /* the sum of squares by the threads of one row group, a slice or two each, as the single layer takes it: the same bits */
+#pragma unroll
+        for (int m = 0; m < MT; ++m) {
+            float ss = 0.0f;
+            if (ti < pl.CT) {
+#pragma unroll
+                for (int c = 0; c < CIT; ++c) {
+                    const int col = ti + c * pl.CT;
+                    const size_t at = (size_t)m * pl.K + (size_t)min(col, pl.cpr - 1) * 32;
+                    uint32_t e[16];
+                    if (direct) load_chunk<true>(e, P.x + at, col < pl.cpr);
+                    else load_chunk<false>(e, xs + at, col < pl.cpr);
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) { ss = fmaf(bf16_lo(e[i]), bf16_lo(e[i]), ss); ss = fmaf(bf16_hi(e[i]), bf16_hi(e[i]), ss); }
+                }
+            }
+            ss = warp_sum(ss);
+            if (lane == 0) sm->norm_red[m][ti >> 5] = ss;
+        }
+        if (lane == 0) mbar_arrive(&sm->norm_full);
+        if (!mbar_wait<20>(&sm->norm_full, (uint32_t)((hand + 1) >> 1) & 1u, &sm->abort_flag)) { /* a warp that gave up does not come */
+            give_up(sm, P.sync, ST_NEXT_X);
+            return false;
+        }
+#pragma unroll
+        for (int m = 0; m < MT; ++m) {
+            float sum = 0.0f;
+#pragma unroll
+            for (int w = 0; w < kConsumerWarps; ++w) sum += sm->norm_red[m][w];
+            inv_rms[m] = rsqrtf(sum / (float)pl.K + P.norm_eps);
+        }
+    }
+    for (int b = 0; b < total; b += batch) {
+        if (b > 0) {
+            load(b);
+            if (PAIRS) load_norm(b);
+        }
+#pragma unroll
+        for (int r = 0; r < kStageRounds; ++r) {
+            const int q0 = b + r * kConsumerThreads + (ti & ~31), q = q0 + lane, chunk = q >> 2, j = q & 3;
+            if (q0 >= total) break; /* the warp agrees */
+            uint32_t e[4] = {v[r].x, v[r].y, v[r].z, v[r].w};
+            if (PAIRS) { /* the reference's expression and its BF16 rounding */
+                const uint4 w = nw[PAIRS ? r : 0];
+                const uint32_t ww[4] = {w.x, w.y, w.z, w.w};
+                const float inv = MT == 2 && q >= per_row ? inv_rms[MT - 1] : inv_rms[0], gemma = P.norm_gemma ? 1.0f : 0.0f;
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const float lo = bf16_lo(e[i]) * inv * (bf16_lo(ww[i]) + gemma);
+                    const float hi = bf16_hi(e[i]) * inv * (bf16_hi(ww[i]) + gemma);
+                    e[i] = (uint32_t)f32_to_bf16_bits(lo) | ((uint32_t)f32_to_bf16_bits(hi) << 16);
+                }
+            }
+            uint32_t top = 0; /* the largest magnitude's bits */
+#pragma unroll
+            for (int i = 0; i < 4; ++i) top = max(top, max(e[i] & 0x7FFFu, (e[i] >> 16) & 0x7FFFu));
+            top = max(top, __shfl_xor_sync(~0u, top, 1));
+            top = max(top, __shfl_xor_sync(~0u, top, 2));
+            __syncwarp(); /* the slice's four lanes have read it */
+            if (q < total) {
+                uint32_t planes[4];
+                const float f = fixed_point8(e, (int)(top >> 7), planes);
+                uint8_t *to = (uint8_t *)xs + j * 4;
+#pragma unroll
+                for (int p = 0; p < 4; ++p) *(uint32_t *)(to + plane_slot(chunk, p)) = planes[p];
+                if (j == 0) fac[chunk] = f;
+            }
+        }
+    }
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&sm->prep_full);
+    if (!mbar_wait<20>(&sm->prep_full, (uint32_t)(hand + 1) & 1u, &sm->abort_flag)) {
+        give_up(sm, P.sync, ST_ACT_READY);
+        return false;
+    }
+    return true;
+}
+
 /* ---- consumer side of one phase ------------------------------------------------------------ */
 /* `hand` numbers the hand-over between CTAs that brings the phase's input (act of the launch's first layer 0,
  * then the residual stream and act in turn), -1: it is there when the kernel starts. */
 template <int CIT, int MT, bool PAIRS, bool STACK>
 __device__ __forceinline__ void consume_phase(const FusedParams &P, const PhasePlan &pl, Smem *sm,
-                                              const uint16_t *xs, uint8_t *ring, int tile0, int hand, const uint16_t *norm_w) {
+                                              uint16_t *xs, uint8_t *ring, int tile0, int hand, const uint16_t *norm_w) {
     constexpr int NVROW = (PAIRS ? 2 : 1) * MT;
     constexpr int VALS = 4 * MT;   /* values a thread carries through a tile: one transposed reduction per four */
     constexpr int JTM = VALS / NVROW; /* row steps per thread per tile: 2 of pairs, 4 of single rows */
@@ -151,88 +277,91 @@ __device__ __forceinline__ void consume_phase(const FusedParams &P, const PhaseP
     const unsigned hmask = 0xFFFFu << (lane & 16);
     const int row_begin = cta_begin(pl.rows_total, blockIdx.x, gridDim.x);
     const int row_end = cta_begin(pl.rows_total, blockIdx.x + 1, gridDim.x);
-    const int ntiles = (row_end - row_begin + pl.TR - 1) / pl.TR;
 
-    /* This thread's 32-element slice(s) of the activation vector(s).  Phase 1 reads x straight from
-     * global memory: it is there when the kernel starts, so the loads are in flight while the
-     * producer is still setting up.  Phase 2 waits for the copy of act the producer brings into
-     * shared memory once the grid barrier has opened. */
-    const bool direct = STACK ? hand < 0 : PAIRS || P.gemv; /* single-matrix mode: the activation is an input too */
-    uint4 nw[STACK && PAIRS ? CIT : 1][4]; /* a stack's norm weights are fetched while the layer before is finished elsewhere */
-    if (STACK && PAIRS) {
+    XChunk xc[CIT][MT]; /* this thread's 32-element slice(s) of the activation vector(s), in registers for the whole phase */
+    if constexpr (STACK) {
+        if (!stage_input<CIT, MT, PAIRS>(P, pl, sm, xs, hand, norm_w)) return;
+        const uint32_t planes = smem_u32(xs);
+        const float *fac = (const float *)((const uint8_t *)xs + P.fac_offset);
 #pragma unroll
         for (int c = 0; c < CIT; ++c)
 #pragma unroll
-            for (int q = 0; q < 4; ++q) nw[c][q] = __ldg((const uint4 *)(norm_w + (size_t)min(ct + c * pl.CT, pl.cpr - 1) * 32 + q * 8));
-    }
-    if (!direct && !mbar_wait<64>(&sm->x_full, (uint32_t)hand & 1u, &sm->abort_flag)) {
-        give_up(sm, P.sync, STACK && PAIRS ? ST_NEXT_X : ST_X_FULL);
-        return;
-    }
-    const uint16_t *src = direct ? P.x : xs;
-    uint32_t xv[CIT][MT][16];
+            for (int m = 0; m < MT; ++m) {
+                const int col = ct + c * pl.CT, chunk = m * pl.cpr + min(col, pl.cpr - 1);
+                const bool on = active && col < pl.cpr; /* an absent slice is all zeros */
+                uint4 p[4];
 #pragma unroll
-    for (int c = 0; c < CIT; ++c)
-#pragma unroll
-        for (int m = 0; m < MT; ++m) {
-            const int col = ct + c * pl.CT;
-            const uint16_t *from = src + (size_t)m * pl.K + (size_t)min(col, pl.cpr - 1) * 32;
-            if (direct) load_chunk<true>(xv[c][m], from, active && col < pl.cpr);
-            else load_chunk<false>(xv[c][m], from, active && col < pl.cpr);
-        }
-    float inv_rms[MT];
-#pragma unroll
-    for (int m = 0; m < MT; ++m) inv_rms[m] = 1.0f;
-    const bool normalize = PAIRS && (STACK || norm_w != nullptr);
-    if (normalize) { /* every CTA needs the whole normalized vector, so every CTA takes the (cheap) norm */
-#pragma unroll
-        for (int m = 0; m < MT; ++m) {
-            float ss = 0.0f;
-            if (rg == 0) { /* row group 0 covers every slice exactly once; absent slices hold zeros */
-#pragma unroll
-                for (int c = 0; c < CIT; ++c)
-#pragma unroll
-                    for (int i = 0; i < 16; ++i) {
-                        const uint32_t pr = xv[c][m][i];
-                        ss = fmaf(bf16_lo(pr), bf16_lo(pr), ss);
-                        ss = fmaf(bf16_hi(pr), bf16_hi(pr), ss);
-                    }
+                for (int i = 0; i < 4; ++i) {
+                    p[i] = lds16_at(planes + plane_slot(chunk, i));
+                    if (!on) p[i] = make_uint4(0, 0, 0, 0);
+                }
+                XChunk &x = xc[c][m];
+                x.he[0] = p[0].x; x.he[1] = p[0].y; x.he[2] = p[0].z; x.he[3] = p[0].w;
+                x.ho[0] = p[1].x; x.ho[1] = p[1].y; x.ho[2] = p[1].z; x.ho[3] = p[1].w;
+                x.le[0] = p[2].x; x.le[1] = p[2].y; x.le[2] = p[2].z; x.le[3] = p[2].w;
+                x.lo[0] = p[3].x; x.lo[1] = p[3].y; x.lo[2] = p[3].z; x.lo[3] = p[3].w;
+                x.fac = on ? fac[chunk] : 0.0f;
             }
-            ss = warp_sum(ss);
-            if (lane == 0) sm->norm_red[m][ti >> 5] = ss;
+    } else {
+        /* This thread's 32-element slice(s) of the activation vector(s).  Phase 1 reads x straight from
+         * global memory: it is there when the kernel starts, so the loads are in flight while the
+         * producer is still setting up.  Phase 2 waits for the copy of act the producer brings into
+         * shared memory once the grid barrier has opened. */
+        const bool direct = PAIRS || P.gemv; /* single-matrix mode: the activation is an input too */
+        if (!direct && !mbar_wait<64>(&sm->x_full, 0u, &sm->abort_flag)) {
+            give_up(sm, P.sync, ST_X_FULL);
+            return;
         }
-        if (STACK) { /* a wait with a limit: a warp that gave up in an earlier phase does not come */
-            if (lane == 0) mbar_arrive(&sm->norm_full);
-            if (!mbar_wait<20>(&sm->norm_full, (uint32_t)((hand + 1) >> 1) & 1u, &sm->abort_flag)) {
-                give_up(sm, P.sync, ST_NEXT_X);
-                return;
+        const uint16_t *src = direct ? P.x : xs;
+        uint32_t xv[CIT][MT][16];
+#pragma unroll
+        for (int c = 0; c < CIT; ++c)
+#pragma unroll
+            for (int m = 0; m < MT; ++m) {
+                const int col = ct + c * pl.CT;
+                const uint16_t *from = src + (size_t)m * pl.K + (size_t)min(col, pl.cpr - 1) * 32;
+                if (direct) load_chunk<true>(xv[c][m], from, active && col < pl.cpr);
+                else load_chunk<false>(xv[c][m], from, active && col < pl.cpr);
             }
-        } else {
+        float inv_rms[MT];
+#pragma unroll
+        for (int m = 0; m < MT; ++m) inv_rms[m] = 1.0f;
+        const bool normalize = PAIRS && norm_w != nullptr;
+        if (normalize) { /* every CTA needs the whole normalized vector, so every CTA takes the (cheap) norm */
+#pragma unroll
+            for (int m = 0; m < MT; ++m) {
+                float ss = 0.0f;
+                if (rg == 0) { /* row group 0 covers every slice exactly once; absent slices hold zeros */
+#pragma unroll
+                    for (int c = 0; c < CIT; ++c)
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) {
+                            const uint32_t pr = xv[c][m][i];
+                            ss = fmaf(bf16_lo(pr), bf16_lo(pr), ss);
+                            ss = fmaf(bf16_hi(pr), bf16_hi(pr), ss);
+                        }
+                }
+                ss = warp_sum(ss);
+                if (lane == 0) sm->norm_red[m][ti >> 5] = ss;
+            }
             asm volatile("bar.sync 1, %0;" ::"n"(kConsumerThreads) : "memory");
-        }
 #pragma unroll
-        for (int m = 0; m < MT; ++m) {
-            float total = 0.0f;
+            for (int m = 0; m < MT; ++m) {
+                float total = 0.0f;
 #pragma unroll
-            for (int w = 0; w < kConsumerWarps; ++w) total += sm->norm_red[m][w];
-            inv_rms[m] = rsqrtf(total / (float)pl.K + P.norm_eps);
-        }
-    }
-    XChunk xc[CIT][MT];
-#pragma unroll
-    for (int c = 0; c < CIT; ++c)
-#pragma unroll
-        for (int m = 0; m < MT; ++m) {
-            const int col = ct + c * pl.CT;
-            const bool on = active && col < pl.cpr;
-            const float gemma = P.norm_gemma ? 1.0f : 0.0f;
-            if (STACK && PAIRS) {
-                if (on) norm_chunk(xv[c][m], nw[STACK && PAIRS ? c : 0], inv_rms[m], gemma);
-                prepare_chunk(xc[c][m], xv[c][m], on);
-            } else {
-                prepare_chunk(xc[c][m], xv[c][m], on, normalize ? norm_w + (size_t)min(col, pl.cpr - 1) * 32 : nullptr, inv_rms[m], gemma);
+                for (int w = 0; w < kConsumerWarps; ++w) total += sm->norm_red[m][w];
+                inv_rms[m] = rsqrtf(total / (float)pl.K + P.norm_eps);
             }
         }
+#pragma unroll
+        for (int c = 0; c < CIT; ++c)
+#pragma unroll
+            for (int m = 0; m < MT; ++m) {
+                const int col = ct + c * pl.CT;
+                const bool on = active && col < pl.cpr;
+                prepare_chunk(xc[c][m], xv[c][m], on, normalize ? norm_w + (size_t)min(col, pl.cpr - 1) * 32 : nullptr, inv_rms[m], P.norm_gemma ? 1.0f : 0.0f);
+            }
+    }
     if (threadIdx.x == 32) stamp(P, PAIRS ? 2 : 7);
 
     /* Instructions bound this loop (some 250 a tile and warp, 62 thousand an SM in a 2560 x 9728 layer, of which the products are
@@ -427,6 +556,7 @@ __device__ __forceinline__ void init_barriers(Smem *sm, int lane, int ns) {
     if (lane >= 8 && lane < 8 + kPartSlots) { mbar_init(&sm->part_full[lane - 8], kConsumerWarps); mbar_init(&sm->part_empty[lane - 8], 1); }
     if (lane == 16) mbar_init(&sm->norm_full, kConsumerWarps);
     if (lane == 17) mbar_init(&sm->x_full, 1);
+    if (lane == 18) mbar_init(&sm->prep_full, kConsumerWarps);
     if (lane == 31) sm->abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 }
@@ -575,10 +705,11 @@ __global__ void __launch_bounds__(kThreads, 1) ffn_fused_kernel(const FusedParam
 
 /* ---- a stack of layers: h <- bf16(h + FFN_l(RMSNorm_l(h))) for every layer in one launch ------- */
 /* HBM bound as the single layer, but its weights stream on through the hand-overs, and what a layer takes is the chain
- * of one: residual stream in (grid barrier, copy, norm and conversion), gate/up, act (the same), down.  Every CTA has rows
- * in both phases (the host sees to it), so an arrival at the barrier says that all the CTA's warps have read the input
- * before, and one copy in shared memory and the barriers' one-bit phases do.  The ring is cut into stages that hold the most
- * (plan_stack).  36 layers of 2560 x 9728, one token: 741 us as 36 launches, 633 so. */
+ * of one: residual stream in (grid barrier, copy, norm and conversion: 2.7 us of 16 for 2560 x 9728), gate/up (4.5, consumers'
+ * instructions), its sums and the arrival (1.8), act in (2.5), down (2.1), its sums and the arrival (2).  Every CTA has
+ * rows in both phases (the host sees to it), so an arrival at the barrier says that all the CTA's warps have read the
+ * input before, and one copy in shared memory and the barriers' one-bit phases do.  36 layers of 2560 x 9728, one
+ * token: 741 us as 36 launches, 633 at first, 587 now. */
 template <int CIT1, int CIT2, int MT>
 __global__ void __launch_bounds__(kThreads, 1) ffn_stack_kernel(const __grid_constant__ StackParams S) {
     const FusedParams &P = S.f;
@@ -630,7 +761,7 @@ __global__ void __launch_bounds__(kThreads, 1) ffn_stack_kernel(const __grid_con
                 const bool of_act = !(fetched & 1);
                 const uint32_t bytes = (uint32_t)(P.M * (of_act ? P.I : P.H) * 2);
                 stamp(P, of_act ? 6 : 13);
-                asm volatile("fence.proxy.async;" ::: "memory"); /* the other CTAs' stores before this thread's copy */
+                asm volatile("fence.proxy.async;" ::: "memory"); /* the other CTAs' stores, and this one's in xs, before the copy */
                 mbar_expect_tx(&sm->x_full, bytes);
                 bulk_g2s(xs, of_act ? P.act : P.residual, bytes, &sm->x_full);
                 ++fetched;
@@ -745,8 +876,8 @@ static int device_state(DeviceState **out) {
 /* The stages of a launch whose tiles and input copy are known. */
 static bool plan_ring(FusedParams &P, int tokens, int smem_optin, size_t &smem) {
     P.stage_w_bytes = round_up(max(2 * P.p1.TR * P.p1.rb, P.p2.TR * P.p2.rb), 128);
-    P.sc_half_bytes = round_up(max(P.p1.TR * P.p1.G * 2, P.p2.TR * P.p2.G * 2) + 32, 16);
-    P.stage_bytes = round_up(P.stage_w_bytes + 2 * P.sc_half_bytes, 128);
+    P.sc_half_bytes = round_up(P.p1.TR * P.p1.G * 2 + 32, 16);
+    P.stage_bytes = round_up(P.stage_w_bytes + max(2 * P.sc_half_bytes, round_up(P.p2.TR * P.p2.G * 2 + 32, 16)), 128);
     const size_t fixed = fused_smem_header(tokens) + (size_t)P.xs_bytes;
     if (fixed + 2 * (size_t)P.stage_bytes > (size_t)smem_optin) return false;
     P.nstages = (int)min((size_t)kMaxStages, ((size_t)smem_optin - fixed) / (size_t)P.stage_bytes);
@@ -920,33 +1051,20 @@ int fused_ffn_launch(cudaStream_t stream, const void *normed, void *act, void *l
 #undef FFN_LAUNCH
 }
 
-/* Bytes of the smaller phase's tiles that the ring holds: what is on its way from HBM at the worst time. */
-static size_t ring_bytes(const FusedParams &P) { return (size_t)P.nstages * min(2 * P.p1.TR * P.p1.rb, P.p2.TR * P.p2.rb); }
-/* The plan of a stack: the threads' columns and rows of a single layer's (the same sums in the same order), with
- * the row steps of both phases' tiles chosen so that the ring holds the most. */
+/* The plan of a stack: a single layer's (the same sums in the same order) with room for either input.  Tiles of fewer rows
+ * would leave more of them in flight, but each tile costs every warp its share of instructions: 2560 x 9728, 36 layers, two and two
+ * row steps / two and four: 1 token 594 / 606 us, 2 tokens 932 / 856. */
 static bool plan_stack(FusedParams &P, int tokens, int H, int I, int smem_optin, int &c1, int &c2, size_t &smem) {
     if (!plan_fused(P, tokens, H, I, smem_optin, kDefaultStageTarget, c1, c2, smem)) return false;
-    FusedParams best = P;
-    const int most1 = P.p1.JT, most2 = P.p2.JT, xs_bytes = round_up(tokens * max(H, I) * 2, 128); /* act or the residual stream */
-    for (int j1 = most1; j1 >= 1; --j1)
-        for (int j2 = most2; j2 >= 1; --j2) {
-            FusedParams T = P;
-            T.p1.JT = j1; T.p1.TR = j1 * T.p1.RG;
-            T.p2.JT = j2; T.p2.TR = j2 * T.p2.RG;
-            T.xs_bytes = xs_bytes;
-            size_t bytes = 0;
-            if (plan_ring(T, tokens, smem_optin, bytes) && (best.xs_bytes != xs_bytes || ring_bytes(T) > ring_bytes(best))) {
-                best = T;
-                smem = bytes;
-            }
-        }
-    P = best;
-    return P.xs_bytes == xs_bytes;
+    const int values = tokens * max(H, I); /* act or the residual stream */
+    P.fac_offset = values * 2;
+    P.xs_bytes = round_up(values * 2 + values / 32 * (int)sizeof(float), 128);
+    return plan_ring(P, tokens, smem_optin, smem);
 }
 
 int fused_stack_launch(cudaStream_t stream, void *h, void *act, void *layer_out, const FfnMlpWeights *layers, int num_layers,
                        int tokens, int H, int I, float eps, int gemma) {
-    if (tokens < 1 || tokens > 2 || num_layers < 2) return FFN_NOT_ADMITTED;
+    if (tokens < 1 || tokens > 2 || num_layers < 1) return FFN_NOT_ADMITTED;
     DeviceState *dp = nullptr;
     const int st = device_state(&dp);
     if (st) return st;

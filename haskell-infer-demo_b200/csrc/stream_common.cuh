@@ -158,59 +158,59 @@ __device__ __forceinline__ void load_chunk(uint32_t (&v)[16], const uint16_t *sr
     }
 }
 
-/* RMSNorm of a slice: the reference's expression and its BF16 rounding */
-__device__ __forceinline__ void norm_chunk(uint32_t (&v)[16], const uint4 (&w)[4], float inv_rms, float gemma) {
+/* Eight values of a slice whose largest magnitude has the biased exponent E: their words {he, ho, le, lo} of the four
+ * planes; returns the slice's factor.  E < 19 (|x| < 2^-108) is treated as an all-zero slice.  A slice that holds an
+ * Inf or a NaN (E == 255) gets the factor NaN, so every row's sum becomes NaN: non-finite inputs give non-finite
+ * outputs, as the reference's FMA chain does (csrc/kernels/gemm_quant.cu:182-199), at no cost in the inner loop. */
+__device__ __forceinline__ float fixed_point8(const uint32_t (&e)[4], int E, uint32_t (&planes)[4]) {
+    const bool live = E >= 19 && E < 255;
+    const float up = live ? __uint_as_float((uint32_t)(268 - E) << 23) : 0.0f;   /* 2^(141-E) */
+    int X[8];
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        const uint32_t ww[4] = {w[q].x, w[q].y, w[q].z, w[q].w};
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const float lo = bf16_lo(v[4 * q + i]) * inv_rms * (bf16_lo(ww[i]) + gemma);
-            const float hi = bf16_hi(v[4 * q + i]) * inv_rms * (bf16_hi(ww[i]) + gemma);
-            v[4 * q + i] = (uint32_t)f32_to_bf16_bits(lo) | ((uint32_t)f32_to_bf16_bits(hi) << 16);
-        }
+    for (int i = 0; i < 4; ++i) {
+        /* 1.5*2^23 + x*up has the rounded (nearest-even) integer in its low mantissa bits; only
+         * the low 16 bits are used below and 0x4B400000 contributes none of them */
+        X[2 * i] = __float_as_int(fmaf(bf16_lo(e[i]), up, 12582912.0f));
+        X[2 * i + 1] = __float_as_int(fmaf(bf16_hi(e[i]), up, 12582912.0f));
     }
+    /* bytes 0/1 of each X are its low/high byte (two's complement 16-bit) */
+    const uint32_t e02 = prmt(X[0], X[2], 0x5140), e46 = prmt(X[4], X[6], 0x5140); /* lo0 lo2 hi0 hi2 */
+    const uint32_t o13 = prmt(X[1], X[3], 0x5140), o57 = prmt(X[5], X[7], 0x5140);
+    planes[0] = prmt(e02, e46, 0x7632);
+    planes[1] = prmt(o13, o57, 0x7632);
+    planes[2] = prmt(e02, e46, 0x5410);
+    planes[3] = prmt(o13, o57, 0x5410);
+    return live ? __uint_as_float((uint32_t)(E - 18) << 23)                    /* 2^(E-141) / 16 */
+                : (E == 255 ? __uint_as_float(0x7FC00000u) : 0.0f);
 }
 
 __device__ __forceinline__ void prepare_chunk(XChunk &xc, uint32_t (&v)[16], bool on,
                                               const uint16_t *norm_w = nullptr /* global, this chunk's 32 weights */,
                                               float inv_rms = 1.0f, float gemma = 0.0f) {
-    if (norm_w != nullptr && on) {
-        uint4 w[4];
+    if (norm_w != nullptr && on) { /* fused RMSNorm: the reference's expression and its BF16 rounding */
 #pragma unroll
-        for (int q = 0; q < 4; ++q) w[q] = __ldg((const uint4 *)(norm_w + q * 8));
-        norm_chunk(v, w, inv_rms, gemma);
+        for (int q = 0; q < 4; ++q) {
+            const uint4 wq = __ldg((const uint4 *)(norm_w + q * 8));
+            const uint32_t ww[4] = {wq.x, wq.y, wq.z, wq.w};
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const float lo = bf16_lo(v[4 * q + i]) * inv_rms * (bf16_lo(ww[i]) + gemma);
+                const float hi = bf16_hi(v[4 * q + i]) * inv_rms * (bf16_hi(ww[i]) + gemma);
+                v[4 * q + i] = (uint32_t)f32_to_bf16_bits(lo) | ((uint32_t)f32_to_bf16_bits(hi) << 16);
+            }
+        }
     }
     uint32_t mx = 0; /* per-halfword maximum of the magnitude bits */
 #pragma unroll
     for (int i = 0; i < 16; ++i) mx = __vmaxu2(mx, v[i] & 0x7FFF7FFFu);
     const uint32_t top = max(mx & 0xFFFFu, mx >> 16);
     const int E = (int)(top >> 7); /* biased exponent of the largest magnitude */
-    /* E < 19 (|x| < 2^-108) is treated as an all-zero slice.  A slice that holds an Inf or a NaN
-     * (E == 255) gets fac = NaN, so every row's sum becomes NaN: non-finite inputs give non-finite
-     * outputs, as the reference's FMA chain does (csrc/kernels/gemm_quant.cu:182-199), at no cost
-     * in the inner loop. */
-    const bool live = E >= 19 && E < 255;
-    const float up = live ? __uint_as_float((uint32_t)(268 - E) << 23) : 0.0f;   /* 2^(141-E) */
-    xc.fac = live ? __uint_as_float((uint32_t)(E - 18) << 23)                    /* 2^(E-141) / 16 */
-                  : (E == 255 ? __uint_as_float(0x7FC00000u) : 0.0f);
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-        int X[8];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            /* 1.5*2^23 + x*up has the rounded (nearest-even) integer in its low mantissa bits; only
-             * the low 16 bits are used below and 0x4B400000 contributes none of them */
-            X[2 * i] = __float_as_int(fmaf(bf16_lo(v[4 * j + i]), up, 12582912.0f));
-            X[2 * i + 1] = __float_as_int(fmaf(bf16_hi(v[4 * j + i]), up, 12582912.0f));
-        }
-        /* bytes 0/1 of each X are its low/high byte (two's complement 16-bit) */
-        const uint32_t e02 = prmt(X[0], X[2], 0x5140), e46 = prmt(X[4], X[6], 0x5140); /* lo0 lo2 hi0 hi2 */
-        const uint32_t o13 = prmt(X[1], X[3], 0x5140), o57 = prmt(X[5], X[7], 0x5140);
-        xc.le[j] = prmt(e02, e46, 0x5410);
-        xc.he[j] = prmt(e02, e46, 0x7632);
-        xc.lo[j] = prmt(o13, o57, 0x5410);
-        xc.ho[j] = prmt(o13, o57, 0x7632);
+        const uint32_t e[4] = {v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]};
+        uint32_t planes[4];
+        xc.fac = fixed_point8(e, E, planes);
+        xc.he[j] = planes[0]; xc.ho[j] = planes[1]; xc.le[j] = planes[2]; xc.lo[j] = planes[3];
     }
 }
 
