@@ -66,6 +66,7 @@ struct FusedParams {
     unsigned *tp_seq;     /* this communicator's call counter (slot parity, tag of the exchanged words) */
     /* optional fused residual update with the reduced output y: h <- bf16(h + y); NULL = off */
     uint16_t *residual;
+    uint16_t *normed;     /* a stack of one layer: optional bf16 [M][H], receives the normalized input */
     /* optional fused RMSNorm of the input (x is then the residual stream h): n = bf16(h * rsqrt(mean(h^2)
      * + eps) * (w + gemma)); NULL = x is already normalized */
     const uint16_t *norm_w;
@@ -234,6 +235,7 @@ __device__ __forceinline__ bool stage_input(const FusedParams &P, const PhasePla
                     e[i] = (uint32_t)f32_to_bf16_bits(lo) | ((uint32_t)f32_to_bf16_bits(hi) << 16);
                 }
             }
+            if (PAIRS && P.normed && blockIdx.x == 0 && q < total) *(uint4 *)(P.normed + (size_t)q * 8) = make_uint4(e[0], e[1], e[2], e[3]);
             uint32_t top = 0; /* the largest magnitude's bits */
 #pragma unroll
             for (int i = 0; i < 4; ++i) top = max(top, max(e[i] & 0x7FFFu, (e[i] >> 16) & 0x7FFFu));
@@ -480,7 +482,7 @@ __device__ __forceinline__ bool epilogue_phase(const FusedParams &P, const Phase
         const int pslot = tile % kPartSlots;
         const int rows = min(pl.TR, row_end - (row_begin + lt * pl.TR));
         float res = 0.0f;
-        if (STACK && !PAIRS && lane < rows * MT) /* this thread's own store of the layer before */
+        if (STACK && !PAIRS && P.residual && lane < rows * MT) /* this thread's own store of the layer before */
             res = bf16_bits_to_f32(P.residual[(size_t)(lane % MT) * P.H + row_begin + lt * pl.TR + lane / MT]);
         if (!mbar_wait<100>(&sm->part_full[pslot], (uint32_t)(tile / kPartSlots) & 1u, &sm->abort_flag)) {
             give_up(sm, P.sync, ST_PART_FULL);
@@ -503,8 +505,10 @@ __device__ __forceinline__ bool epilogue_phase(const FusedParams &P, const Phase
             } else if (STACK) {
                 const size_t o = (size_t)m * P.H + row;
                 const float y = round_bf16(a);
-                if (i != lane) res = bf16_bits_to_f32(P.residual[o]);
-                P.residual[o] = f32_to_bf16_bits(res + y);
+                if (P.residual) {
+                    if (i != lane) res = bf16_bits_to_f32(P.residual[o]);
+                    P.residual[o] = f32_to_bf16_bits(res + y);
+                }
                 if (store_out) P.out[o] = f32_to_bf16_bits(y);
             } else if (P.tp == 1) {
                 const float y = round_bf16(a);
@@ -1062,8 +1066,8 @@ static bool plan_stack(FusedParams &P, int tokens, int H, int I, int smem_optin,
     return plan_ring(P, tokens, smem_optin, smem);
 }
 
-int fused_stack_launch(cudaStream_t stream, void *h, void *act, void *layer_out, const FfnMlpWeights *layers, int num_layers,
-                       int tokens, int H, int I, float eps, int gemma) {
+int fused_stack_launch(cudaStream_t stream, const void *x, void *residual, void *normed, void *act, void *layer_out,
+                       const FfnMlpWeights *layers, int num_layers, int tokens, int H, int I, float eps, int gemma) {
     if (tokens < 1 || tokens > 2 || num_layers < 1) return FFN_NOT_ADMITTED;
     DeviceState *dp = nullptr;
     const int st = device_state(&dp);
@@ -1071,7 +1075,7 @@ int fused_stack_launch(cudaStream_t stream, void *h, void *act, void *layer_out,
     DeviceState &d = *dp;
     const int grid = d.sm_count;
     if (!d.cooperative || H < grid || I < grid) return FFN_NOT_ADMITTED; /* every CTA has rows in both phases */
-    uintptr_t any = (uintptr_t)h | (uintptr_t)act;
+    uintptr_t any = (uintptr_t)x | (uintptr_t)act | (uintptr_t)normed;
     for (int l = 0; l < num_layers; ++l) {
         const FfnMlpWeights &w = layers[l];
         if (!w.gate_up_i4 || !w.gate_up_i4_scales || !w.down_i4 || !w.down_i4_scales || w.i4_group != FFN_INT4_GROUP || !w.post_norm_w) return FFN_NOT_ADMITTED;
@@ -1084,7 +1088,7 @@ int fused_stack_launch(cudaStream_t stream, void *h, void *act, void *layer_out,
     int c1 = 0, c2 = 0;
     size_t smem = 0;
     if (!plan_stack(P, tokens, H, I, d.smem_optin, c1, c2, smem)) return FFN_NOT_ADMITTED;
-    P.x = (const uint16_t *)h; P.residual = (uint16_t *)h;
+    P.x = (const uint16_t *)x; P.residual = (uint16_t *)residual; P.normed = (uint16_t *)normed;
     P.act = (uint16_t *)act; P.out = (uint16_t *)layer_out;
     P.sync = d.sync;
     P.tp = 1;

@@ -117,9 +117,10 @@ struct FusedNorm {
 int fused_ffn_launch(cudaStream_t stream, const void *normed, void *act, void *layer_out,
                      const FfnMlpWeights *w, int tokens, int H, int I, const FusedTp *tp, void *residual,
                      const FusedNorm *norm);
-/* One rank's stack of layers, one or two tokens, in one launch per 64 layers: `h` is the residual stream, updated in place. */
-int fused_stack_launch(cudaStream_t stream, void *h, void *act, void *layer_out, const FfnMlpWeights *layers, int num_layers,
-                       int tokens, int H, int I, float eps, int gemma);
+/* One rank's stack of layers, one or two tokens, in one launch per 64 layers.  `residual` is the residual stream, x at first
+ * and updated in place.  One layer alone may do without it, and leave its normalized input in `normed`. */
+int fused_stack_launch(cudaStream_t stream, const void *x, void *residual, void *normed, void *act, void *layer_out,
+                       const FfnMlpWeights *layers, int num_layers, int tokens, int H, int I, float eps, int gemma);
 /* Reads (synchronously) the status word the fused kernel writes when a bounded wait runs out:
  * 0 = fine, else (where | cta << 8).  With reset, a non-zero status also clears the kernel's
  * synchronisation words so the next launch starts clean. */

@@ -408,7 +408,7 @@ int ffn_decode_stack(FfnTpComm *comm, void *stream, void *h, void *ws, void *lay
             st = kmajor_ffn_launch((cudaStream_t)stream, h, act, layer_out, layers, num_layers, tokens, H, I, tp, h, 1, dims->rms_eps,
                                    dims->norm_style == 0, status);
             if (st != FFN_NOT_ADMITTED) return st;
-            if (!tp && (st = fused_stack_launch((cudaStream_t)stream, h, act, layer_out, layers, num_layers, tokens, H, I, dims->rms_eps,
+            if (!tp && (st = fused_stack_launch((cudaStream_t)stream, h, h, nullptr, act, layer_out, layers, num_layers, tokens, H, I, dims->rms_eps,
                                                 dims->norm_style == 0)) != FFN_NOT_ADMITTED) return st;
         }
     }

@@ -51,3 +51,28 @@ def test_two_launches_in_a_graph(cuda):
     torch.cuda.synchronize()
     L.device_status()
     assert all(same(o, w) for o, w in zip(out, want))
+
+
+@pytest.mark.parametrize("tokens", [1, 2])
+@pytest.mark.parametrize("hidden,inter", [(256, 256), (128, 1024), (1024, 3072), (2560, 9728), (8192, 512), (512, 12288), (512, 12416), (4096, 14336)])
+def test_norm_and_ffn_in_one_launch(cuda, tokens, hidden, inter):
+    """ffn_forward_mlp of one and two tokens: against FP64 at the FFN bar, the normalized rows in the workspace within
+    one BF16 step of the norm kernel's, output over input."""
+    (mlp,), draw = layers_of(cuda, hidden, inter, 1)
+    x = draw(tokens)
+    ws = mlp.workspace(tokens)
+    ws.zero_()
+    y = mlp.forward_mlp(x, ws)
+    L.device_status()
+    gate_up, gate_up_scales, down, down_scales, w_norm = mlp.tensors
+    xd = x.double()
+    normed = xd * torch.rsqrt(xd.square().mean(dim=1, keepdim=True) + 1e-6) * (1 + w_norm.double())
+    got = ws.view(-1)[:tokens * hidden].view(tokens, hidden).double()
+    # half a BF16 step, and a whole one where FP32 rounds a product or two to the other side
+    assert ((got - normed).abs() <= normed.abs() * 2.0 ** -7).all()
+    g, u = (normed.to(torch.bfloat16).double() @ ops.dequantize_int4(gate_up, gate_up_scales)[0].double().T).chunk(2, dim=1)
+    want = (torch.nn.functional.silu(g) * u) @ ops.dequantize_int4(down, down_scales)[0].double().T
+    assert (y.double() - want).norm() <= 5e-3 * want.norm()
+    z = x.clone()
+    mlp.forward_mlp(z, ws, z)
+    assert same(z, y)
