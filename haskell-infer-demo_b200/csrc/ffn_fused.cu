@@ -936,8 +936,27 @@ static int launch_resident(DeviceState &d, bool &attr_set, bool &fits, void (*ke
      * Whether the driver takes the attribute next to a cooperative launch is found out once per
      * device, outside stream capture; until then, and wherever it is refused, the launch is the
      * plain cooperative one. */
+    cudaLaunchAttribute attrs[2];
+    attrs[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attrs[0].val.programmaticStreamSerializationAllowed = 1;
+    attrs[1].id = cudaLaunchAttributeCooperative;
+    attrs[1].val.cooperative = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cfg.attrs = attrs;
+    if (P.gemv) {
+        /* Nothing waits for another CTA, and nothing is read early: the weights of a GEMM may come from the launch before.
+         * us back to back, cooperative -> so: 1 row 4096 x 5120 8.4 -> 6.1, 12288 x 5120 12.5 -> 10.5,
+         * 5120 x 17408 16.1 -> 13.3, 34816 x 5120 20.9 -> 18.5, 248320 x 5120 101 -> 98; 2 rows 4096 x 5120 10.4 -> 7.2, 34816 x 5120 29.4 -> 27.0. */
+        cfg.numAttrs = g_launch_overlap ? 1 : 0;
+        FFN_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, params), "streaming GEMV launch");
+        return FFN_OK;
+    }
     int overlap = 0;
-    if (g_launch_overlap && !P.gemv) {
+    if (g_launch_overlap) {
         if (d.overlap_ok == 1) {
             overlap = 1;
         } else if (d.overlap_ok == 0) {
@@ -947,17 +966,6 @@ static int launch_resident(DeviceState &d, bool &attr_set, bool &fits, void (*ke
     }
     if (overlap) {
         P.early_weights = 1;
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(grid);
-        cfg.blockDim = dim3(kThreads);
-        cfg.dynamicSmemBytes = smem;
-        cfg.stream = stream;
-        cudaLaunchAttribute attrs[2];
-        attrs[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attrs[0].val.programmaticStreamSerializationAllowed = 1;
-        attrs[1].id = cudaLaunchAttributeCooperative;
-        attrs[1].val.cooperative = 1;
-        cfg.attrs = attrs;
         cfg.numAttrs = plain ? 1 : 2;
         const cudaError_t err = cudaLaunchKernelEx(&cfg, kernel, params);
         if (err == cudaSuccess) {
