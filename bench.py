@@ -393,8 +393,8 @@ def run_ours(args):
         one_rank = world == 1 and L.load().ffn_int4_set_batched_kernel(-1) == 2    # the norm is then part of the input pre-pass
         per_layer = 1 if (m <= 2 or kmajor) else (4 if stack and not one_rank else 3)
         launches = nl * per_layer
-        if stack and kmajor:
-            launches = -(-nl // 64)          # the whole stack in one persistent launch per 64 layers
+        if stack and (kmajor or (m <= 2 and world == 1)):
+            launches = -(-nl // 64)          # the whole stack in one launch per 64 layers
         line = {
             "metric": METRIC, "value": round(us_step, 3), "unit": "us/step", "n_gpus": world,
             "steps": args.steps, "warmup": max(args.warmup, 3), "ms_per_step": round(us_step / 1e3, 6),
