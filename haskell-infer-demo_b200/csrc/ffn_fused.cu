@@ -877,11 +877,13 @@ static int device_state(DeviceState **out) {
     return FFN_OK;
 }
 
-/* The stages of a launch whose tiles and input copy are known. */
-static bool plan_ring(FusedParams &P, int tokens, int smem_optin, size_t &smem) {
+/* The stages of a launch whose tiles and input copy are known.  `tight`: room for scales as each phase needs it, instead of
+ * two runs of the longer kind - what lets a stack's factors in beside three stages of the 5120 x 17408 layer. */
+static bool plan_ring(FusedParams &P, int tokens, int smem_optin, size_t &smem, bool tight = false) {
     P.stage_w_bytes = round_up(max(2 * P.p1.TR * P.p1.rb, P.p2.TR * P.p2.rb), 128);
-    P.sc_half_bytes = round_up(P.p1.TR * P.p1.G * 2 + 32, 16);
-    P.stage_bytes = round_up(P.stage_w_bytes + max(2 * P.sc_half_bytes, round_up(P.p2.TR * P.p2.G * 2 + 32, 16)), 128);
+    const int run1 = round_up(P.p1.TR * P.p1.G * 2 + 32, 16), run2 = round_up(P.p2.TR * P.p2.G * 2 + 32, 16);
+    P.sc_half_bytes = tight ? run1 : max(run1, run2);
+    P.stage_bytes = round_up(P.stage_w_bytes + max(2 * P.sc_half_bytes, run2), 128);
     const size_t fixed = fused_smem_header(tokens) + (size_t)P.xs_bytes;
     if (fixed + 2 * (size_t)P.stage_bytes > (size_t)smem_optin) return false;
     P.nstages = (int)min((size_t)kMaxStages, ((size_t)smem_optin - fixed) / (size_t)P.stage_bytes);
@@ -1071,7 +1073,7 @@ static bool plan_stack(FusedParams &P, int tokens, int H, int I, int smem_optin,
     const int values = tokens * max(H, I); /* act or the residual stream */
     P.fac_offset = values * 2;
     P.xs_bytes = round_up(values * 2 + values / 32 * (int)sizeof(float), 128);
-    return plan_ring(P, tokens, smem_optin, smem);
+    return plan_ring(P, tokens, smem_optin, smem, true);
 }
 
 int fused_stack_launch(cudaStream_t stream, const void *x, void *residual, void *normed, void *act, void *layer_out,
