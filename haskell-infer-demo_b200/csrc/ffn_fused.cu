@@ -369,7 +369,9 @@ __device__ __forceinline__ void consume_phase(const FusedParams &P, const PhaseP
     /* Instructions bound this loop (some 250 a tile and warp, 62 thousand an SM in a 2560 x 9728 layer, of which the products are
      * a third), so what a tile needs is carried along instead of computed from its number, and a ragged last tile leaves out the
      * row steps that it does not have.  Together, us per call: 5120 x 17408 1 token 30.6 -> 29.9, 2 tokens 45.8 -> 42.5; 2560 x 9728
-     * 1 token 16.1 -> 15.0, 2 tokens with a norm 25.7 -> 23.4; 5120 x 2176 1 token 12.0 -> 11.1; 1024 x 3072 10.1 -> 9.6. */
+     * 1 token 16.1 -> 15.0, 2 tokens with a norm 25.7 -> 23.4; 5120 x 2176 1 token 12.0 -> 11.1; 1024 x 3072 10.1 -> 9.6.  Addresses
+     * by steps instead of from clamped rows, then: 5120 x 17408 1 token 29.8 -> 29.6, 2 tokens 42.6 -> 41.5; 2560 x 9728 2 tokens with a norm
+     * 23.6 -> 23.0.  (Looking at the next tile's barriers ahead of time costs more instructions than the waits: +1.5 %.) */
     int s = tile0 % nstages, pslot = tile0 % kPartSlots; /* the tile's stage and partial slot, and the parities of their rounds */
     uint32_t s_phase = (uint32_t)(tile0 / nstages) & 1u, p_phase = (uint32_t)(tile0 / kPartSlots) & 1u;
     uint32_t st = ring_addr + (uint32_t)s * (uint32_t)stage_bytes; /* 32-bit shared-window addresses */
@@ -385,13 +387,12 @@ __device__ __forceinline__ void consume_phase(const FusedParams &P, const PhaseP
         part_row[q] = (lane & 3) == 0 && j < pl.JT ? p : pl.TR;
         part_at[q] = (p * NVROW + i) * pl.nhw + (ct >> 4);
     }
-    uint32_t coff[CIT], soff[CIT]; /* a column chunk past the row end reads a clamped address against an all-zero prepared slice */
-#pragma unroll
-    for (int c = 0; c < CIT; ++c) {
-        const int col = min(ct + c * pl.CT, pl.cpr - 1);
-        coff[c] = (uint32_t)col * 16u;
-        soff[c] = (uint32_t)(col >> 2) * 2u;
-    }
+    /* This thread's first chunk in a tile, its scale, and the way to its other column chunk; a chunk past the row end reads a
+     * clamped address against an all-zero prepared slice.  A row step is RG rows on. */
+    const int col0 = min(ct, pl.cpr - 1), col1 = min(ct + (CIT - 1) * pl.CT, pl.cpr - 1);
+    const uint32_t my_w = (uint32_t)rg * (uint32_t)pl.rb + (uint32_t)col0 * 16u, my_s = (uint32_t)rg * g2 + (uint32_t)(col0 >> 2) * 2u;
+    const uint32_t next_w = (uint32_t)(col1 - col0) * 16u, next_s = (uint32_t)((col1 >> 2) - (col0 >> 2)) * 2u;
+    const uint32_t step_w = (uint32_t)(pl.RG * pl.rb), step_s = (uint32_t)pl.RG * g2;
     for (int left = row_end - row_begin; left > 0; left -= pl.TR) {
         const int rows = min(pl.TR, left);
         if (!mbar_wait<32>(&sm->full[s], s_phase, &sm->abort_flag)) {
@@ -414,27 +415,26 @@ __device__ __forceinline__ void consume_phase(const FusedParams &P, const PhaseP
 #pragma unroll
         for (int v = 0; v < VALS; ++v) val[v] = 0.0f;
         if (active && !FFN_DEBUG_BIT(P, 1)) {
-            /* No data-dependent branches in here: a row past the tile end reads the tile's last row and its value is
-             * dropped at the store.  That leaves the compiler free to overlap the shared-memory loads and the
-             * integer chains of all chunks of a row step. */
+            /* No data-dependent branches in here: a row past the tile's end reads what the stage held before (still inside
+             * it) and its value is dropped at the store.  That leaves the compiler free to overlap the shared-memory
+             * loads and the integer chains of all chunks of a row step. */
             const uint32_t up_bytes = (uint32_t)rows * (uint32_t)pl.rb;
+            uint32_t wp = st + my_w, s0p = sc0 + my_s, s1p = sc1 + my_s;
 #pragma unroll
             for (int j = 0; j < JTM; ++j) {
                 if (j < pl.JT && j * pl.RG < rows) { /* uniform over the CTA; a ragged last tile's absent steps are left out */
-                    const int pj = min(rg + j * pl.RG, rows - 1);
-                    const uint32_t wp = st + (uint32_t)pj * (uint32_t)pl.rb;
-                    const uint32_t s0p = sc0 + (uint32_t)pj * g2, s1p = sc1 + (uint32_t)pj * g2;
                     uint4 w0[CIT], w1[CIT];
                     float f0[CIT], f1[CIT];
 #pragma unroll
                     for (int c = 0; c < CIT; ++c) {
-                        w0[c] = lds16_at(wp + coff[c]);
-                        f0[c] = lds_bf16_at(s0p + soff[c]);
+                        w0[c] = lds16_at(c ? wp + next_w : wp);
+                        f0[c] = lds_bf16_at(c ? s0p + next_s : s0p);
                         if (PAIRS) {
-                            w1[c] = lds16_at(wp + up_bytes + coff[c]);
-                            f1[c] = lds_bf16_at(s1p + soff[c]);
+                            w1[c] = lds16_at(wp + up_bytes + (c ? next_w : 0u));
+                            f1[c] = lds_bf16_at(c ? s1p + next_s : s1p);
                         }
                     }
+                    wp += step_w; s0p += step_s; s1p += step_s;
 #pragma unroll
                     for (int c = 0; c < CIT; ++c) {
 #pragma unroll
