@@ -168,10 +168,10 @@ __device__ __forceinline__ float fixed_point8(const uint32_t (&e)[4], int E, uin
     int X[8];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-        /* 1.5*2^23 + x*up has the rounded (nearest-even) integer in its low mantissa bits; only
+        /* two to an instruction; 1.5*2^23 + x*up has the rounded (nearest-even) integer in its low mantissa bits; only
          * the low 16 bits are used below and 0x4B400000 contributes none of them */
-        X[2 * i] = __float_as_int(fmaf(bf16_lo(e[i]), up, 12582912.0f));
-        X[2 * i + 1] = __float_as_int(fmaf(bf16_hi(e[i]), up, 12582912.0f));
+        asm("{\n.reg .b64 x, u, m;\nmov.b64 x, {%2, %3};\nmov.b64 u, {%4, %4};\nmov.b64 m, {%5, %5};\nfma.rn.f32x2 x, x, u, m;\nmov.b64 {%0, %1}, x;\n}"
+            : "=r"(X[2 * i]), "=r"(X[2 * i + 1]) : "f"(bf16_lo(e[i])), "f"(bf16_hi(e[i])), "f"(up), "f"(12582912.0f));
     }
     /* bytes 0/1 of each X are its low/high byte (two's complement 16-bit) */
     const uint32_t e02 = prmt(X[0], X[2], 0x5140), e46 = prmt(X[4], X[6], 0x5140); /* lo0 lo2 hi0 hi2 */
