@@ -12,15 +12,18 @@
  * writes anything; so does this file (one checking pass, then the writing pass).
  *
  * HBM bound: the FP32 input is read once.  The checking pass quantizes into scratch as it goes, and a second
- * launch moves the bytes to the caller once nothing was refused - it looks at the verdict itself, so the host
+ * launch moves the bytes to the caller once nothing was refused - it looks at the verdict itself and tells the host, which
  * waits once, at the end.  5120 x 17408: 221 us with a checking and a writing pass over the input, a wait
- * between them and cudaMalloc / cudaFree around them; 111 now.  Where the bytes exceed the scratch that
+ * between them and cudaMalloc / cudaFree around them; 111 with the verdict cleared and copied by operations of
+ * their own, 104 now (1024 x 2560: 46 -> 38 as the caller sees it).  Where the bytes exceed the scratch that
  * the library keeps (kScratchMost), or there is no memory for them, the second launch quantizes again instead.
  *
  * Eight lanes per group: a lane holds sixteen elements in four 16-byte loads (128 contiguous bytes of a group
  * each), so the group's division, reciprocal and reduction are paid once per sixteen elements: instructions, not
  * bytes, are what is left (142 us with a warp per group and four elements a lane).
  */
+#include <mutex>
+
 #include "common.cuh"
 #include "kernels.h"
 
@@ -39,6 +42,20 @@ struct QuantStatus {
     unsigned long long bad_group;   /* 1 + (row * groups + group) of an unrepresentable scale, 0 = none */
 };
 
+/* The verdict of a call.  Every launch of a call is handed all of it: the checking pass marks what it finds in `here`
+ * (none at the start of the call) and leaves `next`, the words of the call after, clear; the last launch tells the host.
+ * So a call needs no clearing and no copy of its own. */
+struct QuantVerdict {
+    QuantStatus *here, *next; /* device memory; next may be null */
+    QuantStatus *host;        /* mapped host memory; may be null */
+};
+__device__ __forceinline__ void quant_clear_next(const QuantVerdict &v) {
+    if (v.next && blockIdx.x == 0 && threadIdx.x == 0) { v.next->bad_element = ~0ull; v.next->bad_group = ~0ull; }
+}
+__device__ __forceinline__ void quant_tell(const QuantVerdict &v) {
+    if (v.host && blockIdx.x == 0 && threadIdx.x == 0) *v.host = *v.here;
+}
+
 constexpr int kGroupsInFlight = 4;
 constexpr int kQuantThreads = 256;
 constexpr size_t kScratchMost = 56ull << 20; /* of the 64 MiB that the library's pool keeps between calls */
@@ -48,7 +65,10 @@ constexpr size_t kScratchMost = 56ull << 20; /* of the 64 MiB that the library's
 template <bool CHECK>
 __global__ void __launch_bounds__(kQuantThreads) quantize_int4_kernel(const float *__restrict__ w, uint8_t *__restrict__ packed,
                                                                      uint16_t *__restrict__ scales, long long groups_total,
-                                                                     QuantStatus *status) {
+                                                                     const QuantVerdict verdict) {
+    QuantStatus *const status = verdict.here;
+    if (CHECK) quant_clear_next(verdict);
+    else quant_tell(verdict);
     if (!CHECK && (status->bad_element != ~0ull || status->bad_group != ~0ull)) return;
     const int lane = threadIdx.x & 31, sub = lane & 7;
     const long long warp = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -114,11 +134,58 @@ __global__ void __launch_bounds__(kQuantThreads) quantize_int4_kernel(const floa
 template <typename T>
 __global__ void __launch_bounds__(kQuantThreads) quantize_deliver_kernel(T *__restrict__ packed, const T *__restrict__ from_packed, long long np,
                                                                         T *__restrict__ scales, const T *__restrict__ from_scales, long long ns,
-                                                                        const QuantStatus *status) {
+                                                                        const QuantVerdict verdict) {
+    const QuantStatus *const status = verdict.here;
+    quant_tell(verdict);
     if (status->bad_element != ~0ull || status->bad_group != ~0ull) return;
     const long long step = (long long)gridDim.x * kQuantThreads, at = (long long)blockIdx.x * kQuantThreads + threadIdx.x;
     for (long long i = at; i < np; i += step) packed[i] = from_packed[i];
     for (long long i = at; i < ns; i += step) scales[i] = from_scales[i];
+}
+
+/* The words of calls in flight: per device eight at most, kept until the process ends, each one call's at a time - a
+ * call ends when the stream has been waited for.  Calls beyond those clear and copy words of their own. */
+struct QuantWords {
+    QuantStatus *device = nullptr, *host = nullptr, *host_mapped = nullptr;
+    int turn = 0;
+    bool busy = false;
+};
+constexpr int kQuantWords = 8;
+static QuantWords g_quant_words[64][kQuantWords];
+static std::mutex g_quant_mutex;
+
+static QuantWords *quant_words_take() {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) { (void)cudaGetLastError(); return nullptr; }
+    std::lock_guard<std::mutex> lock(g_quant_mutex);
+    for (QuantWords &w : g_quant_words[dev]) {
+        if (w.busy) continue;
+        if (!w.device) {
+            QuantStatus *device = nullptr, *host = nullptr, *mapped = nullptr;
+            cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed; /* another thread's capture in global mode goes on */
+            (void)cudaThreadExchangeStreamCaptureMode(&mode);
+            const bool failed = cudaMalloc(&device, 2 * sizeof(QuantStatus)) != cudaSuccess || cudaHostAlloc(&host, sizeof(QuantStatus), cudaHostAllocMapped) != cudaSuccess ||
+                cudaHostGetDevicePointer(&mapped, host, 0) != cudaSuccess ||
+                cudaMemsetAsync(device, 0xFF, 2 * sizeof(QuantStatus), cudaStreamPerThread) != cudaSuccess || cudaStreamSynchronize(cudaStreamPerThread) != cudaSuccess;
+            (void)cudaThreadExchangeStreamCaptureMode(&mode);
+            if (failed) {
+                (void)cudaGetLastError();
+                if (device) cudaFree(device);
+                if (host) cudaFreeHost(host);
+                return nullptr;
+            }
+            w.device = device; w.host = host; w.host_mapped = mapped;
+        }
+        w.busy = true;
+        return &w;
+    }
+    return nullptr;
+}
+static void quant_words_return(QuantWords *w, bool sound) {
+    if (!w) return;
+    std::lock_guard<std::mutex> lock(g_quant_mutex);
+    w->turn ^= 1;
+    w->busy = !sound; /* words that a failed launch may have left anyhow are not used again */
 }
 
 }  // namespace ffn
@@ -137,21 +204,24 @@ extern "C" int ffn_quantize_int4(const void *weights, void *packed, void *scales
     const long long groups = n * (k / FFN_INT4_GROUP);
     const long long packed_bytes = n * k / 2, scale_bytes = groups * 2;
     bool keep = (size_t)(packed_bytes + scale_bytes) <= kScratchMost;
+    QuantWords *const words = quant_words_take();
     const size_t scales_at = 256 + ((size_t)packed_bytes + 255) / 256 * 256;
     uint8_t *scratch = nullptr;
     const bool pooled = scratch_alloc((void **)&scratch, keep ? scales_at + (size_t)scale_bytes : 256, stream) == FFN_OK;
     if (!pooled) {
         /* no room for the bytes (the call is made while weights fill the device): two passes and the status words */
         keep = false;
-        if (cudaMalloc(&scratch, sizeof(QuantStatus)) != cudaSuccess) { (void)cudaGetLastError(); return fail(FFN_ERR_ALLOC, "ffn_quantize_int4: cannot allocate the status words"); }
+        if (!words && cudaMalloc(&scratch, sizeof(QuantStatus)) != cudaSuccess) { (void)cudaGetLastError(); return fail(FFN_ERR_ALLOC, "ffn_quantize_int4: cannot allocate the status words"); }
     }
-    QuantStatus *status = (QuantStatus *)scratch;
     int rc = FFN_OK;
+    bool sound = true;
     QuantStatus host;
+    QuantVerdict status = {(QuantStatus *)scratch, nullptr, nullptr};
+    if (words) status = {words->device + words->turn, words->device + (words->turn ^ 1), words->host_mapped};
     const long long turns = (groups + kGroupsInFlight * 8 - 1) / (kGroupsInFlight * 8);
     const unsigned grid = (unsigned)(turns < 148ll * 16 ? turns : 148ll * 16);
     do {
-        if (cudaMemsetAsync(status, 0xFF, sizeof(QuantStatus), stream) != cudaSuccess) { rc = fail(FFN_ERR_CUDA, "ffn_quantize_int4: memset failed"); break; }
+        if (!words && cudaMemsetAsync(status.here, 0xFF, sizeof(QuantStatus), stream) != cudaSuccess) { rc = fail(FFN_ERR_CUDA, "ffn_quantize_int4: memset failed"); break; }
         quantize_int4_kernel<true><<<grid, kQuantThreads, 0, stream>>>((const float *)weights, keep ? scratch + 256 : nullptr,
                                                                        keep ? (uint16_t *)(scratch + scales_at) : nullptr, groups, status);
         if (!keep) {
@@ -163,11 +233,13 @@ extern "C" int ffn_quantize_int4(const void *weights, void *packed, void *scales
             quantize_deliver_kernel<uint16_t><<<148 * 8, kQuantThreads, 0, stream>>>((uint16_t *)packed, (const uint16_t *)(scratch + 256), packed_bytes / 2,
                                                                                      (uint16_t *)scales, (const uint16_t *)(scratch + scales_at), scale_bytes / 2, status);
         }
-        if (cudaGetLastError() != cudaSuccess || cudaMemcpyAsync(&host, status, sizeof(host), cudaMemcpyDeviceToHost, stream) != cudaSuccess ||
+        if (cudaGetLastError() != cudaSuccess || (!words && cudaMemcpyAsync(&host, status.here, sizeof(host), cudaMemcpyDeviceToHost, stream) != cudaSuccess) ||
             cudaStreamSynchronize(stream) != cudaSuccess) {
             rc = fail(FFN_ERR_CUDA, "ffn_quantize_int4: quantizing failed: %s", cudaGetErrorString(cudaGetLastError()));
+            sound = false;
             break;
         }
+        if (words) host = *words->host;
         if (host.bad_element != ~0ull) {
             rc = fail(FFN_ERR_WEIGHTS, "ffn_quantize_int4: element %llu is not finite; a quantizer cannot invent a scale for it",
                       host.bad_element - 1ull);
@@ -180,7 +252,8 @@ extern "C" int ffn_quantize_int4(const void *weights, void *packed, void *scales
             break;
         }
     } while (0);
+    quant_words_return(words, sound);
     if (pooled) (void)cudaFreeAsync(scratch, stream);
-    else cudaFree(scratch);
+    else if (scratch) cudaFree(scratch);
     return rc;
 }
