@@ -740,10 +740,8 @@ static int st_reserve(StScratch &sc, size_t bytes, cudaStream_t stream) {
 
 int stream_tc_ffn_launch(cudaStream_t stream, const void *x, void *act, void *layer_out, const FfnMlpWeights *w, int tokens, int H,
                          int I, void *residual, const FusedNorm *norm, void *normed, unsigned *status) {
-    /* One and two tokens are the single-launch kernel's.  At two, without a norm, us on the device, that kernel / this:
-     * 1024 x 3072 11.0 / 13.1, 2560 x 9728 20.7 / 22.6, 5120 x 4352 17.7 / 21.7, 5120 x 8704 27.3 / 27.6, 4096 x 14336
-     * 33.1 / 32.9, 5120 x 17408 46.7 / 43.5; with the norm as a launch of its own before it 13.0 / 13.2, 22.7 / 22.5,
-     * 19.6 / 22.1, 29.3 / 28.0, 35.2 / 32.9, 48.4 / 44.5. */
+    /* One and two tokens are the decode kernels'.  At two, without a norm, us back to back, those / this: 1024 x 3072 11.0 /
+     * 13.1, 2560 x 9728 19.4 / 22.6, 5120 x 4352 18.0 / 21.7, 5120 x 8704 25.7 / 27.6, 4096 x 14336 30.9 / 32.9, 5120 x 17408 41.5 / 43.5. */
     if (tokens <= 2 || tc_get_mode() != 2) return FFN_NOT_ADMITTED;
     if (((uintptr_t)w->gate_up_i4 & 15) || ((uintptr_t)w->down_i4 & 15) || ((uintptr_t)x & 15) || ((uintptr_t)normed & 15)) return FFN_NOT_ADMITTED;
     int dev = 0, sm_count = 0, st = st_device(&dev, &sm_count);
