@@ -76,3 +76,23 @@ def test_norm_and_ffn_in_one_launch(cuda, tokens, hidden, inter):
     z = x.clone()
     mlp.forward_mlp(z, ws, z)
     assert same(z, y)
+
+
+def test_without_launch_overlap(cuda):
+    """Cooperative launches, as with the overlap off, and plain ones in turn: the same results."""
+    mlps, draw = layers_of(cuda, 1024, 3072, 3)
+    x, h0 = draw(2), draw(1)
+
+    def call():
+        h = h0.clone()
+        ops.decode_stack(mlps, h)
+        return mlps[0].forward_mlp_prepared(x).clone(), mlps[1].forward_mlp(x).clone(), h
+
+    want = call()
+    for on in (0, 1, 0, 1):
+        old = L.load().ffn_int4_set_launch_overlap(on)
+        try:
+            assert all(same(a, b) for a, b in zip(call(), want))
+        finally:
+            L.load().ffn_int4_set_launch_overlap(old)
+    L.device_status()
